@@ -1,0 +1,66 @@
+"""The run-time scheduled kernels (wavesim_b200/csrc/ws_uni.cuh) against the
+generic kernels and the FP32 oracle where they can go wrong: lines of two,
+three and four stages, odd and even last radices (padding), every radix class,
+rows that do not fill a tile, columns that do not fill a block, one wiggle (a
+periodic grid) and eight, three components, and next to a fast inner pass.
+
+A dozen iterations of single-precision transforms of these lengths differ by a
+few 1e-7; 1e-5 leaves room for that and none for a wrong element."""
+
+import numpy as np
+import pytest
+
+from oracle import mbs_oracle as ref
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+CASES = {
+    # name: (roi shape, boundary widths (0: periodic, the size is taken as it is), vector)
+    "2d_4x6_one_wiggle": ((4, 6), [0, 0], False),
+    "2d_45x60": ((33, 42), [6, 8], False),
+    "2d_26x39": ((26, 39), [0, 0], False),
+    "2d_1100x21": ((1068, 21), [16, 0], False),
+    "2d_four_stages_2401x18": ((2401, 18), [0, 0], False),
+    "2d_18x2401": ((18, 2401), [0, 0], False),
+    "2d_64_columns_x_56": ((48, 40), [8, 8], False),
+    "2d_225x256": ((225, 256), [0, 0], False),
+    "3d_27x25x50": ((15, 13, 38), [6, 6, 6], False),
+    "3d_125x24x33": ((109, 12, 21), [8, 6, 6], False),
+    "3d_15x198x243": ((15, 198, 243), [0, 0, 0], False),
+    "3d_64_planes_z_50": ((48, 48, 38), [8, 8, 6], False),
+    "3d_vector_26x30x21": ((26, 18, 9), [0, 6, 6], True),
+    "3d_vector_63x16x105": ((47, 16, 89), [8, 0, 8], True),
+}
+
+
+def rel(a, b):
+    return float(np.linalg.norm(np.ravel(a) - np.ravel(b)) / np.linalg.norm(np.ravel(b)))
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_uni_matches_generic_and_oracle(gpu, name, monkeypatch):
+    import wavesim_b200 as ws
+    shape, bw, vector = CASES[name]
+    rng = np.random.default_rng(11)
+    n = 1.2 + 0.2 * rng.random(shape) + 0.005j
+    iters = 8 if len(shape) == 3 else 12
+    opt = {"lambda": 1.0, "pixel_size": 0.125 if vector else 0.25, "boundary_widths": bw, "energy_threshold": 1e-99,
+           "max_iterations": iters}
+    val = rng.standard_normal(shape[:2]) + 1j * rng.standard_normal(shape[:2])
+    pos = [1] * len(shape) + ([2] if vector else [])
+
+    def product():
+        sim = (ws.WaveSimVector if vector else ws.WaveSim)(n, opt)
+        E, st = sim.exec(ws.Source(val, pos))
+        sim.close()
+        return E, st
+
+    E, st = product()
+    monkeypatch.setenv("WAVESIM_B200_PATH", "generic")
+    Eg, sg = product()
+    Eo, so = (ref.WaveSimVector if vector else ref.WaveSim)(n, opt).exec(ref.Source(val, pos), max_iterations=iters)
+    assert st.it == sg.it == so.it
+    assert rel(E, Eg) < TOL and rel(E, Eo) < TOL, (rel(E, Eg), rel(E, Eo))
+    np.testing.assert_allclose(st.diff_energy, so.diff_energy, rtol=2e-4)

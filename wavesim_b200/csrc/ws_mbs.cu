@@ -22,6 +22,7 @@
 #include "ws_kernels.cuh"
 #include "ws_mixed.cuh"
 #include "ws_tma.cuh"
+#include "ws_uni.cuh"
 
 namespace ws {
 
@@ -280,6 +281,126 @@ static const std::vector<FastPencil>& fast_pencil_table() {
   return t;
 }
 
+// A pass of the run-time scheduled kernels (ws_uni.cuh).
+struct UniPass {
+  uni::Plan plan{};
+  int lines = 0;  // column pass: columns per block; pencils: consecutive y per block
+  int threads = 0;
+  size_t smem = 0;
+  long long grid = 0;  // blocks of a right-hand side
+};
+
+// The line's schedule: the fewest stages of radices 2 .. 16, of those the
+// smallest largest radix (registers), then the smallest sum; in ascending
+// order, so that the column pass's epilogue (stage 0) has the fewest elements
+// in registers.  False where the length has none (1, primes, factors above 16).
+static bool uni_plan(int n, uni::Plan& P) {
+  int best[uni::kStages] = {}, best_n = 0, best_max = 1 << 30, best_sum = 1 << 30;
+  int cur[uni::kStages];
+  auto search = [&](auto&& self, int left, int from, int k) -> void {
+    if (left == 1) {
+      if (k < 2) return;
+      int sum = 0;
+      for (int i = 0; i < k; ++i) sum += cur[i];
+      if (best_n && (k > best_n || (k == best_n && (cur[k - 1] > best_max || (cur[k - 1] == best_max && sum >= best_sum)))))
+        return;
+      best_n = k;
+      best_max = cur[k - 1];
+      best_sum = sum;
+      std::copy(cur, cur + k, best);
+      return;
+    }
+    if (k == uni::kStages) return;
+    for (int r = from; r <= 16 && r <= left; ++r)
+      if (left % r == 0) {
+        cur[k] = r;
+        self(self, left / r, r, k + 1);
+      }
+  };
+  search(search, n, 2, 0);
+  if (!best_n) return false;
+  P = uni::Plan{};
+  P.n = n;
+  P.nst = best_n;
+  P.cls = 0;
+  while (uni::kClassRadix[P.cls] < best_max) ++P.cls;
+  const int rl = best[best_n - 1];
+  P.pad = rl % 2 == 0 ? 1 : 0;
+  auto padded = [&](int i) { return i + (P.pad ? i / rl : 0); };
+  P.np = padded(n);
+  P.mrl = uni::magic(rl);
+  int block = n;
+  for (int s = 0; s < best_n; ++s) {
+    uni::Stage& S = P.st[s];
+    S.R = best[s];
+    S.sub = block / S.R;
+    S.units = n / S.R;
+    S.subp = padded(S.sub);
+    S.blkp = padded(block);
+    S.msub = uni::magic(S.sub);
+    S.munits = uni::magic(S.units);
+    block = S.sub;
+  }
+  return true;
+}
+
+// The frequency of each element of a forward transform in the order of T.
+static std::vector<int> uni_permutation(const uni::Plan& P) {
+  std::vector<int> k(P.n);
+  const uni::Stage& L = P.st[P.nst - 1];
+  for (int u = 0; u < L.units; ++u) {
+    int rev = 0, w = 1, rest = u, span = L.units;
+    for (int s = 0; s < P.nst - 1; ++s) {  // digit of stage s, the most significant first
+      span /= P.st[s].R;
+      rev += w * (rest / span);
+      rest %= span;
+      w *= P.st[s].R;
+    }
+    for (int i = 0; i < L.R; ++i) k[u + i * L.units] = rev + i * L.units;
+  }
+  return k;
+}
+
+static int uni_units(const uni::Plan& P) {
+  int m = 1;
+  for (int s = 0; s < P.nst; ++s) m = std::max(m, P.st[s].units);
+  return m;
+}
+
+// The column pass: one butterfly per thread, as many columns as fill 256 threads,
+// fewer where the grid would not give every SM two blocks, at least a warp.
+static void uni_columns(UniPass& p, long long total) {
+  const int um = uni_units(p.plan);
+  const long long most = std::max(1, uni::kMaxThreads / um), least = (32 + um - 1) / um;
+  long long l = std::min(most, std::max(least, total / (2 * kNumSms)));
+  while (l > 1 && l * p.plan.np * sizeof(float2) > 64 * 1024) l /= 2;
+  p.lines = (int)std::min(l, total);
+  p.threads = (int)std::min<long long>(uni::kMaxThreads, (p.lines * (long long)um + 31) / 32 * 32);
+  p.smem = p.lines * (p.plan.np * sizeof(float2) + 32);
+  p.grid = (total + p.lines - 1) / p.lines;
+}
+
+// Pencils: 16 consecutive y (one 128-byte row segment) per block, 8 where a
+// butterfly per thread would not fit 256 threads or the tile 72 KB (three
+// blocks per SM), down to 4 (one sector) where the grid would not give every
+// SM two blocks.  Measured at 150 x 80 x 198 (66 butterflies a line): 8 y with
+// two butterflies per thread 93 us an iteration, 4 y 105 us; at 512^2 4 y 21.8
+// us, 8 y (64 blocks) 24.8 us.
+static void uni_pencils(UniPass& p, int ny, int nc, long long mids) {
+  const int um = uni_units(p.plan);
+  const size_t row = (size_t)nc * p.plan.n * sizeof(float2);
+  int ty = 16;
+  while (ty > 8 && (ty * um > uni::kMaxThreads || ty * row > 72 * 1024)) ty /= 2;
+  while (ty > 4 && (ny + ty - 1) / ty * mids < 2 * kNumSms) ty /= 2;
+  while (ty > 1 && ty * row > 150 * 1024) ty /= 2;
+  p.lines = ty;
+  int w = std::max(1, std::min(um, uni::kMaxThreads / ty));
+  while ((w * ty) % 32 && w * ty + ty <= uni::kMaxThreads) ++w;
+  p.threads = w * ty;
+  p.smem = ty * row;
+  p.grid = (long long)((ny + ty - 1) / ty) * mids;
+}
+
 struct Layout {
   const FastInner* fi = nullptr;   // fast K1/K3, or null (generic)
   const FastPencil* fp = nullptr;  // fast K2, or null (generic)
@@ -293,6 +414,9 @@ struct Layout {
   int th_inner = 256, th_outer = 256;
   size_t smem_inner = 0, smem_outer = 0;
   long long grid_inner = 0, grid_outer = 0;
+  bool uni_in = false, uni_out = false;  // the run-time scheduled kernels for the inner / the outer pass
+  UniPass ucol, ux, uout;
+  long long pitch = 0;  // elements between the columns of T
 };
 
 static bool is_pow2(long long n) { return n >= 1 && (n & (n - 1)) == 0; }
@@ -312,8 +436,10 @@ struct LayoutChoice {
   }
 };
 
-static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutChoice& ch = LayoutChoice{}) {
+static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutChoice& ch = LayoutChoice{},
+                       bool pstd = false) {
   L = Layout{};
+  L.pitch = g.ny;
   L.mode3d = g.nz > 1;
   L.rset = kPow2;
   for (long long n : {(long long)g.ny, (long long)g.nx, (long long)g.nz})
@@ -461,6 +587,25 @@ static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutC
         }
     }
   }
+  // lengths without a compile-time schedule: the run-time scheduled kernels
+  // (3-6 times the generic ones' speed at 2-D and 3-D grids of 45 to 1100
+  // points a side, see ws_uni.cuh), unless the generic ones are asked for.  T is then in digit-reversed order
+  // along the lines that those kernels transform: along the outer dimension
+  // for every pairing, along y and x only if they run both passes.  (PSTD
+  // feeds T through K1 a second time, which needs natural order there.)
+  L.uni_out = !L.tp && !L.fp && ch.outer != 2 && uni_plan(no, L.uout.plan);
+  if (L.uni_out) {
+    uni_pencils(L.uout, g.ny, g.nc, mids);
+    L.grid_outer = L.uout.grid;
+  }
+  L.uni_in = L.uni_out && !L.fi && !pstd && ch.inner != 2 && !ch.csize && !ch.ncols && !ch.sched &&
+             uni_plan(g.ny, L.ucol.plan) && (!L.mode3d || uni_plan(g.nx, L.ux.plan));
+  if (L.uni_in) {
+    uni_columns(L.ucol, (long long)g.nx * g.nz * g.nc);
+    if (L.mode3d) uni_pencils(L.ux, g.ny, 1, (long long)g.nz * g.nc);
+    L.grid_inner = L.ucol.grid;
+    L.pitch = (g.ny + 3) / 4 * 4;
+  }
   return WS_OK;
 }
 
@@ -537,6 +682,10 @@ struct Solver {
                                  // dependent launch (measured: 256^3 solve 46.3 against 44.3 ms,
                                  // 96^3 3.38 against 2.80 ms, 1024^2 8.50 against 8.71 ms; off)
   float2* d_tw = nullptr;
+  float2* d_utw = nullptr;       // run-time scheduled kernels: twiddles, then
+  int* d_uperm = nullptr;        //   the permutation of the p tables and
+  float* d_uwigf = nullptr;      //   the wiggles' p tables in the order of T
+  std::vector<Wig> uwig;
   FftPlan py{}, pxl{}, po{};
   const float2* twx = nullptr;
   cudaGraph_t graph = nullptr;
@@ -558,7 +707,7 @@ static void update_fuse(Solver* s) {
   const char* e = std::getenv("WAVESIM_B200_FUSE");
   const bool on3 = s->lay.fi && (s->lay.fi->fused || s->lay.xp) && s->lay.mode3d;
   const bool on2 = s->lay.fi && !s->lay.mode3d && s->lay.fi->col_step;  // 2-D: K2 + the column pass
-  const int f = ((on3 || on2) && !s->pstd && !(e && std::strcmp(e, "0") == 0)) ? 1 : 0;
+  const int f = ((on3 || on2 || s->lay.uni_in) && !s->pstd && !(e && std::strcmp(e, "0") == 0)) ? 1 : 0;
   if (f != s->fuse) free_graph(s);
   s->fuse = f;
 }
@@ -569,7 +718,7 @@ static void destroy_solver(Solver* s) {
   free_graph(s);
   void* ptrs[] = {s->d_wigf, s->d_wigc,  s->d_gamma,  s->d_E,        s->d_dE, s->d_T,   s->d_src,
                   s->d_stage, s->d_out, s->d_state, s->d_hist, s->d_energy, s->d_tw, s->d_partials, s->d_init,
-                  s->d_err};
+                  s->d_err, s->d_utw};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& e : s->ev)
@@ -642,6 +791,12 @@ static int set_kernel_attributes() {
   }
   for (const FastPencil& f : fast_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (const TmaPencil& f : tma_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
+  for (int c = 0; c < uni::kClasses; ++c) {
+    const uni::Kernels& k = uni::kernels(c);
+    for (const void* f : k.col) WS_CUDA(allow_dynamic_smem(f, optin));
+    for (const void* f : k.x) WS_CUDA(allow_dynamic_smem(f, optin));
+    for (const void* f : k.pencil) WS_CUDA(allow_dynamic_smem(f, optin));
+  }
   for (const XPencil& f : x_pencil_table()) {
     WS_CUDA(allow_dynamic_smem(f.fwd, optin));
     WS_CUDA(allow_dynamic_smem(f.inv, optin));
@@ -681,6 +836,76 @@ static int check_args(const int64_t N[4], int64_t n_wiggles, const ws_wiggle* wi
 static cudaMemcpyKind kind_from(int memory) { return memory == WS_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice; }
 
 static size_t field_elems(const Solver* s) { return (size_t)s->g.npts * s->g.nc; }
+// T of one right-hand side: allocated for a y pitch of whole sectors, used with the layout's
+static size_t t_alloc_elems(const Solver* s) { return (size_t)((s->g.ny + 3) / 4 * 4) * s->g.nx * s->g.nz * s->g.nc; }
+static long long t_stride(const Solver* s) { return s->lay.pitch * s->g.nx * s->g.nz * s->g.nc; }
+
+// The wiggles' p tables in the order in which the layout's run-time scheduled
+// plans leave T (natural along the axes that other kernels transform):
+// per[w][i] = nat[w][perm[i]].
+static __global__ void k_permute_tables(float* __restrict__ per, const float* __restrict__ nat,
+                                        const int* __restrict__ perm, int nf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nf) per[(long long)blockIdx.y * nf + i] = nat[(long long)blockIdx.y * nf + perm[i]];
+}
+static cudaError_t permute_wiggles(Solver* s) {
+  if (!s->lay.uni_out) return cudaSuccess;
+  cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);  // the tables' uploads
+  if (e != cudaSuccess) return e;
+  const int nf = s->g.nx + s->g.ny + s->g.nz;
+  k_permute_tables<<<dim3((nf + 255) / 256, s->nw), 256, 0, s->stream>>>(s->d_uwigf, s->d_wigf, s->d_uperm, nf);
+  return cudaGetLastError();
+}
+
+// The device tables of the layout's run-time scheduled plans, in one buffer:
+// twiddles, the permutation of the p tables, the permuted p tables.
+static cudaError_t ensure_uni(Solver* s) {
+  Layout& L = s->lay;
+  if (!L.uni_out) return cudaSuccess;
+  const Geom& g = s->g;
+  const int len[3] = {g.nx, g.ny, g.nz};  // the order of d_wigf
+  const uni::Plan* axis[3] = {L.mode3d ? (L.uni_in ? &L.ux.plan : nullptr) : &L.uout.plan,
+                              L.uni_in ? &L.ucol.plan : nullptr, L.mode3d ? &L.uout.plan : nullptr};
+  std::vector<float2> tw;
+  std::vector<std::pair<uni::Stage*, size_t>> at;
+  for (UniPass* p : {&L.ucol, &L.ux, &L.uout})
+    for (int k = 0; k < p->plan.nst; ++k) {
+      uni::Stage& S = p->plan.st[k];
+      at.push_back({&S, tw.size()});
+      const int n = S.R * S.sub;
+      for (int r = 0; r < S.R; ++r)
+        for (int j = 0; j < S.sub; ++j) {
+          const double a = -2.0 * M_PI * (double)((long long)j * r % n) / (double)n;
+          tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+        }
+    }
+  std::vector<int> perm;
+  for (int d = 0; d < 3; ++d) {
+    const int off = (int)perm.size();
+    const std::vector<int> k = axis[d] ? uni_permutation(*axis[d]) : std::vector<int>();
+    for (int i = 0; i < len[d]; ++i) perm.push_back(off + (axis[d] ? k[i] : i));
+  }
+  const size_t twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
+  if (s->d_utw) cudaFree(s->d_utw);
+  s->d_utw = nullptr;
+  cudaError_t e = cudaMalloc(&s->d_utw, twb + pb * (1 + s->nw));
+  if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_utw, tw.data(), twb, cudaMemcpyHostToDevice, s->stream);
+  s->d_uperm = reinterpret_cast<int*>(reinterpret_cast<char*>(s->d_utw) + twb);
+  s->d_uwigf = reinterpret_cast<float*>(reinterpret_cast<char*>(s->d_uperm) + pb);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_uperm, perm.data(), pb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = permute_wiggles(s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // tw and perm end here
+  if (e != cudaSuccess) return e;
+  for (auto& a : at) a.first->tw = s->d_utw + a.second;
+  s->uwig = s->wig;
+  for (int w = 0; w < s->nw; ++w) {
+    const float* f = s->d_uwigf + perm.size() * w;
+    s->uwig[w].pxe = f;
+    s->uwig[w].pye = f + g.nx;
+    s->uwig[w].pze = f + g.nx + g.ny;
+  }
+  return cudaSuccess;
+}
 
 // Buffers for nrhs right-hand sides (kept when large enough).
 // d_partials holds at least n per-block energies (graphs hold the old pointer)
@@ -711,7 +936,7 @@ static int ensure_batch(Solver* s, int nrhs) {
   const size_t nb = field_elems(s) * nrhs * sizeof(float2);
   WS_CUDA(cudaMalloc(&s->d_E, nb));
   WS_CUDA(cudaMalloc(&s->d_dE, nb));
-  WS_CUDA(cudaMalloc(&s->d_T, nb));
+  WS_CUDA(cudaMalloc(&s->d_T, t_alloc_elems(s) * nrhs * sizeof(float2)));
   WS_CUDA(cudaMalloc(&s->d_src, nb));
   WS_CUDA(cudaMalloc(&s->d_state, nrhs * sizeof(DevState)));
   WS_CUDA(cudaMalloc(&s->d_energy, nrhs * sizeof(double)));
@@ -725,7 +950,8 @@ static int ensure_batch(Solver* s, int nrhs) {
 }
 
 static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_wiggles, const ws_wiggle* wiggles,
-                         float epsilon, ws_complex k02e, const int64_t roi[8], int memory, int device, Solver** out) {
+                         float epsilon, ws_complex k02e, const int64_t roi[8], int memory, int device, Solver** out,
+                         bool pstd = false) {
   Geom g{};
   int rc = check_args(N, n_wiggles, wiggles, gamma, roi, g);
   if (rc) return rc;
@@ -742,7 +968,8 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
   s->eps = epsilon;
   s->k02e = make_float2(k02e.re, k02e.im);
   std::string why;
-  rc = make_layout(g, s->lay, why);
+  s->pstd = pstd ? 1 : 0;
+  rc = make_layout(g, s->lay, why, LayoutChoice{}, pstd);
   if (rc) {
     destroy_solver(s);
     return fail(rc, why);
@@ -813,6 +1040,7 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     WS_TRY(cudaMemcpy(c + g.nx + g.ny, W.gz, g.nz * sizeof(float2), kind));
     s->wig.push_back(Wig{f, f + g.nx, f + g.nx + g.ny, c, c + g.nx, c + g.nx + g.ny});
   }
+  WS_TRY(ensure_uni(s));
   WS_TRY(cudaMalloc(&s->d_gamma, (size_t)g.npts * sizeof(float2)));
   WS_TRY(cudaMemcpy(s->d_gamma, gamma, (size_t)g.npts * sizeof(float2), kind));
 #undef WS_TRY
@@ -848,6 +1076,7 @@ static int reload_medium(Solver* s, const int64_t N[4], const ws_complex* gamma,
     WS_CUDA(cudaMemcpy(c + g.nx, W.gy, g.ny * sizeof(float2), kind));
     WS_CUDA(cudaMemcpy(c + g.nx + g.ny, W.gz, g.nz * sizeof(float2), kind));
   }
+  WS_CUDA(permute_wiggles(s));
   WS_CUDA(cudaMemcpy(s->d_gamma, gamma, (size_t)g.npts * sizeof(float2), kind));
   const float2 k = make_float2(k02e.re, k02e.im);
   bool same = s->eps == epsilon && s->k02e.x == k.x && s->k02e.y == k.y;
@@ -983,12 +1212,100 @@ static cudaError_t launch_pdl(const Solver* s, const void* fn, dim3 grid, dim3 b
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+// The passes of the run-time scheduled kernels (ws_uni.cuh).
+static cudaError_t launch_uni(const Solver* s, const void* fn, const UniPass& p, void* args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(p.grid * s->nrhs));
+  cfg.blockDim = dim3(p.threads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = s->stream;
+  void* argv[] = {args};
+  return cudaLaunchKernelExC(&cfg, fn, argv);
+}
+
+// mode kFwd: K1's column transforms of `in`; kInv: K3's; kStep: K3 with
+// wiggle w and K1 of the next iteration with wiggle w1
+static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, const float2* in, const float2* src,
+                                  float2* T, float a_mult) {
+  const UniPass& p = s->lay.ucol;
+  uni::ColArgs a{};
+  a.g = s->g;
+  a.py = p.plan;
+  a.gx = s->wig[w].gx;
+  a.gy = s->wig[w].gy;
+  a.gz = s->wig[w].gz;
+  a.gx1 = s->wig[w1].gx;
+  a.gy1 = s->wig[w1].gy;
+  a.gz1 = s->wig[w1].gz;
+  a.dE_in = in;
+  a.src = src;
+  a.A = make_float2(0.f, a_mult * (float)(1.0f / s->eps / (float)s->nw));  // 1i/epsilon/Nwiggles
+  a.T = T;
+  a.dE = s->d_dE;
+  a.E = s->d_E;
+  a.gamma = s->d_gamma;
+  a.st = s->d_state;
+  a.partials = s->d_partials;
+  a.pitch = s->lay.pitch;
+  a.fstride = (long long)field_elems(s);
+  a.tstride = t_stride(s);
+  a.gstride = s->n_media > 1 ? (long long)s->g.npts : 0;
+  a.total = s->g.nx * s->g.nz * s->g.nc;
+  a.lines = p.lines;
+  a.bpr = (int)p.grid;
+  a.acc2 = (s->nw % 2 == 0) ? 1 : 0;
+  return launch_uni(s, uni::kernels(p.plan.cls).col[mode], p, &a);
+}
+
+static cudaError_t launch_uni_x(const Solver* s, bool inv, float2* T) {
+  const UniPass& p = s->lay.ux;
+  uni::XArgs a{};
+  a.px = p.plan;
+  a.T = T;
+  a.st = s->d_state;
+  a.pitch = s->lay.pitch;
+  a.tstride = t_stride(s);
+  a.ny = s->g.ny;
+  a.nx = s->g.nx;
+  a.ty = p.lines;
+  a.nyt = (s->g.ny + p.lines - 1) / p.lines;
+  a.bpr = (int)p.grid;
+  return launch_uni(s, uni::kernels(p.plan.cls).x[inv ? 1 : 0], p, &a);
+}
+
+static cudaError_t launch_uni_k2(const Solver* s, int w) {
+  const UniPass& p = s->lay.uout;
+  uni::PencilArgs a{};
+  a.g = s->g;
+  a.po = p.plan;
+  a.w = s->uwig[w];
+  a.k02e = s->k02e;
+  const double kk = (double)s->k02e.x * s->k02e.x + (double)s->k02e.y * s->k02e.y;
+  if (kk > 0) a.ik02e = make_float2((float)(s->k02e.x / kk), (float)(-s->k02e.y / kk));
+  a.norm = (float)(1.0 / ((double)s->g.npts));
+  a.T = s->d_T;
+  a.st = s->d_state;
+  a.pitch = s->lay.pitch;
+  a.tstride = t_stride(s);
+  a.cstride = s->lay.pitch * s->g.nx * s->g.nz;
+  a.ty = p.lines;
+  a.nyt = (s->g.ny + p.lines - 1) / p.lines;
+  a.bpr = (int)p.grid;
+  a.mode3d = s->lay.mode3d;
+  a.pstd = s->pstd;
+  return launch_uni(s, uni::kernels(p.plan.cls).pencil[s->g.nc == 3 ? 1 : 0], p, &a);
+}
+
 // K1 on explicit buffers: out = inner FFT of (in + a_mult A src) times the
 // ramps of wiggle w (A = i/epsilon/Nw, the reference's per-iteration share of
 // the source; a_mult = Nw gives the whole source, for the warm start's
 // residual probe)
 static cudaError_t launch_k1_io(const Solver* s, int w, const float2* in, const float2* src, float2* out,
                                 float a_mult = 1.f) {
+  if (s->lay.uni_in) {
+    cudaError_t e = launch_uni_col(s, uni::kFwd, w, w, in, src, out, a_mult);
+    return e != cudaSuccess || !s->lay.mode3d ? e : launch_uni_x(s, false, out);
+  }
   if (s->lay.fi) {
     InnerArgs a = inner_args(s, w);
     a.ncols = s->lay.ncols;
@@ -1077,10 +1394,15 @@ static cudaError_t launch_k2(const Solver* s, int w) {
     void* args[] = {&a, &T, &st};
     return launch_pdl(s, f->fn, dim3(grid), dim3(f->threads), args, f->smem);
   }
+  if (s->lay.uni_out) return launch_uni_k2(s, w);
   return s->lay.rset == kPow2 ? launch_k2_t<kPow2>(s, w) : launch_k2_t<kMixed>(s, w);
 }
 static cudaError_t launch_k3_only(const Solver* s, int w) {
   cudaError_t e;
+  if (s->lay.uni_in) {
+    if (s->lay.mode3d && (e = launch_uni_x(s, true, s->d_T)) != cudaSuccess) return e;
+    return launch_uni_col(s, uni::kInv, w, w, nullptr, nullptr, s->d_T, 1.f);
+  }
   if (s->lay.fi) {
     InnerArgs a = inner_args(s, w);
     a.ncols = s->lay.ncols;
@@ -1261,6 +1583,12 @@ static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next,
 // split step (inverse x pencils, column pass, forward x pencils).
 static cudaError_t launch_step(const Solver* s, int w, int w1, bool src_next, const StopRule* rule = nullptr,
                                const Hist* h = nullptr) {
+  if (s->lay.uni_in) {
+    cudaError_t e = s->lay.mode3d ? launch_uni_x(s, true, s->d_T) : cudaSuccess;
+    if (e != cudaSuccess) return e;
+    e = launch_uni_col(s, uni::kStep, w, w1, nullptr, src_next ? s->d_src : nullptr, s->d_T, 1.f);
+    return e != cudaSuccess || !s->lay.mode3d ? e : launch_uni_x(s, false, s->d_T);
+  }
   if (!s->lay.mode3d) return launch_colstep(s, w, w1, src_next, rule, h);  // 2-D: K2 already transformed along x
   if (!s->lay.xp) return launch_k3k1(s, w, w1, src_next);
   cudaError_t e = launch_xpencil(s, true);
@@ -1271,7 +1599,9 @@ static cudaError_t launch_step(const Solver* s, int w, int w1, bool src_next, co
 
 // Whether the loop's column pass runs the stop rule itself (2-D, or the
 // split step of 3-D planes; WAVESIM_B200_FIN=1).
-static bool finish_in_step(const Solver* s) { return s->fin_fuse && (!s->lay.mode3d || s->lay.xp); }
+static bool finish_in_step(const Solver* s) {
+  return s->fin_fuse && !s->lay.uni_in && (!s->lay.mode3d || s->lay.xp);
+}
 
 // One iteration of the fused loop: T already holds K1's output for it.
 static cudaError_t launch_iteration_fused(const Solver* s, int i, bool src_next, const StopRule& rule,
@@ -1836,7 +2166,7 @@ int ws_solver_launches_per_iteration(ws_solver h) {
   const Solver* s = reinterpret_cast<Solver*>(h);
   // K2, K3 + next K1 (one kernel, or the split step's three), stop rule; or K1, K2, K3, stop rule
   if (!s->fuse) return 4;                                   // K1, K2, K3, the stop rule
-  if (s->lay.mode3d && !s->lay.xp) return 3;                // K2, K3K1 on a cluster, the stop rule
+  if (s->lay.mode3d && !s->lay.xp && !s->lay.uni_in) return 3;  // K2, K3K1 on a cluster, the stop rule
   const int step = s->lay.mode3d ? 4 : 2;                   // K2 (+ x pencils), the column pass (+ x pencils)
   return finish_in_step(s) ? step : step + 1;
 }
@@ -1879,7 +2209,7 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
     const double n = (double)s->g.npts * s->g.nc;
     // K3's bytes (as ws_solver_time_kernels) plus the write of T for the next
     // iteration; the split step also reads and writes T in each x pass
-    *bytes_out = (s->nw % 2 == 0 ? 40.0 : 48.0) * n + 8.0 * (double)s->g.npts + (s->lay.xp ? 32.0 * n : 0.0);
+    *bytes_out = (s->nw % 2 == 0 ? 40.0 : 48.0) * n + 8.0 * (double)s->g.npts + (s->lay.mode3d && (s->lay.xp || s->lay.uni_in) ? 32.0 * n : 0.0);
   }
   return WS_OK;
 }
@@ -1887,7 +2217,7 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
 int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double bytes_out[3]) {
   if (!h || !ms_out || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
-  if (!s->fuse || !s->lay.xp) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
+  if (!s->fuse || !s->lay.mode3d || !(s->lay.xp || s->lay.uni_in)) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
   WS_CUDA(cudaSetDevice(s->device));
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
@@ -1904,11 +2234,12 @@ int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double 
     const int w = i % s->nw;
     WS_CUDA(launch_k2(s, w));
     WS_CUDA(cudaEventRecord(s->ev[0], s->stream));
-    WS_CUDA(launch_xpencil(s, true));
+    WS_CUDA(s->lay.uni_in ? launch_uni_x(s, true, s->d_T) : launch_xpencil(s, true));
     WS_CUDA(cudaEventRecord(s->ev[1], s->stream));
-    WS_CUDA(launch_colstep(s, w, (i + 1) % s->nw, false));
+    WS_CUDA(s->lay.uni_in ? launch_uni_col(s, uni::kStep, w, (i + 1) % s->nw, nullptr, nullptr, s->d_T, 1.f)
+                          : launch_colstep(s, w, (i + 1) % s->nw, false));
     WS_CUDA(cudaEventRecord(s->ev[2], s->stream));
-    WS_CUDA(launch_xpencil(s, false));
+    WS_CUDA(s->lay.uni_in ? launch_uni_x(s, false, s->d_T) : launch_xpencil(s, false));
     WS_CUDA(cudaEventRecord(s->ev[3], s->stream));
     WS_CUDA(launch_finish(s, rule, hh));
     WS_CUDA(cudaEventSynchronize(s->ev[3]));
@@ -2118,13 +2449,14 @@ static void apply_sched(Solver* s, int sched) {
 static bool apply_choice(Solver* s, const LayoutChoice& c) {
   Layout L;
   std::string why;
-  if (make_layout(s->g, L, why, c) != WS_OK) return false;
+  if (make_layout(s->g, L, why, c, s->pstd != 0) != WS_OK) return false;
   // the generic 3-D kernels transform x-local lines of Nx / csize points with
   // the plan and twiddles made for the solver's first layout: a layout with
   // another cluster size would run them on lines of another length
-  if (L.mode3d && !L.fi && s->g.nx / L.csize != s->pxl.n) return false;
+  if (L.mode3d && !L.fi && !L.uni_in && s->g.nx / L.csize != s->pxl.n) return false;
   if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap)) != WS_OK) return false;
   s->lay = L;
+  if (ensure_uni(s) != cudaSuccess) return false;
   apply_sched(s, c.sched);
   update_fuse(s);
   free_graph(s);
@@ -2515,14 +2847,12 @@ int ws_pstd_create(const int64_t N[3], const float* c1, const float* c2, const f
               (const ws_complex*)one.data()};
   Pstd* p = new Pstd();
   int rc = create_solver(N4, (const ws_complex*)c12.data(), 1, &w, 1.0f, ws_complex{0.f, 0.f}, roi, WS_HOST, device,
-                         &p->s);
+                         &p->s, true);
   if (rc) {
     delete p;
     return rc;
   }
   Solver* s = p->s;
-  s->pstd = 1;
-  s->fuse = 0;
   p->nparts = (int)std::min<long long>(((long long)npts + 255) / 256, 8LL * kNumSms);
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = cudaMalloc(&p->d_Ebuf, 2 * npts * sizeof(float2));

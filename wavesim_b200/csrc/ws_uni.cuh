@@ -1,0 +1,128 @@
+// Loop kernels for line lengths without a compile-time schedule of their own
+// (any length that factors into two to four radices of at most 16): the same
+// passes as the split step (column pass, x pencils, outer pencils), with the
+// schedule chosen at run time and every radix's butterfly compiled once.
+//
+// A line of N = R0 R1 .. RS-1 points is transformed in place by decimation in
+// frequency: stage s splits each block of n_s = N / (R0 .. Rs-1) elements
+// into butterflies {j + r sub}, sub = n_s / R_s, and multiplies output r by
+// W_{n_s}^{j r}.  Forward transforms go from natural order to digit-reversed
+// order, inverse transforms run the stages backwards (conjugate twiddles
+// first, then the butterfly) from digit-reversed to natural order.  A thread
+// takes one butterfly at a time: it reads and writes the same R elements, so
+// a stage needs one barrier, no second buffer, and R complex registers
+// whatever N is.  Two consequences shape the passes:
+//
+// * The spectrum never needs its natural order: only the Green's function
+//   looks at k, through tables of p that are permuted once when the solver is
+//   made (uni_permutation).  In global memory, element i of the last stage's
+//   butterfly u sits at u + i N / RS-1, so that consecutive threads touch
+//   consecutive elements; a pass therefore starts with the last stage
+//   straight from global memory, or ends with it straight into it.
+// * Where an inverse transform is followed by a forward one (the column pass:
+//   inverse y, f_mix, forward y; the outer pencils: forward, Green's function,
+//   inverse), the last stage of the first and the first stage of the second
+//   are the same butterfly on the same elements and stay in registers.  A
+//   two-stage line crosses shared memory twice in the whole pass.
+//
+// T has its y pitch rounded up to 4 elements (one 32-byte sector), so that
+// the pencils' rows start on sectors for odd Ny too.
+//
+// Measured against the generic three-pass kernels (ws_kernels.cuh), which
+// hold every radix inlined with all of a thread's elements in local memory
+// (1.3-3.7 KB a thread), device time of one iteration: 125 x 144 x 99 64 us
+// against 361, 210 x 189 x 216 334 against 2311, 1100 x 768 40 against 102,
+// 63 x 77 x 70 x 3 52 against 138, 105 x 120 x 63 x 3 85 against 490.  Grids
+// whose passes fit the L2 are bound by the latency of a pass (load, two
+// butterflies, store) and the launches; larger ones by memory, at 2-3 times
+// the bytes' time.  The compile-time schedules stay where they exist: 192^3
+// takes 153 us with them and 232 with these.
+#pragma once
+#include "ws_kernels.cuh"
+
+namespace ws {
+namespace uni {
+
+constexpr int kStages = 4;
+constexpr int kMaxThreads = 256;
+
+struct Stage {
+  int R;           // radix
+  int sub;         // distance between the elements of a butterfly; twiddles W^{j r}, j < sub, at tw[r sub + j]
+  int units;       // butterflies of a line: n / R
+  int subp, blkp;  // sub and the block R sub in a padded column (Plan::pad)
+  unsigned msub, munits;  // multipliers of the division by sub and units (magic)
+  const float2* tw;
+};
+
+struct Plan {
+  int n, nst;
+  int cls;       // kernels (kClassRadix) that its radices need
+  int pad;       // columns: one slot of padding after every last-stage butterfly (its radix even), else 0
+  int np;        // elements of a padded column
+  unsigned mrl;  // multiplier of the division by the last stage's radix
+  Stage st[kStages];
+};
+
+// a / d for 0 <= a < 65536 from m = magic(d)
+__host__ __device__ constexpr unsigned magic(int d) {
+  return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / (unsigned)d);
+}
+__device__ __forceinline__ int quot(int a, unsigned m) { return m ? (int)__umulhi((unsigned)a, m) : a; }
+
+struct ColArgs {
+  Geom g;
+  Plan py;
+  const float2 *gx, *gy, *gz;     // ramps of this iteration's wiggle (its conjugate ramps)
+  const float2 *gx1, *gy1, *gz1;  // ramps applied before the forward transform
+  const float2* dE_in;            // forward pass: the field to transform
+  const float2* src;              // added with weight A before the forward transform, or null
+  float2 A;
+  float2 *T, *dE, *E;
+  const float2* gamma;
+  const DevState* st;
+  double* partials;
+  long long pitch;    // T: elements between columns
+  long long fstride;  // fields: elements between right-hand sides
+  long long tstride;  // T: elements between right-hand sides
+  long long gstride;
+  int total;          // columns of a right-hand side
+  int lines;          // columns per block
+  int bpr;            // blocks per right-hand side
+  int acc2;
+};
+
+struct PencilArgs {
+  Geom g;
+  Plan po;
+  Wig w;  // p tables in the order of T
+  float2 k02e, ik02e;  // k0^2 e + i e and its inverse
+  float norm;
+  float2* T;
+  const DevState* st;
+  long long pitch, tstride, cstride;  // cstride: elements between the components of T
+  int ty, nyt, bpr, mode3d, pstd;
+};
+
+struct XArgs {
+  Plan px;
+  float2* T;
+  const DevState* st;
+  long long pitch, tstride;
+  int ny, nx, ty, nyt, bpr;
+};
+
+enum { kFwd = 0, kInv = 1, kStep = 2 };
+
+// the kernels compiled for radices up to kClassRadix[c]
+constexpr int kClasses = 3;
+constexpr int kClassRadix[kClasses] = {8, 12, 16};
+struct Kernels {
+  const void* col[3];     // by kFwd, kInv, kStep
+  const void* x[2];       // forward, inverse
+  const void* pencil[2];  // one component, three
+};
+const Kernels& kernels(int cls);
+
+}  // namespace uni
+}  // namespace ws
