@@ -321,8 +321,8 @@ def run_ours(args):
     value = total_ms / (args.steps * ws)
     n_iter = iters[-1]
     # K1, K2, K3 (or K2 and K3 fused with the next K1, plus one K1 per solve)
-    # and the stop-rule kernel per iteration, the cycle guard per wiggle
-    # cycle, state reset, source scatter, finalize
+    # per iteration, the stop rule with the cycle guard per wiggle cycle,
+    # state reset, source scatter, finalize
     per_it = _lib.lib.ws_solver_launches_per_iteration(h)
     fused = _lib.lib.ws_solver_fused(h) == 1
     launches_per_solve = (per_it * n_iter + (n_iter // len(sim.wiggles)) + 1 + len(s.values) + 1

@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, C >= 16 ? 3 : 2)
   st += rhs;
   if (load_done(st)) return;
   // with a.acc2, E' takes dE'_{k-1} + dE'_k after even iterations k only
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;  // the same for every block of a cluster
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;  // the same for every block of a cluster
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -1124,7 +1124,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = rb / a.bpr, bid = rb - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -1236,7 +1236,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (tid == 0) partials[bid] = (double)v;
   }
-  if (a.fin) finish_in_last_block(const_cast<DevState*>(st), a.rule, a.hist, partials, a.bpr, rhs);
 }
 
 // The 2-D form: K2 already transforms along x, so K3 of iteration k and K1
@@ -1262,7 +1261,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -1367,7 +1366,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (tid == 0) partials[bid] = (double)v;
   }
-  if (a.fin) finish_in_last_block(const_cast<DevState*>(st), a.rule, a.hist, partials, a.bpr, rhs);
 }
 
 // The same fused step with K1's half of the plane exchange pushed: each block
@@ -1399,7 +1397,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;  // the same for every block of a cluster
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;

@@ -57,7 +57,6 @@ struct DevState {
   int converged;    // state.converged
   int calc_energy;  // state.calculate_energy
   int status;       // 0 or WS_ERR_DIVERGED
-  unsigned int blocks_done;
   long long cycles;  // wiggle cycles completed (loop guard)
   double e_acc;             // partial sums of this iteration's ROI energy
   double last_step_energy;  // state.last_step_energy
@@ -85,6 +84,11 @@ struct Hist {
   long long stride;  // distance between the histories of consecutive right-hand sides
 };
 
+// E' += dE': every iteration, or in pairs (Nw even: every stop falls after an
+// even iteration), skipped after odd iterations and dE'_{k-1} + dE'_k added
+// after even ones (dE'_{k-1} is read anyway for f_mix).
+enum { kAccEach = 0, kAccPair = 1, kAccSkip = 2 };
+
 struct InnerArgs {
   Geom g;
   Wig w;
@@ -97,12 +101,9 @@ struct InnerArgs {
   int bpr;      // blocks per right-hand side (a batch of sources runs as consecutive block ranges)
   long long fstride;  // elements between the fields of consecutive right-hand sides
   int pf;       // fast kernels: block b pulls the inputs of block b + pf into L2 (0: off)
-  int acc2;     // K3: E' += dE' in pairs, every second iteration (Nw even; 0: every iteration)
+  int acc2;     // K3: what E' takes in this iteration (kAccEach ..)
   int* err;     // fast kernels: set to 1 when a cluster exchange wait gives up (may be null)
   long long gstride;  // elements between the gammas of consecutive right-hand sides (0: one shared gamma)
-  int fin;            // column passes: the last block of a right-hand side runs the stop rule
-  StopRule rule;      //   (finish_in_last_block) with this rule and history
-  Hist hist;
 };
 
 struct OuterArgs {
@@ -314,8 +315,8 @@ __global__ void __launch_bounds__(512, 1) k_outer(OuterArgs a, float2* __restric
   }
 }
 
-// Simulation.next (Simulation.m:193-217), run by one thread after the energy
-// of iteration st->it is complete.
+// Simulation.next (Simulation.m:193-217), run by one thread on the energy
+// st->e_acc of iteration st->it.
 __device__ __forceinline__ void finish_iteration(DevState* st, const StopRule& rule, const Hist& h) {
   const double e = st->e_acc;
   st->e_acc = 0.0;
@@ -341,41 +342,6 @@ __device__ __forceinline__ void finish_iteration(DevState* st, const StopRule& r
   }
   st->calc_energy = ((it - 1) % rule.interval) == 0;
   st->it = it + 1;
-  st->blocks_done = 0;
-}
-
-// The stop rule of an iteration run by the last block (of 256 threads) of
-// the pass that wrote the iteration's energy partials, instead of a separate
-// k_finish_iteration launch: each block counts itself in st->blocks_done
-// after its partial is visible; the block that completes the count (all
-// others have then finished, and read st->it before it changes) sums the
-// partials in k_finish_iteration's order (thread i takes i, i + 256, ...,
-// then the same tree) and runs finish_iteration, which clears the count.
-// st and partials are those of the block's right-hand side.
-__device__ __forceinline__ void finish_in_last_block(DevState* st, const StopRule& rule, Hist h,
-                                                    const double* partials, int nparts, int rhs) {
-  __shared__ unsigned s_last;
-  __shared__ double red[256];
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(&st->blocks_done, 1u) == (unsigned)(nparts - 1) ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  h.diff += rhs * h.stride;
-  if (h.fresh) h.fresh += rhs * h.stride;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += __ldcg(&partials[i]);
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    st->e_acc = red[0];
-    finish_iteration(st, rule, h);
-  }
 }
 
 // K3 -------------------------------------------------------------------------
@@ -386,8 +352,7 @@ __global__ void __launch_bounds__(512, 1) k_inv_inner(InnerArgs a, const float2*
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;
-  // with a.acc2, E' takes dE'_{k-1} + dE'_k after even iterations k only
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -475,30 +440,75 @@ __global__ void __launch_bounds__(512, 1) k_inv_inner(InnerArgs a, const float2*
   }
 }
 
-// The stop rule after each iteration: sums the per-block ROI energies of K3 in
-// a fixed order (so the energy history is reproducible bit for bit) and runs
-// Simulation.next (Simulation.m:193-217).  One block.
-static __global__ void __launch_bounds__(256) k_finish_iteration(DevState* st, StopRule rule, Hist h,
-                                                          const double* __restrict__ partials, int nparts) {
+// The stop rule of the iterations of a wiggle cycle (or of fewer): sums the
+// per-block ROI energies of K3 in a fixed order (so the energy history is
+// reproducible bit for bit) and runs Simulation.next (Simulation.m:193-217)
+// for one iteration after the other.  A solve can only stop at a multiple of
+// Nw, so nothing between two iterations of a cycle waits for their energies;
+// one launch per cycle replaces one per iteration, 2-4 us each (512^2 21.4 ->
+// 19.5 us an iteration, 96^3 32.1 -> 29.5, 125 x 144 x 99 64 -> 60, 256^3 286 ->
+// 284).  (An energy that is not finite
+// ends the history at its iteration and the solve with the cycle.)
+//
+// One block per right-hand side; 256 threads sum one iteration's nparts
+// partials (slot k at partials + k slot_stride), four iterations at a time.
+// With `guard` (one right-hand side) the kernel is also the cycle's guard
+// (k_cycle_guard).
+struct CycleGuard {
+  int on;
+  cudaGraphConditionalHandle cond;
+  long long max_cycles;
+};
+__device__ __forceinline__ void cycle_guard(DevState* st, int n, const CycleGuard& g) {
+  const long long c = ++st->cycles;
+  bool any = false;
+  for (int i = 0; i < n; ++i) any |= !st[i].done;
+  const bool go = any && c < g.max_cycles;
+  if (!go)
+    for (int i = 0; i < n; ++i) st[i].done = 1;
+  cudaGraphSetConditional(g.cond, go ? 1u : 0u);
+}
+
+constexpr int kMaxWiggles = 64;
+static __global__ void __launch_bounds__(1024) k_finish_iterations(DevState* st, StopRule rule, Hist h,
+                                                                   const double* __restrict__ partials, int nparts,
+                                                                   long long slot_stride, int slots, CycleGuard guard) {
   pdl_begin();
-  const int rhs = blockIdx.x;  // one block per right-hand side
+  const int rhs = blockIdx.x;
   st += rhs;
   partials += (long long)rhs * nparts;
   h.diff += rhs * h.stride;
   if (h.fresh) h.fresh += rhs * h.stride;
-  if (load_done(st)) return;
-  __shared__ double red[256];
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) acc += partials[i];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
+  __shared__ double red[4][256];
+  __shared__ double energy[kMaxWiggles];
+  const bool live = !load_done(st);
+  if (live) {
+    const int t = threadIdx.x & 255, grp = threadIdx.x >> 8;
+    for (int k0 = 0; k0 < slots; k0 += 4) {
+      const int k = k0 + grp;
+      double acc = 0.0;
+      if (k < slots)
+        for (int i = t; i < nparts; i += 256) acc += partials[k * slot_stride + i];
+      red[grp][t] = acc;
+      __syncthreads();
+      for (int o = 128; o > 0; o >>= 1) {
+        if (t < o) red[grp][t] += red[grp][t + o];
+        __syncthreads();
+      }
+      if (t == 0 && k < slots) energy[k] = red[grp][0];
+    }
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    st->e_acc = red[0];
-    finish_iteration(st, rule, h);
+    if (live) {
+      DevState s = *st;
+      for (int k = 0; k < slots && !s.done; ++k) {
+        s.e_acc = energy[k];
+        finish_iteration(&s, rule, h);
+      }
+      *st = s;
+    }
+    if (guard.on) cycle_guard(st, 1, guard);
   }
 }
 
@@ -511,7 +521,6 @@ static __global__ void k_reset_state(DevState* st, int n) {
     s->converged = 0;
     s->calc_energy = 1;
     s->status = 0;
-    s->blocks_done = 0;
     s->cycles = 0;
     s->e_acc = 0.0;
     s->last_step_energy = __longlong_as_double(0x7ff0000000000000LL);  // inf (Simulation.m:169)
@@ -558,7 +567,6 @@ static __global__ void k_warm_restart(DevState* st, int n) {
     s->done = 0;
     s->converged = 0;
     s->calc_energy = 1;
-    s->blocks_done = 0;
     s->e_acc = 0.0;
     s->last_step_energy = __longlong_as_double(0x7ff0000000000000LL);
     s->diff1_locked = 1;
@@ -665,22 +673,13 @@ static __global__ void k_warm_check(DevState* st, int n, double ratio, double nw
 // Runs after each wiggle cycle of the graph: continues the device-side while
 // loop only if the stop rule has not fired and fewer than max_cycles cycles
 // have run, so the loop ends even if the stop logic were never reached.
-static __global__ void k_cycle_guard(DevState* st, int n, cudaGraphConditionalHandle cond, long long max_cycles) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    const long long c = ++st->cycles;
-    bool any = false;
-    for (int i = 0; i < n; ++i) any |= !st[i].done;
-    const bool go = any && c < max_cycles;
-    if (!go)
-      for (int i = 0; i < n; ++i) st[i].done = 1;
-    cudaGraphSetConditional(cond, go ? 1u : 0u);
-  }
+static __global__ void k_cycle_guard(DevState* st, int n, CycleGuard guard) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) cycle_guard(st, n, guard);
 }
 
 static __global__ void k_resume_state(DevState* st) {
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     st->done = 0;
-    st->blocks_done = 0;
     st->e_acc = 0.0;
   }
 }

@@ -675,9 +675,6 @@ struct Solver {
   LayoutChoice tuned{};          // the autotuner's choice (all zero: the heuristics)
   double warm_ratio = 0.0;       // discard threshold of the current solve
   long long wait_clocks = 0;     // bound of the TMA pencils' tile waits (0: the default)
-  int fin_fuse = 0;              // WAVESIM_B200_FIN=1: the column pass's last block runs the stop rule instead
-                                 // of k_finish_iteration (measured: 256^3 46.05 against 45.63 ms, 1024^2
-                                 // 8.83 against 8.74 ms, 320^2 5.52 against 5.40 ms; off)
   int pdl = 0;                   // WAVESIM_B200_PDL=1: launch the loop's kernels with programmatic
                                  // dependent launch (measured: 256^3 solve 46.3 against 44.3 ms,
                                  // 96^3 3.38 against 2.80 ms, 1024^2 8.50 against 8.71 ms; off)
@@ -940,7 +937,7 @@ static int ensure_batch(Solver* s, int nrhs) {
   WS_CUDA(cudaMalloc(&s->d_src, nb));
   WS_CUDA(cudaMalloc(&s->d_state, nrhs * sizeof(DevState)));
   WS_CUDA(cudaMalloc(&s->d_energy, nrhs * sizeof(double)));
-  s->partials_cap = std::max<long long>(1, s->lay.grid_inner) * nrhs;
+  s->partials_cap = std::max<long long>(1, s->lay.grid_inner) * nrhs * s->nw;
   WS_CUDA(cudaMalloc(&s->d_partials, (size_t)s->partials_cap * sizeof(double)));
   WS_CUDA(cudaMemset(s->d_E, 0, nb));
   WS_CUDA(cudaMemset(s->d_dE, 0, nb));
@@ -986,7 +983,6 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     s->pf_outer = per_sm * kNumSms;
     if (const char* e = std::getenv("WAVESIM_B200_FUSED_TMA")) s->fused_tma = std::atoi(e) ? 1 : 0;
     if (const char* e = std::getenv("WAVESIM_B200_PDL")) s->pdl = std::atoi(e) ? 1 : 0;
-    if (const char* e = std::getenv("WAVESIM_B200_FIN")) s->fin_fuse = std::atoi(e) ? 1 : 0;
   }
 #define WS_TRY(call)                 \
   do {                               \
@@ -1091,7 +1087,16 @@ static int reload_medium(Solver* s, const int64_t N[4], const ws_complex* gamma,
   return WS_OK;
 }
 
-static InnerArgs inner_args(const Solver* s, int w) {
+// what E' takes in iteration i of a cycle (counted from 0)
+static int acc_of(const Solver* s, int i) { return s->nw % 2 ? kAccEach : (i % 2 ? kAccPair : kAccSkip); }
+// the energy partials of iteration i of a cycle
+static double* partials_of(const Solver* s, int i) {
+  return s->d_partials + (long long)(i % s->nw) * s->lay.grid_inner * s->nrhs;
+}
+
+// iteration i of a cycle (wiggle i mod Nw)
+static InnerArgs inner_args(const Solver* s, int i) {
+  const int w = i % s->nw;
   InnerArgs a{};
   a.g = s->g;
   a.w = s->wig[w];
@@ -1106,8 +1111,7 @@ static InnerArgs inner_args(const Solver* s, int w) {
   a.err = s->d_err;
   a.gstride = s->n_media > 1 ? (long long)s->g.npts : 0;
   a.pf = 0;  // K3 (and the generic kernels) measured slower with it
-  // E' += dE' in pairs when every stop (a multiple of Nw) falls after an even iteration
-  a.acc2 = (s->nw % 2 == 0) ? 1 : 0;
+  a.acc2 = acc_of(s, i);
   return a;
 }
 
@@ -1170,7 +1174,7 @@ static cudaError_t launch_k3_t(const Solver* s, int w) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k_inv_inner<kEmax, RS>, inner_args(s, w), (const float2*)s->d_T, s->d_dE,
-                            s->d_E, (const float2*)s->d_gamma, (const DevState*)s->d_state, s->d_partials);
+                            s->d_E, (const float2*)s->d_gamma, (const DevState*)s->d_state, partials_of(s, w));
 }
 
 static size_t fast_inner_smem(const Solver* s, bool fwd) {
@@ -1245,7 +1249,7 @@ static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, cons
   a.E = s->d_E;
   a.gamma = s->d_gamma;
   a.st = s->d_state;
-  a.partials = s->d_partials;
+  a.partials = partials_of(s, w);
   a.pitch = s->lay.pitch;
   a.fstride = (long long)field_elems(s);
   a.tstride = t_stride(s);
@@ -1253,7 +1257,7 @@ static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, cons
   a.total = s->g.nx * s->g.nz * s->g.nc;
   a.lines = p.lines;
   a.bpr = (int)p.grid;
-  a.acc2 = (s->nw % 2 == 0) ? 1 : 0;
+  a.acc2 = acc_of(s, w);
   return launch_uni(s, uni::kernels(p.plan.cls).col[mode], p, &a);
 }
 
@@ -1411,7 +1415,7 @@ static cudaError_t launch_k3_only(const Solver* s, int w) {
     float2* E = s->d_E;
     const float2* gamma = s->d_gamma;
     const DevState* st = s->d_state;
-    double* partials = s->d_partials;
+    double* partials = partials_of(s, w);
     void* args[] = {&a, &T, &dE, &E, &gamma, &st, &partials};
     e = launch_fast_inner(s, s->lay.fi->inv, args);
   } else {
@@ -1420,26 +1424,29 @@ static cudaError_t launch_k3_only(const Solver* s, int w) {
   return e;
 }
 
-static cudaError_t launch_finish(const Solver* s, const StopRule& rule, const Hist& h) {
+// The stop rule for the iterations first .. first + slots - 1 of a cycle.
+static cudaError_t launch_finish(const Solver* s, const StopRule& rule, const Hist& h, int first, int slots,
+                                 CycleGuard guard = CycleGuard{}) {
   DevState* st = s->d_state;
   StopRule r = rule;
   Hist hh = h;
-  const double* partials = s->d_partials;
+  const double* partials = partials_of(s, first);
   int nparts = (int)s->lay.grid_inner;
-  void* args[] = {&st, &r, &hh, &partials, &nparts};
-  cudaError_t e0 = launch_pdl(s, (const void*)k_finish_iteration, dim3(s->nrhs), dim3(256), args, 0);
-  if (e0 != cudaSuccess) return e0;
+  long long stride = s->lay.grid_inner * s->nrhs;
+  void* args[] = {&st, &r, &hh, &partials, &nparts, &stride, &slots, &guard};
+  const int th = slots > 1 ? 1024 : 256;  // 256 threads per iteration, four at a time
+  return launch_pdl(s, (const void*)k_finish_iterations, dim3(s->nrhs), dim3(th), args, 0);
+}
+// ... of a whole cycle, with the guard of the graph's while loop
+static cudaError_t launch_cycle_end(const Solver* s, const StopRule& rule, const Hist& h, CycleGuard guard) {
+  const CycleGuard one = s->nrhs == 1 ? guard : CycleGuard{};
+  cudaError_t e = launch_finish(s, rule, h, 0, s->nw, one);
+  if (e != cudaSuccess || !guard.on || one.on) return e;
+  k_cycle_guard<<<1, 32, 0, s->stream>>>(s->d_state, s->nrhs, guard);
   return cudaGetLastError();
 }
 
-static cudaError_t launch_k3(const Solver* s, int w, const StopRule& rule, const Hist& h) {
-  cudaError_t e = launch_k3_only(s, w);
-  if (e != cudaSuccess) return e;
-  return launch_finish(s, rule, h);
-}
-
-static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source, const StopRule& rule,
-                                    const Hist& h);
+static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source);
 
 // K3 of the iteration with wiggle w fused with K1 of the next (wiggle w1,
 // with the source when that iteration is one of the first Nw)
@@ -1483,7 +1490,7 @@ static cudaError_t launch_k3k1(const Solver* s, int w, int w1, bool src_next) {
   float2* E = s->d_E;
   const float2* gamma = s->d_gamma;
   const DevState* st = s->d_state;
-  double* partials = s->d_partials;
+  double* partials = partials_of(s, w);
   void* args[] = {&a, &W1, &src1, &A, &T, &dE, &E, &gamma, &st, &partials};
   void* args_tma[] = {const_cast<CUtensorMap*>(&s->tmap_slab), &a, &W1, &src1, &A, &T, &dE, &E, &gamma, &st,
                       &partials};
@@ -1554,17 +1561,9 @@ static cudaError_t launch_xpencil(const Solver* cs, bool inv) {
 
 // The column pass of the split fused step (kc_col_step): the columns of every
 // plane kernel block, no cluster.
-// With rule and h, the pass's last block per right-hand side also runs the
-// stop rule (finish_in_last_block), in place of k_finish_iteration.
-static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next, const StopRule* rule = nullptr,
-                                  const Hist* h = nullptr) {
+static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next) {
   InnerArgs a = inner_args(s, w);
   a.ncols = s->lay.ncols;
-  if (rule && h) {
-    a.fin = 1;
-    a.rule = *rule;
-    a.hist = *h;
-  }
   Wig W1 = s->wig[w1];
   const float2* src1 = src_next ? s->d_src : nullptr;
   float2 A = make_float2(0.f, (float)(1.0f / s->eps / (float)s->nw));
@@ -1573,7 +1572,7 @@ static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next,
   float2* E = s->d_E;
   const float2* gamma = s->d_gamma;
   const DevState* st = s->d_state;
-  double* partials = s->d_partials;
+  double* partials = partials_of(s, w);
   void* args[] = {&a, &W1, &src1, &A, &T, &dE, &E, &gamma, &st, &partials};
   return launch_pdl(s, s->lay.fi->col_step, dim3((unsigned)(s->lay.grid_inner * s->nrhs)), dim3(fast::kThreads), args,
                     s->lay.fi->smem_col);
@@ -1581,52 +1580,40 @@ static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next,
 
 // K3 of an iteration and K1 of the next: one kernel on a cluster, or the
 // split step (inverse x pencils, column pass, forward x pencils).
-static cudaError_t launch_step(const Solver* s, int w, int w1, bool src_next, const StopRule* rule = nullptr,
-                               const Hist* h = nullptr) {
+static cudaError_t launch_step(const Solver* s, int w, int w1, bool src_next) {
   if (s->lay.uni_in) {
     cudaError_t e = s->lay.mode3d ? launch_uni_x(s, true, s->d_T) : cudaSuccess;
     if (e != cudaSuccess) return e;
     e = launch_uni_col(s, uni::kStep, w, w1, nullptr, src_next ? s->d_src : nullptr, s->d_T, 1.f);
     return e != cudaSuccess || !s->lay.mode3d ? e : launch_uni_x(s, false, s->d_T);
   }
-  if (!s->lay.mode3d) return launch_colstep(s, w, w1, src_next, rule, h);  // 2-D: K2 already transformed along x
+  if (!s->lay.mode3d) return launch_colstep(s, w, w1, src_next);  // 2-D: K2 already transformed along x
   if (!s->lay.xp) return launch_k3k1(s, w, w1, src_next);
   cudaError_t e = launch_xpencil(s, true);
   if (e != cudaSuccess) return e;
-  if ((e = launch_colstep(s, w, w1, src_next, rule, h)) != cudaSuccess) return e;
+  if ((e = launch_colstep(s, w, w1, src_next)) != cudaSuccess) return e;
   return launch_xpencil(s, false);
 }
 
-// Whether the loop's column pass runs the stop rule itself (2-D, or the
-// split step of 3-D planes; WAVESIM_B200_FIN=1).
-static bool finish_in_step(const Solver* s) {
-  return s->fin_fuse && !s->lay.uni_in && (!s->lay.mode3d || s->lay.xp);
-}
-
 // One iteration of the fused loop: T already holds K1's output for it.
-static cudaError_t launch_iteration_fused(const Solver* s, int i, bool src_next, const StopRule& rule,
-                                          const Hist& h) {
+static cudaError_t launch_iteration_fused(const Solver* s, int i, bool src_next) {
   const int w = i % s->nw, w1 = (i + 1) % s->nw;
   cudaError_t e = launch_k2(s, w);
-  if (e != cudaSuccess) return e;
-  if (finish_in_step(s)) return launch_step(s, w, w1, src_next, &rule, &h);
-  if ((e = launch_step(s, w, w1, src_next)) != cudaSuccess) return e;
-  return launch_finish(s, rule, h);
+  return e != cudaSuccess ? e : launch_step(s, w, w1, src_next);
 }
 
 // A steady iteration (no source) of the loop, fused or not.
-static cudaError_t launch_steady(const Solver* s, int i, const StopRule& rule, const Hist& h) {
-  return s->fuse ? launch_iteration_fused(s, i, false, rule, h) : launch_iteration(s, i, false, rule, h);
+static cudaError_t launch_steady(const Solver* s, int i) {
+  return s->fuse ? launch_iteration_fused(s, i, false) : launch_iteration(s, i, false);
 }
 
-static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source, const StopRule& rule,
-                                    const Hist& h) {
+static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source) {
   const int w = it0 % s->nw;
   cudaError_t e = launch_k1(s, w, with_source);
   if (e != cudaSuccess) return e;
   e = launch_k2(s, w);
   if (e != cudaSuccess) return e;
-  return launch_k3(s, w, rule, h);
+  return launch_k3_only(s, w);
 }
 
 // Energy histories: per right-hand side r, diff at r * 2cap and fresh at r * 2cap + cap.
@@ -1647,7 +1634,7 @@ static int ensure_hist(Solver* s, long long cap) {
 // the residual probe of the start and the discard check (k_warm_resid_*,
 // k_warm_check), the restart from dE' = v, E' = 0, iterations 1..Nw with the
 // source and the shift dE' -= v.
-static cudaError_t launch_prologue(const Solver* s, const StopRule& rule, const Hist& h) {
+static cudaError_t launch_prologue(const Solver* s, const StopRule& rule, const Hist& h, CycleGuard guard) {
   const size_t nbytes = field_elems(s) * s->nrhs * sizeof(float2);
   cudaError_t e;
   if ((e = cudaMemsetAsync(s->d_E, 0, nbytes, s->stream)) != cudaSuccess) return e;
@@ -1655,7 +1642,8 @@ static cudaError_t launch_prologue(const Solver* s, const StopRule& rule, const 
   k_reset_state<<<1, 256, 0, s->stream>>>(s->d_state, s->nrhs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (s->warm) {
-    if ((e = launch_iteration(s, 0, true, rule, h)) != cudaSuccess) return e;  // the probe
+    if ((e = launch_iteration(s, 0, true)) != cudaSuccess) return e;  // the probe
+    if ((e = launch_finish(s, rule, h, 0, 1)) != cudaSuccess) return e;
     const long long n = (long long)field_elems(s) * s->nrhs;
     const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 8 * kNumSms);
     const float nw = (float)s->nw;
@@ -1682,12 +1670,14 @@ static cudaError_t launch_prologue(const Solver* s, const StopRule& rule, const 
     // next iteration (with the source while that one is among the first Nw)
     if ((e = launch_k1(s, 0, true)) != cudaSuccess) return e;
     for (int i = 0; i < s->nw; ++i)
-      if ((e = launch_iteration_fused(s, i, i + 1 < s->nw, rule, h)) != cudaSuccess) return e;
+      if ((e = launch_iteration_fused(s, i, i + 1 < s->nw)) != cudaSuccess) return e;
   } else {
     for (int i = 0; i < s->nw; ++i)
-      if ((e = launch_iteration(s, i, true, rule, h)) != cudaSuccess) return e;
+      if ((e = launch_iteration(s, i, true)) != cudaSuccess) return e;
   }
-  if (s->warm) {
+  if (!s->warm) return launch_cycle_end(s, rule, h, guard);
+  if ((e = launch_finish(s, rule, h, 0, s->nw)) != cudaSuccess) return e;
+  {
     const long long fe = (long long)field_elems(s);
     const unsigned bpr = (unsigned)std::max<long long>(1, std::min<long long>((fe + 255) / 256, 4 * kNumSms));
     k_warm_shift<<<dim3(bpr, s->nrhs), 256, 0, s->stream>>>(s->d_dE, s->d_init, s->g, fe, s->d_state);
@@ -1695,7 +1685,8 @@ static cudaError_t launch_prologue(const Solver* s, const StopRule& rule, const 
     // the shift changed dE': the fused loop's T is recomputed from it
     if (s->fuse && (e = launch_k1(s, 0, false)) != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  if (guard.on) k_cycle_guard<<<1, 32, 0, s->stream>>>(s->d_state, s->nrhs, guard);
+  return cudaGetLastError();
 }
 
 static int build_graph(Solver* s, const StopRule& rule, const Hist& h) {
@@ -1714,11 +1705,7 @@ static int build_graph(Solver* s, const StopRule& rule, const Hist& h) {
   // prologue + first cycle (with the source)
   e = cudaStreamBeginCaptureToGraph(s->stream, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    e = launch_prologue(s, rule, h);
-    if (e == cudaSuccess) {
-      k_cycle_guard<<<1, 32, 0, s->stream>>>(s->d_state, s->nrhs, cond, max_cycles);
-      e = cudaGetLastError();
-    }
+    e = launch_prologue(s, rule, h, CycleGuard{1, cond, max_cycles});
     cudaGraph_t g2 = graph;
     cudaError_t e2 = cudaStreamEndCapture(s->stream, &g2);
     if (e == cudaSuccess) e = e2;
@@ -1752,11 +1739,8 @@ static int build_graph(Solver* s, const StopRule& rule, const Hist& h) {
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   e = cudaStreamBeginCaptureToGraph(s->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    for (int i = 0; i < s->nw && e == cudaSuccess; ++i) e = launch_steady(s, i, rule, h);
-    if (e == cudaSuccess) {
-      k_cycle_guard<<<1, 32, 0, s->stream>>>(s->d_state, s->nrhs, cond, max_cycles);
-      e = cudaGetLastError();
-    }
+    for (int i = 0; i < s->nw && e == cudaSuccess; ++i) e = launch_steady(s, i);
+    if (e == cudaSuccess) e = launch_cycle_end(s, rule, h, CycleGuard{1, cond, max_cycles});
     cudaGraph_t b2 = body;
     cudaError_t e2 = cudaStreamEndCapture(s->stream, &b2);
     if (e == cudaSuccess) e = e2;
@@ -1894,7 +1878,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     return fail(WS_ERR_INVALID_ARGUMENT, "batch too large for one launch");
   int rc = ensure_batch(s, nrhs);
   if (rc) return rc;
-  rc = ensure_partials(s, s->lay.grid_inner * (long long)nrhs);
+  rc = ensure_partials(s, s->lay.grid_inner * (long long)nrhs * s->nw);
   if (rc) return rc;
   if (s->nrhs != nrhs) free_graph(s);
   s->nrhs = nrhs;
@@ -1949,13 +1933,14 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     for (long long cycle = 0;; ++cycle) {
       if (cycle >= max_cycles) return fail(WS_ERR_CUDA, "loop did not stop within max_iterations (internal error)");
       if (cycle == 0) {
-        WS_CUDA(launch_prologue(s, rule, h));
+        WS_CUDA(launch_prologue(s, rule, h, CycleGuard{}));
         it += s->nw;
       } else {
         for (int i = 0; i < s->nw; ++i) {
-          WS_CUDA(launch_steady(s, (int)(it % s->nw), rule, h));
+          WS_CUDA(launch_steady(s, (int)(it % s->nw)));
           ++it;
         }
+        WS_CUDA(launch_cycle_end(s, rule, h, CycleGuard{}));
       }
       WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
       WS_CUDA(cudaStreamSynchronize(s->stream));
@@ -2164,11 +2149,11 @@ int ws_solver_set_wait_limit(ws_solver h, int64_t clocks) {
 int ws_solver_launches_per_iteration(ws_solver h) {
   if (!h) return 0;
   const Solver* s = reinterpret_cast<Solver*>(h);
-  // K2, K3 + next K1 (one kernel, or the split step's three), stop rule; or K1, K2, K3, stop rule
-  if (!s->fuse) return 4;                                   // K1, K2, K3, the stop rule
-  if (s->lay.mode3d && !s->lay.xp && !s->lay.uni_in) return 3;  // K2, K3K1 on a cluster, the stop rule
-  const int step = s->lay.mode3d ? 4 : 2;                   // K2 (+ x pencils), the column pass (+ x pencils)
-  return finish_in_step(s) ? step : step + 1;
+  // K2, K3 + next K1 (one kernel, or the split step's three); or K1, K2, K3
+  // (the stop rule is one launch per wiggle cycle)
+  if (!s->fuse) return 3;
+  if (!s->lay.mode3d) return 2;
+  return s->lay.xp || s->lay.uni_in ? 4 : 2;
 }
 
 int ws_solver_fused(ws_solver h) {
@@ -2198,7 +2183,7 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
     WS_CUDA(cudaEventRecord(s->ev[0], s->stream));
     WS_CUDA(launch_step(s, w, (i + 1) % s->nw, false));
     WS_CUDA(cudaEventRecord(s->ev[1], s->stream));
-    WS_CUDA(launch_finish(s, rule, hh));
+    WS_CUDA(launch_finish(s, rule, hh, w, 1));
     WS_CUDA(cudaEventSynchronize(s->ev[1]));
     float t;
     WS_CUDA(cudaEventElapsedTime(&t, s->ev[0], s->ev[1]));
@@ -2241,7 +2226,7 @@ int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double 
     WS_CUDA(cudaEventRecord(s->ev[2], s->stream));
     WS_CUDA(s->lay.uni_in ? launch_uni_x(s, false, s->d_T) : launch_xpencil(s, false));
     WS_CUDA(cudaEventRecord(s->ev[3], s->stream));
-    WS_CUDA(launch_finish(s, rule, hh));
+    WS_CUDA(launch_finish(s, rule, hh, w, 1));
     WS_CUDA(cudaEventSynchronize(s->ev[3]));
     float t;
     for (int k = 0; k < 3; ++k) {
@@ -2283,7 +2268,7 @@ int ws_solver_time_kernels(ws_solver h, int n_iterations, float ms_out[3], doubl
     WS_CUDA(cudaEventRecord(s->ev[2], s->stream));
     WS_CUDA(launch_k3_only(s, w));
     WS_CUDA(cudaEventRecord(s->ev[3], s->stream));
-    WS_CUDA(launch_finish(s, rule, hh));
+    WS_CUDA(launch_finish(s, rule, hh, w, 1));
     WS_CUDA(cudaEventSynchronize(s->ev[3]));
     float t;
     for (int k = 0; k < 3; ++k) {
@@ -2381,7 +2366,7 @@ static int tune_probe(Solver* s, const StopRule& rule, const Hist& hh, float2* o
   } else {
     WS_CUDA(launch_k3_only(s, 0));
   }
-  WS_CUDA(launch_finish(s, rule, hh));
+  WS_CUDA(launch_finish(s, rule, hh, 0, 1));
   WS_CUDA(cudaMemcpyAsync(out, s->d_dE, n * sizeof(float2), cudaMemcpyDeviceToDevice, s->stream));
   WS_CUDA(cudaStreamSynchronize(s->stream));
   return WS_OK;
@@ -2401,7 +2386,7 @@ static int tune_time(Solver* s, const StopRule& rule, const Hist& hh, int iters,
       WS_CUDA(cudaEventRecord(s->ev[1], s->stream));
       WS_CUDA(launch_step(s, w, (i + 1) % s->nw, false));
       WS_CUDA(cudaEventRecord(s->ev[2], s->stream));
-      WS_CUDA(launch_finish(s, rule, hh));
+      WS_CUDA(launch_finish(s, rule, hh, w, 1));
       WS_CUDA(cudaEventSynchronize(s->ev[2]));
       float t;
       WS_CUDA(cudaEventElapsedTime(&t, s->ev[0], s->ev[1]));
@@ -2421,7 +2406,7 @@ static int tune_time(Solver* s, const StopRule& rule, const Hist& hh, int iters,
     WS_CUDA(cudaEventRecord(s->ev[2], s->stream));
     WS_CUDA(launch_k3_only(s, w));
     WS_CUDA(cudaEventRecord(s->ev[3], s->stream));
-    WS_CUDA(launch_finish(s, rule, hh));
+    WS_CUDA(launch_finish(s, rule, hh, w, 1));
     WS_CUDA(cudaEventSynchronize(s->ev[3]));
     float t;
     for (int k = 0; k < 3; ++k) {
@@ -2454,7 +2439,7 @@ static bool apply_choice(Solver* s, const LayoutChoice& c) {
   // the plan and twiddles made for the solver's first layout: a layout with
   // another cluster size would run them on lines of another length
   if (L.mode3d && !L.fi && !L.uni_in && s->g.nx / L.csize != s->pxl.n) return false;
-  if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap)) != WS_OK) return false;
+  if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap) * s->nw) != WS_OK) return false;
   s->lay = L;
   if (ensure_uni(s) != cudaSuccess) return false;
   apply_sched(s, c.sched);

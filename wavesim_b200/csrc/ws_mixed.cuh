@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   st += rhs;
   if (load_done(st)) return;
   // with a.acc2, E' takes dE'_{k-1} + dE'_k after even iterations k only
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;  // the same for every block of a cluster
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;  // the same for every block of a cluster
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int rhs = rb / a.bpr, bid = rb - rhs * a.bpr;
   st += rhs;
   if (load_done(st)) return;
-  const bool acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+  const bool acc_now = a.acc2 != kAccSkip;
   T += rhs * a.fstride;
   dE += rhs * a.fstride;
   E += rhs * a.fstride;
@@ -926,7 +926,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (tid == 0) partials[bid] = (double)v;
   }
-  if (a.fin) finish_in_last_block(const_cast<DevState*>(st), a.rule, a.hist, partials, a.bpr, rhs);
 }
 
 // 2-D grids on the mixed-radix lines: the y transforms of whole columns, as
@@ -975,7 +974,7 @@ __device__ __forceinline__ void col2d(const InnerArgs& a, const Wig& w1, const f
   if constexpr (MODE == kCol2dFwd) {
     din += rhs * a.fstride;
   } else {
-    acc_now = !a.acc2 || (__ldcg(&st->it) & 1) == 0;
+    acc_now = a.acc2 != kAccSkip;
     dE += rhs * a.fstride;
     E += rhs * a.fstride;
     partials += (long long)rhs * a.bpr;
@@ -1101,8 +1100,6 @@ __device__ __forceinline__ void col2d(const InnerArgs& a, const Wig& w1, const f
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (tid == 0) partials[bid] = (double)v;
     }
-    if (MODE == kCol2dStep && a.fin)
-      finish_in_last_block(const_cast<DevState*>(st), a.rule, a.hist, partials, a.bpr, rhs);
   }
 }
 

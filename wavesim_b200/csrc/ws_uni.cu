@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kMaxThreads, (MODE == kFwd ? kBlocks<RM> : kBl
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
   const DevState* st = a.st + rhs;
   if (load_done(st)) return;
-  const bool acc_now = MODE != kFwd && (!a.acc2 || (__ldcg(&st->it) & 1) == 0);
+  const bool acc_now = MODE != kFwd && a.acc2 != kAccSkip;
   extern __shared__ float2 tile[];
   const Geom& g = a.g;
   const int tid = threadIdx.x, nthr = blockDim.x;
