@@ -64,3 +64,62 @@ def test_uni_matches_generic_and_oracle(gpu, name, monkeypatch):
     assert st.it == sg.it == so.it
     assert rel(E, Eg) < TOL and rel(E, Eo) < TOL, (rel(E, Eg), rel(E, Eo))
     np.testing.assert_allclose(st.diff_energy, so.diff_energy, rtol=2e-4)
+
+
+LOOPS = {
+    # the loop in one launch: on a cluster of 16 blocks, at the edges of its tiles, with E' in shared
+    # memory and not, and on a grid that has compile-time kernels for its launched passes
+    "64x56_cluster": ((48, 40), [8, 8]),
+    "4x6": ((4, 6), [0, 0]),
+    "160x264": ((96, 200), [32, 32]),
+    "225x150": ((225, 150), [0, 0]),
+    "1100x768_E_in_global": ((1068, 736), [16, 16]),
+    "512x512_fast_passes": ((448, 448), [32, 32]),
+}
+
+
+def loop_sim(ws, name, **more):
+    shape, bw = LOOPS[name]
+    rng = np.random.default_rng(5)
+    n = 1.1 + 0.2 * rng.random(shape) + 0.01j
+    opt = {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": bw, "energy_threshold": 1e-3, "max_iterations": 40}
+    opt.update(more)
+    return ws.WaveSim(n, opt), ws.Source(np.ones((shape[0], 1)) + 0.4j, [1, 1])
+
+
+@pytest.mark.parametrize("name", list(LOOPS))
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_loop_in_one_launch_is_bit_identical(gpu, name, use_graph, monkeypatch):
+    """One launch for the whole loop (use_graph) or per cycle, against one launch per pass."""
+    import wavesim_b200 as ws
+    got = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("WAVESIM_B200_FUSE", fuse)
+        sim, src = loop_sim(ws, name, use_graph=use_graph)
+        got.append(sim.exec(src))
+        sim.close()
+    (E, st), (Eu, su) = got
+    assert st.it == su.it
+    np.testing.assert_array_equal(st.diff_energy, su.diff_energy)
+    np.testing.assert_array_equal(E, Eu)
+
+
+def test_loop_over_several_launches_and_batches(gpu):
+    """More cycles than one launch takes; and several right-hand sides in one launch."""
+    import wavesim_b200 as ws
+    sim, src = loop_sim(ws, "64x56_cluster", energy_threshold=1e-99, max_iterations=2200)
+    E, st = sim.exec(src)
+    sim.use_graph = False  # a launch per cycle
+    Eh, sh = sim.exec(src)
+    assert st.it == sh.it == 2201
+    np.testing.assert_array_equal(st.diff_energy, sh.diff_energy)
+    np.testing.assert_array_equal(E, Eh)
+    sim.close()
+    sim, src = loop_sim(ws, "64x56_cluster", energy_threshold=1e-6, max_iterations=4000)
+    sources = [src, ws.Source(1.0, [24, 20]), src]
+    Eb, sb = sim.exec_batch(sources)
+    for s, e, t in zip(sources, Eb, sb):
+        E1, s1 = sim.exec(s)
+        assert t.it == s1.it and t.converged
+        np.testing.assert_array_equal(e, E1)
+    sim.close()

@@ -20,7 +20,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include")]
 
 TARGETS = {
-    "libwavesim_b200.so": ["ws_mbs.cu", "ws_uni.cu", "ws_noalloc.cu", "ws_net.cu", "ws_setup.cu"],
+    "libwavesim_b200.so": ["ws_mbs.cu", "ws_uni_r8.cu", "ws_uni_r12.cu", "ws_uni_r16.cu", "ws_noalloc.cu", "ws_net.cu", "ws_setup.cu"],
 }
 
 

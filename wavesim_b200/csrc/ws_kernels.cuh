@@ -450,8 +450,8 @@ __global__ void __launch_bounds__(512, 1) k_inv_inner(InnerArgs a, const float2*
 // 284).  (An energy that is not finite
 // ends the history at its iteration and the solve with the cycle.)
 //
-// One block per right-hand side; 256 threads sum one iteration's nparts
-// partials (slot k at partials + k slot_stride), four iterations at a time.
+// One block per right-hand side, one warp per iteration (slot k's nparts
+// partials at partials + k slot_stride).
 // With `guard` (one right-hand side) the kernel is also the cycle's guard
 // (k_cycle_guard).
 struct CycleGuard {
@@ -469,33 +469,36 @@ __device__ __forceinline__ void cycle_guard(DevState* st, int n, const CycleGuar
   cudaGraphSetConditional(g.cond, go ? 1u : 0u);
 }
 
+// The sum of n partials by a warp, in an order that depends on n alone.
+__device__ __forceinline__ double sum_partials(const double* partials, int n) {
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i = threadIdx.x & 31; i < n; i += 128) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i + 32 * q < n) a[q] += __ldcg(&partials[i + 32 * q]);
+  }
+  double e = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  return e;
+}
+
 constexpr int kMaxWiggles = 64;
-static __global__ void __launch_bounds__(1024) k_finish_iterations(DevState* st, StopRule rule, Hist h,
-                                                                   const double* __restrict__ partials, int nparts,
-                                                                   long long slot_stride, int slots, CycleGuard guard) {
+static __global__ void __launch_bounds__(256) k_finish_iterations(DevState* st, StopRule rule, Hist h,
+                                                                  const double* __restrict__ partials, int nparts,
+                                                                  long long slot_stride, int slots, CycleGuard guard) {
   pdl_begin();
   const int rhs = blockIdx.x;
   st += rhs;
   partials += (long long)rhs * nparts;
   h.diff += rhs * h.stride;
   if (h.fresh) h.fresh += rhs * h.stride;
-  __shared__ double red[4][256];
   __shared__ double energy[kMaxWiggles];
   const bool live = !load_done(st);
   if (live) {
-    const int t = threadIdx.x & 255, grp = threadIdx.x >> 8;
-    for (int k0 = 0; k0 < slots; k0 += 4) {
-      const int k = k0 + grp;
-      double acc = 0.0;
-      if (k < slots)
-        for (int i = t; i < nparts; i += 256) acc += partials[k * slot_stride + i];
-      red[grp][t] = acc;
-      __syncthreads();
-      for (int o = 128; o > 0; o >>= 1) {
-        if (t < o) red[grp][t] += red[grp][t + o];
-        __syncthreads();
-      }
-      if (t == 0 && k < slots) energy[k] = red[grp][0];
+    for (int k = threadIdx.x >> 5; k < slots; k += 8) {
+      const double e = sum_partials(partials + k * slot_stride, nparts);
+      if ((threadIdx.x & 31) == 0) energy[k] = e;
     }
     __syncthreads();
   }

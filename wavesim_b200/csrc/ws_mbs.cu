@@ -31,6 +31,7 @@ constexpr int kMaxThreadsPow2 = 512;
 constexpr int kMaxThreadsMixed = 512;
 constexpr size_t kSmemBudget = 150 * 1024;  // per-block tile budget (bytes)
 constexpr int kNumSms = 148;
+constexpr long long kLoopCycles = 512;  // wiggle cycles of one cooperative launch (uni::k_loop)
 
 thread_local std::string g_last_error;
 
@@ -339,6 +340,8 @@ static bool uni_plan(int n, uni::Plan& P) {
     S.blkp = padded(block);
     S.msub = uni::magic(S.sub);
     S.munits = uni::magic(S.units);
+    S.two = P.ntw;
+    P.ntw += block;
     block = S.sub;
   }
   return true;
@@ -367,16 +370,19 @@ static int uni_units(const uni::Plan& P) {
   return m;
 }
 
+// energies that a block of the column pass sums: one per 32 butterflies of its first stage
+static int uni_groups(const UniPass& p) { return (p.lines * p.plan.st[0].units + 31) / 32; }
+
 // The column pass: one butterfly per thread, as many columns as fill 256 threads,
 // fewer where the grid would not give every SM two blocks, at least a warp.
-static void uni_columns(UniPass& p, long long total) {
+static void uni_columns(UniPass& p, long long total, int lines = 0) {
   const int um = uni_units(p.plan);
   const long long most = std::max(1, uni::kMaxThreads / um), least = (32 + um - 1) / um;
   long long l = std::min(most, std::max(least, total / (2 * kNumSms)));
   while (l > 1 && l * p.plan.np * sizeof(float2) > 64 * 1024) l /= 2;
-  p.lines = (int)std::min(l, total);
+  p.lines = lines ? lines : (int)std::min(l, total);
   p.threads = (int)std::min<long long>(uni::kMaxThreads, (p.lines * (long long)um + 31) / 32 * 32);
-  p.smem = p.lines * (p.plan.np * sizeof(float2) + 32);
+  p.smem = p.lines * (p.plan.np * sizeof(float2) + 32) + 2 * p.plan.n * sizeof(float2) + uni_groups(p) * sizeof(float);
   p.grid = (total + p.lines - 1) / p.lines;
 }
 
@@ -397,8 +403,15 @@ static void uni_pencils(UniPass& p, int ny, int nc, long long mids) {
   int w = std::max(1, std::min(um, uni::kMaxThreads / ty));
   while ((w * ty) % 32 && w * ty + ty <= uni::kMaxThreads) ++w;
   p.threads = w * ty;
-  p.smem = ty * row;
+  p.smem = ty * row + p.plan.n * sizeof(float);
   p.grid = (long long)((ny + ty - 1) / ty) * mids;
+}
+
+static const uni::Kernels& uni_kernels(int cls) {
+  static const uni::Kernels t[uni::kClasses] = {uni::kernels_up_to<uni::kClassRadix[0]>(),
+                                                uni::kernels_up_to<uni::kClassRadix[1]>(),
+                                                uni::kernels_up_to<uni::kClassRadix[2]>()};
+  return t[cls];
 }
 
 struct Layout {
@@ -419,6 +432,7 @@ struct Layout {
   long long pitch = 0;  // elements between the columns of T
 };
 
+static int log2_of(int n) { return n > 1 ? 1 + log2_of(n / 2) : 0; }
 static bool is_pow2(long long n) { return n >= 1 && (n & (n - 1)) == 0; }
 
 // Overrides of the layout heuristics, for the autotuner (0 = heuristic).
@@ -435,6 +449,46 @@ struct LayoutChoice {
            sched == o.sched && xp == o.xp;
   }
 };
+
+// The loop of a 2-D grid in one launch: a column tile per SM, the tables of
+// all nw wiggles, gamma and dE' of the tile (E' where it fits) in shared memory.
+static size_t loop_smem(const Layout& L, const Geom& g, int nw, bool e_resident, int* tile_elems = nullptr) {
+  const size_t l = L.ucol.lines;
+  const size_t tile = std::max(l * L.ucol.plan.np, (size_t)L.uout.lines * L.uout.plan.n);
+  if (tile_elems) *tile_elems = (int)tile;
+  const size_t tables = L.ucol.plan.ntw + L.uout.plan.ntw + nw * (g.ny + l);
+  return (tile + tables + l * g.ny * (e_resident ? 3 : 2)) * sizeof(float2) + l * 16 +
+         (uni_groups(L.ucol) + (size_t)nw * L.uout.plan.n) * sizeof(float);
+}
+constexpr size_t kLoopSmem = 225 * 1024;
+// The layout of single solves of small 2-D grids, `L` being the one of the
+// grid's launched passes; false if there is none.  Measured against the
+// launched passes, us an iteration: 64 x 56 7.6 (12.8), 160 x 264 12.4 (21.4),
+// 396 x 315 11.0 (19.7), 512^2 12.6 (18.8, compile-time kernels), 632^2 20.3
+// (23.9), 1100 x 768 27.8 (38); 1024^2 38.7 (34.2, compile-time kernels).  So
+// it takes every grid whose columns fit the SMs' shared memory, but those with
+// compile-time kernels in both passes only up to 400 000 points.
+static bool loop_layout(const Geom& g, const Layout& L, const LayoutChoice& ch, bool pstd, Layout& out) {
+  if (pstd || L.mode3d || g.nc != 1 || ch.inner == 2 || ch.outer == 2) return false;
+  const char* path = std::getenv("WAVESIM_B200_PATH");
+  if (path && std::strcmp(path, "generic") == 0) return false;
+  if (L.fi && L.fp && g.npts > 400000) return false;
+  Layout t{};
+  if (!uni_plan(g.nx, t.uout.plan) || !uni_plan(g.ny, t.ucol.plan)) return false;
+  t.uni_in = t.uni_out = true;
+  uni_pencils(t.uout, g.ny, 1, 1);
+  // a tile per SM; up to 8192 points the tiles of 16 SMs, which then form one
+  // cluster and meet at its hardware barrier (64 x 56: 7.6 us against 8.6)
+  const int sms = t.uout.grid <= 16 && g.npts <= 8192 ? 16 : kNumSms;
+  uni_columns(t.ucol, g.nx, (g.nx + sms - 1) / sms);
+  if (loop_smem(t, g, 4, false) > kLoopSmem) return false;
+  t.grid_inner = t.ucol.grid;
+  t.grid_outer = t.uout.grid;
+  t.rset = L.rset;
+  t.pitch = (g.ny + 3) / 4 * 4;
+  out = t;
+  return true;
+}
 
 static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutChoice& ch = LayoutChoice{},
                        bool pstd = false) {
@@ -615,13 +669,23 @@ static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutC
 struct GraphKey {
   double threshold = -1;
   long long max_iter = -1;
-  int interval = -1, stop_rule = -1, nan_stop = -1, nrhs = -1, warm = -1;
+  int interval = -1, stop_rule = -1, nan_stop = -1, nrhs = -1, warm = -1, layout = -1;
   double warm_ratio = -1;
   bool operator==(const GraphKey& o) const {
     return threshold == o.threshold && max_iter == o.max_iter && interval == o.interval &&
-           stop_rule == o.stop_rule && nan_stop == o.nan_stop && nrhs == o.nrhs && warm == o.warm &&
+           stop_rule == o.stop_rule && nan_stop == o.nan_stop && nrhs == o.nrhs && warm == o.warm && layout == o.layout &&
            warm_ratio == o.warm_ratio;
   }
+};
+
+// Device tables of a layout's run-time scheduled plans, in one buffer: the
+// wiggles (natural, and with the p tables in the order of T), the twiddles, the
+// permutation of the p tables, the permuted p tables.
+struct UniTables {
+  Wig* wigs = nullptr;
+  int* perm = nullptr;
+  float* p = nullptr;
+  std::vector<Wig> uwig;
 };
 
 struct Solver {
@@ -679,10 +743,11 @@ struct Solver {
                                  // dependent launch (measured: 256^3 solve 46.3 against 44.3 ms,
                                  // 96^3 3.38 against 2.80 ms, 1024^2 8.50 against 8.71 ms; off)
   float2* d_tw = nullptr;
-  float2* d_utw = nullptr;       // run-time scheduled kernels: twiddles, then
-  int* d_uperm = nullptr;        //   the permutation of the p tables and
-  float* d_uwigf = nullptr;      //   the wiggles' p tables in the order of T
-  std::vector<Wig> uwig;
+  Layout lays[2];                // the layouts of the launched passes [0] and of the loop in one launch [1];
+  bool has_loop = false;         //   `lay` is the one in use, lays[active]
+  int active = 0;
+  int fuses[2] = {};             // `fuse` of each
+  UniTables ut[2];               // their tables
   FftPlan py{}, pxl{}, po{};
   const float2* twx = nullptr;
   cudaGraph_t graph = nullptr;
@@ -700,13 +765,11 @@ static void free_graph(Solver* s) {
 
 // The fused K3 + K1 step is used where the layout has one (3-D fast planes on
 // a cluster); WAVESIM_B200_FUSE=0 keeps the three kernels separate.
-static void update_fuse(Solver* s) {
+static int fuse_of(const Solver* s, const Layout& L) {
   const char* e = std::getenv("WAVESIM_B200_FUSE");
-  const bool on3 = s->lay.fi && (s->lay.fi->fused || s->lay.xp) && s->lay.mode3d;
-  const bool on2 = s->lay.fi && !s->lay.mode3d && s->lay.fi->col_step;  // 2-D: K2 + the column pass
-  const int f = ((on3 || on2 || s->lay.uni_in) && !s->pstd && !(e && std::strcmp(e, "0") == 0)) ? 1 : 0;
-  if (f != s->fuse) free_graph(s);
-  s->fuse = f;
+  const bool on3 = L.fi && (L.fi->fused || L.xp) && L.mode3d;
+  const bool on2 = L.fi && !L.mode3d && L.fi->col_step;  // 2-D: K2 + the column pass
+  return ((on3 || on2 || L.uni_in) && !s->pstd && !(e && std::strcmp(e, "0") == 0)) ? 1 : 0;
 }
 
 static void destroy_solver(Solver* s) {
@@ -715,7 +778,7 @@ static void destroy_solver(Solver* s) {
   free_graph(s);
   void* ptrs[] = {s->d_wigf, s->d_wigc,  s->d_gamma,  s->d_E,        s->d_dE, s->d_T,   s->d_src,
                   s->d_stage, s->d_out, s->d_state, s->d_hist, s->d_energy, s->d_tw, s->d_partials, s->d_init,
-                  s->d_err, s->d_utw};
+                  s->d_err, s->ut[0].wigs, s->ut[1].wigs};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& e : s->ev)
@@ -789,10 +852,12 @@ static int set_kernel_attributes() {
   for (const FastPencil& f : fast_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (const TmaPencil& f : tma_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (int c = 0; c < uni::kClasses; ++c) {
-    const uni::Kernels& k = uni::kernels(c);
+    const uni::Kernels& k = uni_kernels(c);
     for (const void* f : k.col) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.x) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.pencil) WS_CUDA(allow_dynamic_smem(f, optin));
+    WS_CUDA(allow_dynamic_smem(k.loop, optin));
+    WS_CUDA(cudaFuncSetAttribute(k.loop, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
   for (const XPencil& f : x_pencil_table()) {
     WS_CUDA(allow_dynamic_smem(f.fwd, optin));
@@ -837,7 +902,7 @@ static size_t field_elems(const Solver* s) { return (size_t)s->g.npts * s->g.nc;
 static size_t t_alloc_elems(const Solver* s) { return (size_t)((s->g.ny + 3) / 4 * 4) * s->g.nx * s->g.nz * s->g.nc; }
 static long long t_stride(const Solver* s) { return s->lay.pitch * s->g.nx * s->g.nz * s->g.nc; }
 
-// The wiggles' p tables in the order in which the layout's run-time scheduled
+// The wiggles' p tables in the order in which a layout's run-time scheduled
 // plans leave T (natural along the axes that other kernels transform):
 // per[w][i] = nat[w][perm[i]].
 static __global__ void k_permute_tables(float* __restrict__ per, const float* __restrict__ nat,
@@ -846,29 +911,33 @@ static __global__ void k_permute_tables(float* __restrict__ per, const float* __
   if (i < nf) per[(long long)blockIdx.y * nf + i] = nat[(long long)blockIdx.y * nf + perm[i]];
 }
 static cudaError_t permute_wiggles(Solver* s) {
-  if (!s->lay.uni_out) return cudaSuccess;
   cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);  // the tables' uploads
   if (e != cudaSuccess) return e;
   const int nf = s->g.nx + s->g.ny + s->g.nz;
-  k_permute_tables<<<dim3((nf + 255) / 256, s->nw), 256, 0, s->stream>>>(s->d_uwigf, s->d_wigf, s->d_uperm, nf);
+  for (const UniTables& t : s->ut)
+    if (t.wigs)
+      k_permute_tables<<<dim3((nf + 255) / 256, s->nw), 256, 0, s->stream>>>(t.p, s->d_wigf, t.perm, nf);
   return cudaGetLastError();
 }
 
-// The device tables of the layout's run-time scheduled plans, in one buffer:
-// twiddles, the permutation of the p tables, the permuted p tables.
-static cudaError_t ensure_uni(Solver* s) {
-  Layout& L = s->lay;
+// The tables of layout k.
+static cudaError_t make_tables(Solver* s, int k) {
+  Layout& L = s->lays[k];
+  UniTables& t = s->ut[k];
+  if (t.wigs) cudaFree(t.wigs);
+  t = UniTables{};
   if (!L.uni_out) return cudaSuccess;
   const Geom& g = s->g;
   const int len[3] = {g.nx, g.ny, g.nz};  // the order of d_wigf
   const uni::Plan* axis[3] = {L.mode3d ? (L.uni_in ? &L.ux.plan : nullptr) : &L.uout.plan,
                               L.uni_in ? &L.ucol.plan : nullptr, L.mode3d ? &L.uout.plan : nullptr};
   std::vector<float2> tw;
-  std::vector<std::pair<uni::Stage*, size_t>> at;
-  for (UniPass* p : {&L.ucol, &L.ux, &L.uout})
-    for (int k = 0; k < p->plan.nst; ++k) {
-      uni::Stage& S = p->plan.st[k];
-      at.push_back({&S, tw.size()});
+  uni::Plan* plans[3] = {&L.ucol.plan, &L.ux.plan, &L.uout.plan};
+  size_t at[3];
+  for (int q = 0; q < 3; ++q) {
+    at[q] = tw.size();
+    for (int i = 0; i < plans[q]->nst; ++i) {
+      const uni::Stage& S = plans[q]->st[i];
       const int n = S.R * S.sub;
       for (int r = 0; r < S.R; ++r)
         for (int j = 0; j < S.sub; ++j) {
@@ -876,32 +945,55 @@ static cudaError_t ensure_uni(Solver* s) {
           tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
         }
     }
+  }
   std::vector<int> perm;
   for (int d = 0; d < 3; ++d) {
     const int off = (int)perm.size();
-    const std::vector<int> k = axis[d] ? uni_permutation(*axis[d]) : std::vector<int>();
-    for (int i = 0; i < len[d]; ++i) perm.push_back(off + (axis[d] ? k[i] : i));
+    const std::vector<int> f = axis[d] ? uni_permutation(*axis[d]) : std::vector<int>();
+    for (int i = 0; i < len[d]; ++i) perm.push_back(off + (axis[d] ? f[i] : i));
   }
-  const size_t twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
-  if (s->d_utw) cudaFree(s->d_utw);
-  s->d_utw = nullptr;
-  cudaError_t e = cudaMalloc(&s->d_utw, twb + pb * (1 + s->nw));
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_utw, tw.data(), twb, cudaMemcpyHostToDevice, s->stream);
-  s->d_uperm = reinterpret_cast<int*>(reinterpret_cast<char*>(s->d_utw) + twb);
-  s->d_uwigf = reinterpret_cast<float*>(reinterpret_cast<char*>(s->d_uperm) + pb);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(s->d_uperm, perm.data(), pb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = permute_wiggles(s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // tw and perm end here
+  const size_t wb = 2 * s->nw * sizeof(Wig), twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
+  char* buf = nullptr;
+  cudaError_t e = cudaMalloc(&buf, wb + twb + pb * (1 + s->nw));
   if (e != cudaSuccess) return e;
-  for (auto& a : at) a.first->tw = s->d_utw + a.second;
-  s->uwig = s->wig;
+  t.wigs = reinterpret_cast<Wig*>(buf);
+  float2* const d_tw = reinterpret_cast<float2*>(buf + wb);
+  t.perm = reinterpret_cast<int*>(buf + wb + twb);
+  t.p = reinterpret_cast<float*>(buf + wb + twb + pb);
+  for (int q = 0; q < 3; ++q) plans[q]->tw = d_tw + at[q];
+  t.uwig = s->wig;
   for (int w = 0; w < s->nw; ++w) {
-    const float* f = s->d_uwigf + perm.size() * w;
-    s->uwig[w].pxe = f;
-    s->uwig[w].pye = f + g.nx;
-    s->uwig[w].pze = f + g.nx + g.ny;
+    const float* f = t.p + perm.size() * w;
+    t.uwig[w].pxe = f;
+    t.uwig[w].pye = f + g.nx;
+    t.uwig[w].pze = f + g.nx + g.ny;
   }
-  return cudaSuccess;
+  std::vector<Wig> wigs(s->wig);
+  wigs.insert(wigs.end(), t.uwig.begin(), t.uwig.end());
+  e = cudaMemcpyAsync(t.wigs, wigs.data(), wb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_tw, tw.data(), twb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(t.perm, perm.data(), pb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // the host tables end here
+  return e;
+}
+
+// Makes lays[k] the layout in use.
+static void use_layout(Solver* s, int k) {
+  s->active = k;
+  s->lay = s->lays[k];
+  s->fuse = s->fuses[k];
+}
+
+// The layouts for choice ch of the launched passes (lays[0], made by the
+// caller), with their tables; the launched passes' is then in use.
+static cudaError_t set_layouts(Solver* s, const LayoutChoice& ch) {
+  s->has_loop = loop_layout(s->g, s->lays[0], ch, s->pstd != 0, s->lays[1]);
+  cudaError_t e = make_tables(s, 0);
+  if (e == cudaSuccess && s->has_loop) e = make_tables(s, 1);
+  if (e == cudaSuccess) e = permute_wiggles(s);
+  for (int k = 0; k < 2; ++k) s->fuses[k] = fuse_of(s, s->lays[k]);
+  use_layout(s, 0);
+  return e;
 }
 
 // Buffers for nrhs right-hand sides (kept when large enough).
@@ -971,7 +1063,6 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     destroy_solver(s);
     return fail(rc, why);
   }
-  update_fuse(s);
   {
     // L2 prefetch distance of the fast kernels: about one wave of resident
     // blocks (2 per SM), a whole number of clusters.  WAVESIM_B200_PREFETCH
@@ -994,8 +1085,8 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     }                                \
   } while (0)
   WS_TRY(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-  WS_TRY(cudaMalloc(&s->d_err, sizeof(int)));
-  WS_TRY(cudaMemset(s->d_err, 0, sizeof(int)));
+  WS_TRY(cudaMalloc(&s->d_err, 2 * sizeof(int)));  // and the loop's barrier counter
+  WS_TRY(cudaMemset(s->d_err, 0, 2 * sizeof(int)));
   for (auto& e : s->ev) WS_TRY(cudaEventCreate(&e));
   // plans and twiddle tables
   std::vector<float2> tw;
@@ -1036,7 +1127,8 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     WS_TRY(cudaMemcpy(c + g.nx + g.ny, W.gz, g.nz * sizeof(float2), kind));
     s->wig.push_back(Wig{f, f + g.nx, f + g.nx + g.ny, c, c + g.nx, c + g.nx + g.ny});
   }
-  WS_TRY(ensure_uni(s));
+  s->lays[0] = s->lay;
+  WS_TRY(set_layouts(s, LayoutChoice{}));
   WS_TRY(cudaMalloc(&s->d_gamma, (size_t)g.npts * sizeof(float2)));
   WS_TRY(cudaMemcpy(s->d_gamma, gamma, (size_t)g.npts * sizeof(float2), kind));
 #undef WS_TRY
@@ -1229,27 +1321,27 @@ static cudaError_t launch_uni(const Solver* s, const void* fn, const UniPass& p,
 
 // mode kFwd: K1's column transforms of `in`; kInv: K3's; kStep: K3 with
 // wiggle w and K1 of the next iteration with wiggle w1
-static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, const float2* in, const float2* src,
-                                  float2* T, float a_mult) {
+static uni::ColArgs uni_col_args(const Solver* s, int w, int w1, const float2* in, const float2* src, float2* T,
+                                 float a_mult) {
   const UniPass& p = s->lay.ucol;
   uni::ColArgs a{};
   a.g = s->g;
   a.py = p.plan;
-  a.gx = s->wig[w].gx;
-  a.gy = s->wig[w].gy;
-  a.gz = s->wig[w].gz;
-  a.gx1 = s->wig[w1].gx;
-  a.gy1 = s->wig[w1].gy;
-  a.gz1 = s->wig[w1].gz;
+  a.it.gx = s->wig[w].gx;
+  a.it.gy = s->wig[w].gy;
+  a.it.gz = s->wig[w].gz;
+  a.it.gx1 = s->wig[w1].gx;
+  a.it.gy1 = s->wig[w1].gy;
+  a.it.gz1 = s->wig[w1].gz;
   a.dE_in = in;
-  a.src = src;
+  a.it.src = src;
   a.A = make_float2(0.f, a_mult * (float)(1.0f / s->eps / (float)s->nw));  // 1i/epsilon/Nwiggles
   a.T = T;
   a.dE = s->d_dE;
   a.E = s->d_E;
   a.gamma = s->d_gamma;
   a.st = s->d_state;
-  a.partials = partials_of(s, w);
+  a.it.partials = partials_of(s, w);
   a.pitch = s->lay.pitch;
   a.fstride = (long long)field_elems(s);
   a.tstride = t_stride(s);
@@ -1257,11 +1349,16 @@ static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, cons
   a.total = s->g.nx * s->g.nz * s->g.nc;
   a.lines = p.lines;
   a.bpr = (int)p.grid;
-  a.acc2 = acc_of(s, w);
-  return launch_uni(s, uni::kernels(p.plan.cls).col[mode], p, &a);
+  a.it.acc = acc_of(s, w);
+  return a;
+}
+static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, const float2* in, const float2* src,
+                                  float2* T, float a_mult) {
+  uni::ColArgs a = uni_col_args(s, w, w1, in, src, T, a_mult);
+  return launch_uni(s, uni_kernels(a.py.cls).col[mode], s->lay.ucol, &a);
 }
 
-static cudaError_t launch_uni_x(const Solver* s, bool inv, float2* T) {
+static uni::XArgs uni_x_args(const Solver* s, float2* T) {
   const UniPass& p = s->lay.ux;
   uni::XArgs a{};
   a.px = p.plan;
@@ -1271,18 +1368,22 @@ static cudaError_t launch_uni_x(const Solver* s, bool inv, float2* T) {
   a.tstride = t_stride(s);
   a.ny = s->g.ny;
   a.nx = s->g.nx;
-  a.ty = p.lines;
-  a.nyt = (s->g.ny + p.lines - 1) / p.lines;
+  a.lty = log2_of(p.lines);
+  a.nyt = p.lines ? (s->g.ny + p.lines - 1) / p.lines : 0;
   a.bpr = (int)p.grid;
-  return launch_uni(s, uni::kernels(p.plan.cls).x[inv ? 1 : 0], p, &a);
+  return a;
+}
+static cudaError_t launch_uni_x(const Solver* s, bool inv, float2* T) {
+  uni::XArgs a = uni_x_args(s, T);
+  return launch_uni(s, uni_kernels(a.px.cls).x[inv ? 1 : 0], s->lay.ux, &a);
 }
 
-static cudaError_t launch_uni_k2(const Solver* s, int w) {
+static uni::PencilArgs uni_pencil_args(const Solver* s, int w) {
   const UniPass& p = s->lay.uout;
   uni::PencilArgs a{};
   a.g = s->g;
   a.po = p.plan;
-  a.w = s->uwig[w];
+  a.w = s->ut[s->active].uwig[w];
   a.k02e = s->k02e;
   const double kk = (double)s->k02e.x * s->k02e.x + (double)s->k02e.y * s->k02e.y;
   if (kk > 0) a.ik02e = make_float2((float)(s->k02e.x / kk), (float)(-s->k02e.y / kk));
@@ -1292,12 +1393,16 @@ static cudaError_t launch_uni_k2(const Solver* s, int w) {
   a.pitch = s->lay.pitch;
   a.tstride = t_stride(s);
   a.cstride = s->lay.pitch * s->g.nx * s->g.nz;
-  a.ty = p.lines;
+  a.lty = log2_of(p.lines);
   a.nyt = (s->g.ny + p.lines - 1) / p.lines;
   a.bpr = (int)p.grid;
   a.mode3d = s->lay.mode3d;
   a.pstd = s->pstd;
-  return launch_uni(s, uni::kernels(p.plan.cls).pencil[s->g.nc == 3 ? 1 : 0], p, &a);
+  return a;
+}
+static cudaError_t launch_uni_k2(const Solver* s, int w) {
+  uni::PencilArgs a = uni_pencil_args(s, w);
+  return launch_uni(s, uni_kernels(a.po.cls).pencil[s->g.nc == 3 ? 1 : 0], s->lay.uout, &a);
 }
 
 // K1 on explicit buffers: out = inner FFT of (in + a_mult A src) times the
@@ -1434,8 +1539,7 @@ static cudaError_t launch_finish(const Solver* s, const StopRule& rule, const Hi
   int nparts = (int)s->lay.grid_inner;
   long long stride = s->lay.grid_inner * s->nrhs;
   void* args[] = {&st, &r, &hh, &partials, &nparts, &stride, &slots, &guard};
-  const int th = slots > 1 ? 1024 : 256;  // 256 threads per iteration, four at a time
-  return launch_pdl(s, (const void*)k_finish_iterations, dim3(s->nrhs), dim3(th), args, 0);
+  return launch_pdl(s, (const void*)k_finish_iterations, dim3(s->nrhs), dim3(256), args, 0);
 }
 // ... of a whole cycle, with the guard of the graph's while loop
 static cudaError_t launch_cycle_end(const Solver* s, const StopRule& rule, const Hist& h, CycleGuard guard) {
@@ -1614,6 +1718,65 @@ static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source) 
   e = launch_k2(s, w);
   if (e != cudaSuccess) return e;
   return launch_k3_only(s, w);
+}
+
+// Whether nrhs right-hand sides can run as one launch of the loop
+// (uni::k_loop): a column tile of each on an SM of its own.
+static bool loop_fits(const Solver* s, int nrhs) {
+  return s->has_loop && nrhs <= uni::kLoopRhs && nrhs * s->lays[1].ucol.grid <= kNumSms &&
+         loop_smem(s->lays[1], s->g, s->nw, false) <= kLoopSmem;
+}
+
+// Cycles of the loop in one cooperative launch, from T as K1 left it, until
+// every right-hand side is done or max_cycles have run.
+static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist& h, long long max_cycles) {
+  const Layout& L = s->lay;
+  uni::LoopArgs a{};
+  a.col = uni_col_args(s, 0, 0, nullptr, nullptr, s->d_T, 1.f);
+  a.pen = uni_pencil_args(s, 0);
+  a.wig = s->ut[1].wigs;
+  a.uwig = s->ut[1].wigs + s->nw;
+  a.src = s->d_src;
+  a.partials = s->d_partials;
+  a.st = s->d_state;
+  a.rule = rule;
+  a.hist = h;
+  a.err = s->d_err;
+  a.arrived = (unsigned*)(s->d_err + 1);
+  a.max_cycles = max_cycles;
+  a.nw = s->nw;
+  a.nrhs = s->nrhs;
+  const void* fn = uni_kernels(std::max(L.ucol.plan.cls, L.uout.plan.cls)).loop;
+  a.groups = uni_groups(L.ucol);
+  a.e_resident = loop_smem(L, s->g, s->nw, true) <= kLoopSmem;
+  const size_t smem = loop_smem(L, s->g, s->nw, a.e_resident != 0, &a.tile_elems);
+  const long long tiles = std::max(L.ucol.grid, L.uout.grid) * s->nrhs;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)std::min<long long>(tiles, kNumSms));
+  const bool cluster = tiles <= 16;
+  cudaError_t e = cudaSuccess;
+  if (cluster)
+    a.arrived = nullptr;
+  else if ((e = cudaMemsetAsync(a.arrived, 0, sizeof(unsigned), s->stream)) != cudaSuccess)
+    return e;
+  // a butterfly per thread, or 512
+  const int work = std::max(L.ucol.lines * uni_units(L.ucol.plan), L.uout.lines * uni_units(L.uout.plan));
+  cfg.blockDim = dim3(work <= 256 ? 256 : uni::kLoopThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->stream;
+  cudaLaunchAttribute attr[1];
+  if (cluster) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cfg.gridDim.x;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* argv[] = {&a};
+  return cudaLaunchKernelExC(&cfg, fn, argv);
 }
 
 // Energy histories: per right-hand side r, diff at r * 2cap and fresh at r * 2cap + cap.
@@ -1876,6 +2039,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   if (want_cb && nrhs > 1) return fail(WS_ERR_INVALID_ARGUMENT, "callbacks need a single right-hand side");
   if (s->lay.grid_inner * (long long)nrhs > (1LL << 31) - 1 || s->lay.grid_outer * (long long)nrhs > (1LL << 31) - 1)
     return fail(WS_ERR_INVALID_ARGUMENT, "batch too large for one launch");
+  use_layout(s, loop_fits(s, nrhs) ? 1 : 0);
   int rc = ensure_batch(s, nrhs);
   if (rc) return rc;
   rc = ensure_partials(s, s->lay.grid_inner * (long long)nrhs * s->nw);
@@ -1916,9 +2080,33 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
         (long long)field_elems(s), s->n_media > 1 ? (long long)s->g.npts : 0LL);
     WS_CUDA(cudaGetLastError());
   }
-  if (opt.use_graph && !want_cb) {
+  const bool in_one = s->active == 1 && s->fuse;  // the loop as one launch, or one per cycle
+  if (opt.use_graph && !want_cb && in_one) {
+    if (s->warm) {
+      WS_CUDA(launch_prologue(s, rule, h, CycleGuard{}));
+    } else {
+      const size_t nbytes = field_elems(s) * nrhs * sizeof(float2);
+      WS_CUDA(cudaMemsetAsync(s->d_E, 0, nbytes, s->stream));
+      WS_CUDA(cudaMemsetAsync(s->d_dE, 0, nbytes, s->stream));
+      k_reset_state<<<1, 256, 0, s->stream>>>(s->d_state, nrhs);
+      WS_CUDA(launch_k1(s, 0, true));
+    }
+    // as many launches as the iteration bound can take, each of a bounded length
+    const long long max_cycles = (rule.max_iter + s->nw - 1) / s->nw + 1;
+    for (long long cycle = 0; cycle < max_cycles; cycle += kLoopCycles) {
+      WS_CUDA(launch_loop(s, rule, h, std::min(kLoopCycles, max_cycles - cycle)));
+      if (max_cycles <= kLoopCycles) break;
+      int kerr = 0;
+      WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
+      WS_CUDA(cudaMemcpyAsync(&kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+      WS_CUDA(cudaStreamSynchronize(s->stream));
+      bool all = true;
+      for (const DevState& d : hs) all = all && d.done;
+      if (all || kerr) break;
+    }
+  } else if (opt.use_graph && !want_cb) {
     GraphKey key{rule.threshold, rule.max_iter, rule.interval, opt.stop_rule, rule.nan_stop, nrhs,
-                 s->warm ? 1 : 0, s->warm ? s->warm_ratio : 0.0};
+                 s->warm ? 1 : 0, s->active, s->warm ? s->warm_ratio : 0.0};
     if (!s->gexec || !(key == s->gkey)) {
       rc = build_graph(s, rule, h);
       if (rc) return rc;
@@ -1927,20 +2115,19 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     WS_CUDA(cudaGraphLaunch(s->gexec, s->stream));
   } else {
     std::vector<double> hist;
-    long long it = 0;
     const long long cb_int = std::max<int64_t>(1, opt.callback_interval);
     const long long max_cycles = (rule.max_iter + s->nw - 1) / s->nw + 1;
     for (long long cycle = 0;; ++cycle) {
       if (cycle >= max_cycles) return fail(WS_ERR_CUDA, "loop did not stop within max_iterations (internal error)");
       if (cycle == 0) {
         WS_CUDA(launch_prologue(s, rule, h, CycleGuard{}));
-        it += s->nw;
       } else {
-        for (int i = 0; i < s->nw; ++i) {
-          WS_CUDA(launch_steady(s, (int)(it % s->nw)));
-          ++it;
+        if (in_one) {
+          WS_CUDA(launch_loop(s, rule, h, 1));
+        } else {
+          for (int i = 0; i < s->nw; ++i) WS_CUDA(launch_steady(s, i));
+          WS_CUDA(launch_cycle_end(s, rule, h, CycleGuard{}));
         }
-        WS_CUDA(launch_cycle_end(s, rule, h, CycleGuard{}));
       }
       WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
       WS_CUDA(cudaStreamSynchronize(s->stream));
@@ -2152,8 +2339,9 @@ int ws_solver_launches_per_iteration(ws_solver h) {
   // K2, K3 + next K1 (one kernel, or the split step's three); or K1, K2, K3
   // (the stop rule is one launch per wiggle cycle)
   if (!s->fuse) return 3;
-  if (!s->lay.mode3d) return 2;
-  return s->lay.xp || s->lay.uni_in ? 4 : 2;
+  const Layout& L = s->lays[0];
+  if (!L.mode3d) return 2;
+  return L.xp || L.uni_in ? 4 : 2;
 }
 
 int ws_solver_fused(ws_solver h) {
@@ -2166,6 +2354,7 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
   Solver* s = reinterpret_cast<Solver*>(h);
   if (!s->fuse) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not fuse K3 with K1");
   WS_CUDA(cudaSetDevice(s->device));
+  use_layout(s, 0);
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2204,6 +2393,7 @@ int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double 
   Solver* s = reinterpret_cast<Solver*>(h);
   if (!s->fuse || !s->lay.mode3d || !(s->lay.xp || s->lay.uni_in)) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
   WS_CUDA(cudaSetDevice(s->device));
+  use_layout(s, 0);
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2249,6 +2439,7 @@ int ws_solver_time_kernels(ws_solver h, int n_iterations, float ms_out[3], doubl
   if (!h || !ms_out || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
   WS_CUDA(cudaSetDevice(s->device));
+  use_layout(s, 0);
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2440,10 +2631,9 @@ static bool apply_choice(Solver* s, const LayoutChoice& c) {
   // another cluster size would run them on lines of another length
   if (L.mode3d && !L.fi && !L.uni_in && s->g.nx / L.csize != s->pxl.n) return false;
   if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap) * s->nw) != WS_OK) return false;
-  s->lay = L;
-  if (ensure_uni(s) != cudaSuccess) return false;
+  s->lays[0] = L;
+  if (set_layouts(s, c) != cudaSuccess) return false;
   apply_sched(s, c.sched);
-  update_fuse(s);
   free_graph(s);
   return true;
 }
@@ -2455,6 +2645,7 @@ int ws_solver_autotune(ws_solver h, int n_iterations, int* n_tried, float* ms_be
   if (!h || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
   WS_CUDA(cudaSetDevice(s->device));
+  use_layout(s, 0);
   if (s->hist_cap < 2) {
     const int rc = ensure_hist(s, 2);
     if (rc) return rc;

@@ -311,7 +311,7 @@ static cudaError_t iteration(Run& r, int w, const Wig* wig, bool with_source, fl
         launch_inner(r, true, args, r.sh.fast ? fast_inv(r.sh) : nullptr, gen, r.sh.fast ? fast::kThreads : r.sh.th);
     if (e != cudaSuccess) return e;
   }
-  k_finish_iterations<<<1, 1024, 0, r.stream>>>(r.st, rule, h, r.partials, (int)r.sh.grid_inner, 0, 1, CycleGuard{});
+  k_finish_iterations<<<1, 256, 0, r.stream>>>(r.st, rule, h, r.partials, (int)r.sh.grid_inner, 0, 1, CycleGuard{});
   return cudaGetLastError();
 }
 

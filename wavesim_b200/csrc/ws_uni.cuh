@@ -48,11 +48,11 @@ constexpr int kMaxThreads = 256;
 
 struct Stage {
   int R;           // radix
-  int sub;         // distance between the elements of a butterfly; twiddles W^{j r}, j < sub, at tw[r sub + j]
+  int sub;         // distance between the elements of a butterfly
   int units;       // butterflies of a line: n / R
+  int two;         // its twiddles in the plan's table: W^{j r} at two + r sub + j
   int subp, blkp;  // sub and the block R sub in a padded column (Plan::pad)
   unsigned msub, munits;  // multipliers of the division by sub and units (magic)
-  const float2* tw;
 };
 
 struct Plan {
@@ -61,6 +61,8 @@ struct Plan {
   int pad;       // columns: one slot of padding after every last-stage butterfly (its radix even), else 0
   int np;        // elements of a padded column
   unsigned mrl;  // multiplier of the division by the last stage's radix
+  int ntw;       // elements of the twiddle table
+  const float2* tw;
   Stage st[kStages];
 };
 
@@ -70,18 +72,24 @@ __host__ __device__ constexpr unsigned magic(int d) {
 }
 __device__ __forceinline__ int quot(int a, unsigned m) { return m ? (int)__umulhi((unsigned)a, m) : a; }
 
+// what changes from one iteration to the next
+struct ColIter {
+  const float2 *gx, *gy, *gz;     // ramps of this iteration's wiggle (its conjugate ramps)
+  const float2 *gx1, *gy1, *gz1;  // ramps applied before the forward transform
+  const float2* src;              // added with weight A before the forward transform, or null
+  double* partials;               // ROI energy of each block's columns
+  int acc;                        // kAccEach ..
+};
+
 struct ColArgs {
   Geom g;
   Plan py;
-  const float2 *gx, *gy, *gz;     // ramps of this iteration's wiggle (its conjugate ramps)
-  const float2 *gx1, *gy1, *gz1;  // ramps applied before the forward transform
-  const float2* dE_in;            // forward pass: the field to transform
-  const float2* src;              // added with weight A before the forward transform, or null
+  ColIter it;
+  const float2* dE_in;  // forward pass: the field to transform
   float2 A;
   float2 *T, *dE, *E;
   const float2* gamma;
   const DevState* st;
-  double* partials;
   long long pitch;    // T: elements between columns
   long long fstride;  // fields: elements between right-hand sides
   long long tstride;  // T: elements between right-hand sides
@@ -89,7 +97,6 @@ struct ColArgs {
   int total;          // columns of a right-hand side
   int lines;          // columns per block
   int bpr;            // blocks per right-hand side
-  int acc2;
 };
 
 struct PencilArgs {
@@ -101,7 +108,7 @@ struct PencilArgs {
   float2* T;
   const DevState* st;
   long long pitch, tstride, cstride;  // cstride: elements between the components of T
-  int ty, nyt, bpr, mode3d, pstd;
+  int lty, nyt, bpr, mode3d, pstd;  // lty: log2 of the y per block
 };
 
 struct XArgs {
@@ -109,7 +116,32 @@ struct XArgs {
   float2* T;
   const DevState* st;
   long long pitch, tstride;
-  int ny, nx, ty, nyt, bpr;
+  int ny, nx, lty, nyt, bpr;
+};
+
+// The whole loop of a 2-D grid in one cooperative launch (k_loop): each block owns one
+// column tile, whose gamma and dE' (and E') stay in its shared memory from the
+// first iteration to the last, walks the pencils' tiles, and meets the others
+// at a barrier in global memory after each pass.
+constexpr int kLoopRhs = 16;  // right-hand sides that it takes
+constexpr int kLoopThreads = 512;
+struct LoopArgs {
+  ColArgs col;
+  PencilArgs pen;
+  const Wig* wig;   // nw of them: natural order,
+  const Wig* uwig;  //   and with the p tables in the order of T
+  const float2* src;
+  double* partials;  // slot i: bpr nrhs energies of iteration i of a cycle
+  DevState* st;
+  StopRule rule;
+  Hist hist;
+  unsigned* arrived;  // zero at launch
+  int* err;
+  long long max_cycles;  // of this launch
+  int tile_elems;        // shared memory: the passes' tile, in float2
+  int groups;            // energies of 32 butterflies of a column tile
+  int e_resident;        // E' fits too
+  int nw, nrhs;
 };
 
 enum { kFwd = 0, kInv = 1, kStep = 2 };
@@ -121,8 +153,10 @@ struct Kernels {
   const void* col[3];     // by kFwd, kInv, kStep
   const void* x[2];       // forward, inverse
   const void* pencil[2];  // one component, three
+  const void* loop;
 };
-const Kernels& kernels(int cls);
+template <int RM>
+Kernels kernels_up_to();
 
 }  // namespace uni
 }  // namespace ws
