@@ -254,11 +254,9 @@ class MediaBatch:
         o = first._options()
         r = first.roi
         shape = tuple(int(r[1, d] - r[0, d] + 1) for d in range(4))
-        if getattr(self, "_hstage", None) is None:
-            self._hstage = _lib.HostStage()
-        buf = self._hstage.get(R * np.prod(shape))
+        buf = np.empty(R * int(np.prod(shape)), np.complex64)
         cap = o.max_iterations + len(first.wiggles) + 1
-        hist = np.zeros((R, cap))
+        hist = np.empty((R, cap))
         n_it = np.zeros(R, dtype=np.int64)
         conv = np.zeros(R, dtype=np.int32)
         t0 = time.perf_counter()
@@ -266,7 +264,7 @@ class MediaBatch:
             self.h, R, (C.c_int64 * R)(*counts), blocks, _lib.WS_HOST, C.byref(o), buf.ctypes.data, _lib.WS_HOST,
             hist.ctypes.data_as(C.POINTER(C.c_double)), cap, n_it.ctypes.data_as(C.POINTER(C.c_int64)),
             conv.ctypes.data_as(C.POINTER(C.c_int))))
-        E = _lib.HostStage.take(buf, (R,) + shape[::-1])
+        E = buf.reshape((R,) + shape[::-1])
         dt = time.perf_counter() - t0
         del keep
         outs, states = [], []

@@ -17,7 +17,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(ROOT, "_build")
 NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-CFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include")]
+CFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-pthread", "-I" + os.path.join(ROOT, "include")]
 
 TARGETS = {
     "libwavesim_b200.so": ["ws_mbs.cu", "ws_uni_r8.cu", "ws_uni_r12.cu", "ws_uni_r16.cu", "ws_noalloc.cu", "ws_net.cu", "ws_setup.cu"],

@@ -14,11 +14,13 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <memory>
 #include <mutex>
 #include <vector>
 
 #include "wavesim_b200.h"
 #include "ws_fast.cuh"
+#include "ws_hostout.h"
 #include "ws_kernels.cuh"
 #include "ws_mixed.cuh"
 #include "ws_tma.cuh"
@@ -924,9 +926,6 @@ static cudaError_t permute_wiggles(Solver* s) {
 static cudaError_t make_tables(Solver* s, int k) {
   Layout& L = s->lays[k];
   UniTables& t = s->ut[k];
-  if (t.wigs) cudaFree(t.wigs);
-  t = UniTables{};
-  if (!L.uni_out) return cudaSuccess;
   const Geom& g = s->g;
   const int len[3] = {g.nx, g.ny, g.nz};  // the order of d_wigf
   const uni::Plan* axis[3] = {L.mode3d ? (L.uni_in ? &L.ux.plan : nullptr) : &L.uout.plan,
@@ -977,23 +976,30 @@ static cudaError_t make_tables(Solver* s, int k) {
   return e;
 }
 
-// Makes lays[k] the layout in use.
-static void use_layout(Solver* s, int k) {
+// Makes lays[k] the layout in use, with its tables (made on its first use:
+// few solvers run both).
+static cudaError_t use_layout(Solver* s, int k) {
+  if (s->lays[k].uni_out && !s->ut[k].wigs) {
+    cudaError_t e = make_tables(s, k);
+    if (e == cudaSuccess) e = permute_wiggles(s);
+    if (e != cudaSuccess) return e;
+  }
   s->active = k;
   s->lay = s->lays[k];
   s->fuse = s->fuses[k];
+  return cudaSuccess;
 }
 
 // The layouts for choice ch of the launched passes (lays[0], made by the
-// caller), with their tables; the launched passes' is then in use.
+// caller); the one of single solves is then in use.
 static cudaError_t set_layouts(Solver* s, const LayoutChoice& ch) {
   s->has_loop = loop_layout(s->g, s->lays[0], ch, s->pstd != 0, s->lays[1]);
-  cudaError_t e = make_tables(s, 0);
-  if (e == cudaSuccess && s->has_loop) e = make_tables(s, 1);
-  if (e == cudaSuccess) e = permute_wiggles(s);
-  for (int k = 0; k < 2; ++k) s->fuses[k] = fuse_of(s, s->lays[k]);
-  use_layout(s, 0);
-  return e;
+  for (int k = 0; k < 2; ++k) {
+    if (s->ut[k].wigs) cudaFree(s->ut[k].wigs);
+    s->ut[k] = UniTables{};
+    s->fuses[k] = fuse_of(s, s->lays[k]);
+  }
+  return use_layout(s, s->has_loop ? 1 : 0);
 }
 
 // Buffers for nrhs right-hand sides (kept when large enough).
@@ -1029,7 +1035,7 @@ static int ensure_batch(Solver* s, int nrhs) {
   WS_CUDA(cudaMalloc(&s->d_src, nb));
   WS_CUDA(cudaMalloc(&s->d_state, nrhs * sizeof(DevState)));
   WS_CUDA(cudaMalloc(&s->d_energy, nrhs * sizeof(double)));
-  s->partials_cap = std::max<long long>(1, s->lay.grid_inner) * nrhs * s->nw;
+  s->partials_cap = std::max<long long>(1, std::max(s->lays[0].grid_inner, s->lays[1].grid_inner)) * nrhs * s->nw;
   WS_CUDA(cudaMalloc(&s->d_partials, (size_t)s->partials_cap * sizeof(double)));
   WS_CUDA(cudaMemset(s->d_E, 0, nb));
   WS_CUDA(cudaMemset(s->d_dE, 0, nb));
@@ -1930,7 +1936,7 @@ static int upload_sources(Solver* s, int nrhs, const int64_t* counts, const ws_s
   const size_t F = field_elems(s);
   WS_CUDA(cudaMemsetAsync(s->d_src, 0, F * nrhs * sizeof(float2), s->stream));
   WS_CUDA(cudaMemsetAsync(s->d_energy, 0, nrhs * sizeof(double), s->stream));
-  size_t need = 0;
+  size_t need = 0, sum = 0;
   long long total = 0;
   for (int r = 0; r < nrhs; ++r) total += counts[r];
   for (long long b = 0; b < total; ++b) {
@@ -1944,6 +1950,7 @@ static int upload_sources(Solver* s, int nrhs, const int64_t* counts, const ws_s
     }
     if (!B.values) return fail(WS_ERR_INVALID_ARGUMENT, "null source values");
     need = std::max(need, n);
+    sum += n;
   }
   if (need > s->stage_cap && memory != WS_DEVICE) {
     if (s->d_stage) cudaFree(s->d_stage);
@@ -1952,12 +1959,20 @@ static int upload_sources(Solver* s, int nrhs, const int64_t* counts, const ws_s
     WS_CUDA(cudaMalloc(&s->d_stage, need * sizeof(float2)));
     s->stage_cap = need;
   }
+  // the energies (only whether there is a source) of small host blocks come
+  // from the host, so that nothing waits for the device here; the copies and
+  // kernels share the staging buffer in stream order, and a pageable copy has
+  // taken its values when it returns
+  energy.assign(nrhs, 0.0);
+  const bool on_host = memory != WS_DEVICE && sum <= (1u << 16);
   long long b = 0;
   for (int r = 0; r < nrhs; ++r) {
     for (int64_t k = 0; k < counts[r]; ++k, ++b) {
       const ws_source_block& B = src[b];
       const size_t n = (size_t)(B.size[0] * B.size[1] * B.size[2] * B.size[3]);
       const float2* vals = (const float2*)B.values;
+      if (on_host)
+        for (size_t i = 0; i < n; ++i) energy[r] += (double)std::fmaf(vals[i].x, vals[i].x, vals[i].y * vals[i].y);
       if (memory != WS_DEVICE) {
         WS_CUDA(cudaMemcpyAsync(s->d_stage, B.values, n * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
         vals = s->d_stage;
@@ -1968,10 +1983,9 @@ static int upload_sources(Solver* s, int nrhs, const int64_t* counts, const ws_s
           s->d_src + F * r, vals, g, (int)B.position[0] - 1, (int)B.position[1] - 1, (int)B.position[2] - 1,
           (int)B.position[3] - 1, (int)B.size[0], (int)B.size[1], (int)B.size[2], (int)B.size[3], s->d_energy + r);
       WS_CUDA(cudaGetLastError());
-      if (memory != WS_DEVICE) WS_CUDA(cudaStreamSynchronize(s->stream));  // staging buffer reuse
     }
   }
-  energy.assign(nrhs, 0.0);
+  if (on_host) return WS_OK;
   WS_CUDA(cudaMemcpyAsync(energy.data(), s->d_energy, nrhs * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   WS_CUDA(cudaStreamSynchronize(s->stream));
   return WS_OK;
@@ -2039,7 +2053,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   if (want_cb && nrhs > 1) return fail(WS_ERR_INVALID_ARGUMENT, "callbacks need a single right-hand side");
   if (s->lay.grid_inner * (long long)nrhs > (1LL << 31) - 1 || s->lay.grid_outer * (long long)nrhs > (1LL << 31) - 1)
     return fail(WS_ERR_INVALID_ARGUMENT, "batch too large for one launch");
-  use_layout(s, loop_fits(s, nrhs) ? 1 : 0);
+  WS_CUDA(use_layout(s, loop_fits(s, nrhs) ? 1 : 0));
   int rc = ensure_batch(s, nrhs);
   if (rc) return rc;
   rc = ensure_partials(s, s->lay.grid_inner * (long long)nrhs * s->nw);
@@ -2065,7 +2079,6 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   rule.threshold = opt.energy_threshold;
   const long long hs_stride = 2 * s->hist_cap;
   Hist h{s->d_hist, s->d_hist + s->hist_cap, s->hist_cap, hs_stride};
-  std::vector<DevState> hs(nrhs);
   s->warm = opt.initial_field != nullptr;
   s->warm_ratio = opt.warm_discard_ratio;
   if (s->warm) {
@@ -2081,6 +2094,72 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     WS_CUDA(cudaGetLastError());
   }
   const bool in_one = s->active == 1 && s->fuse;  // the loop as one launch, or one per cycle
+  // What comes back with the first wait: the states, the error flag and the
+  // first kHead energies of each right-hand side.
+  constexpr size_t kHead = 4096;
+  const bool head = diff_out && nrhs <= 16;
+  const size_t state_bytes = (nrhs * sizeof(DevState) + 15) / 16 * 16;
+  HostLease back(state_bytes + 16 + (head ? nrhs * kHead * sizeof(double) : 0));
+  if (!back.p) return fail(WS_ERR_OUT_OF_MEMORY, "no page-locked memory for the loop's state");
+  const DevState* const hs = (const DevState*)back.p;
+  const int* const kerr = (const int*)((char*)back.p + state_bytes);
+  const double* const hhead = (const double*)((char*)back.p + state_bytes + 16);
+  const long long nhead = std::min<long long>((long long)kHead, s->hist_cap);
+  auto fetch_state = [&]() -> cudaError_t {
+    cudaError_t e = cudaMemcpyAsync((void*)hs, s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync((void*)kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
+    for (int r = 0; head && r < nrhs && e == cudaSuccess; ++r)
+      e = cudaMemcpyAsync((void*)(hhead + r * kHead), s->d_hist + r * hs_stride, nhead * sizeof(double),
+                          cudaMemcpyDeviceToHost, s->stream);
+    return e;
+  };
+  auto all_done = [&]() {
+    bool all = true;
+    for (int r = 0; r < nrhs; ++r) all = all && hs[r].done;
+    return all;
+  };
+  // The fields: E' itself, or E on the roi through k_finalize (in groups of
+  // right-hand sides for host memory, so that the device copy stays below 512 MB).
+  const size_t F = field_elems(s);
+  const bool field = opt.output == WS_OUTPUT_FIELD;
+  const size_t per = (field ? roi_elems(s->g) : F) * sizeof(float2);  // bytes of a right-hand side
+  const bool to_host = E_out && out_memory != WS_DEVICE;
+  const int group = (int)std::min<size_t>(nrhs, std::max<size_t>(1, (512u << 20) / per));
+  if (to_host && field && group * (per / sizeof(float2)) > s->out_cap) {
+    if (s->d_out) cudaFree(s->d_out);
+    s->d_out = nullptr;
+    s->out_cap = 0;
+    WS_CUDA(cudaMalloc(&s->d_out, group * per));
+    s->out_cap = group * (per / sizeof(float2));
+  }
+  bool pageable = false;
+  if (to_host) {
+    cudaPointerAttributes at{};
+    pageable = cudaPointerGetAttributes(&at, E_out) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+  }
+  // E of right-hand sides r0 .. r1 - 1 where the caller wants it, or in d_out
+  auto finalize = [&](int r0, int r1) -> cudaError_t {
+    for (int r = r0; r < r1 && field; ++r) {
+      const size_t n = per / sizeof(float2);
+      const long long blocks = std::min<long long>(((long long)n + 255) / 256, 8 * kNumSms);
+      k_finalize<<<(unsigned)blocks, 256, 0, s->stream>>>(
+          s->d_E + F * r, s->d_gamma + (s->n_media > 1 ? (long long)r * s->g.npts : 0LL), s->g,
+          to_host ? s->d_out + n * (r - r0) : (float2*)E_out + n * r);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+  };
+  std::unique_ptr<OutCopy> copy;  // of the first group: its threads touch the caller's pages meanwhile
+  auto begin_copy = [&]() -> cudaError_t {
+    if (!pageable) return cudaSuccess;
+    if (!copy) copy.reset(new OutCopy(E_out, per * group, s->device));
+    if (!copy->ok()) return cudaErrorMemoryAllocation;
+    const cudaError_t e = copy->stage(field ? (const void*)s->d_out : (const void*)s->d_E, s->stream);
+    copy->touch();
+    return e;
+  };
   if (opt.use_graph && !want_cb && in_one) {
     if (s->warm) {
       WS_CUDA(launch_prologue(s, rule, h, CycleGuard{}));
@@ -2095,14 +2174,11 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     const long long max_cycles = (rule.max_iter + s->nw - 1) / s->nw + 1;
     for (long long cycle = 0; cycle < max_cycles; cycle += kLoopCycles) {
       WS_CUDA(launch_loop(s, rule, h, std::min(kLoopCycles, max_cycles - cycle)));
-      if (max_cycles <= kLoopCycles) break;
-      int kerr = 0;
-      WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
-      WS_CUDA(cudaMemcpyAsync(&kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+      if (E_out) WS_CUDA(finalize(0, to_host ? group : nrhs));
+      WS_CUDA(fetch_state());
+      WS_CUDA(begin_copy());
       WS_CUDA(cudaStreamSynchronize(s->stream));
-      bool all = true;
-      for (const DevState& d : hs) all = all && d.done;
-      if (all || kerr) break;
+      if (all_done() || *kerr) break;
     }
   } else if (opt.use_graph && !want_cb) {
     GraphKey key{rule.threshold, rule.max_iter, rule.interval, opt.stop_rule, rule.nan_stop, nrhs,
@@ -2113,6 +2189,10 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
       s->gkey = key;
     }
     WS_CUDA(cudaGraphLaunch(s->gexec, s->stream));
+    if (E_out) WS_CUDA(finalize(0, to_host ? group : nrhs));
+    WS_CUDA(fetch_state());
+    WS_CUDA(begin_copy());
+    WS_CUDA(cudaStreamSynchronize(s->stream));
   } else {
     std::vector<double> hist;
     const long long cb_int = std::max<int64_t>(1, opt.callback_interval);
@@ -2129,7 +2209,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
           WS_CUDA(launch_cycle_end(s, rule, h, CycleGuard{}));
         }
       }
-      WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
+      WS_CUDA(fetch_state());
       WS_CUDA(cudaStreamSynchronize(s->stream));
       if (want_cb) {
         const long long done_it = hs[0].it - 1;
@@ -2139,16 +2219,11 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
           if (k >= 1 && (k % cb_int == 0 || (hs[0].done && k == done_it)))
             opt.callback(opt.callback_type, hist.data(), k, opt.energy_threshold, opt.user_data);
       }
-      bool all = true;
-      for (const DevState& d : hs) all = all && d.done;
-      if (all) break;
+      if (all_done() || (in_one && *kerr)) break;
     }
+    if (E_out) WS_CUDA(finalize(0, to_host ? group : nrhs));
   }
-  WS_CUDA(cudaMemcpyAsync(hs.data(), s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream));
-  int kerr = 0;
-  WS_CUDA(cudaMemcpyAsync(&kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  WS_CUDA(cudaStreamSynchronize(s->stream));
-  if (kerr) {
+  if (*kerr) {
     cudaMemset(s->d_err, 0, sizeof(int));
     return fail(WS_ERR_CUDA, "a bounded wait of the FFT kernels (cluster exchange or TMA tile load) timed out");
   }
@@ -2158,40 +2233,35 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     if (n_it) n_it[r] = n_iter;
     if (converged) converged[r] = hs[r].converged;
     diverged = diverged || hs[r].status == WS_ERR_DIVERGED;
-    if (diff_out && n_iter > 0)
-      WS_CUDA(cudaMemcpy(diff_out + r * diff_cap, s->d_hist + r * hs_stride,
-                         std::min<long long>(std::min(n_iter, cap), diff_cap) * sizeof(double),
+    const long long nd = std::min<long long>(std::min(n_iter, cap), diff_cap);
+    if (!diff_out || nd <= 0) continue;
+    if (head && nd <= nhead)
+      std::memcpy(diff_out + r * diff_cap, hhead + r * kHead, nd * sizeof(double));
+    else
+      WS_CUDA(cudaMemcpy(diff_out + r * diff_cap, s->d_hist + r * hs_stride, nd * sizeof(double),
                          cudaMemcpyDeviceToHost));
   }
   if (E_out) {
-    const Geom& g = s->g;
-    const cudaMemcpyKind k = out_memory == WS_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    const size_t F = field_elems(s);
-    if (opt.output == WS_OUTPUT_FIELD) {
-      const size_t n = roi_elems(g);
-      for (int r = 0; r < nrhs; ++r) {
-        float2* dst = (float2*)E_out + n * r;
-        if (out_memory != WS_DEVICE) {
-          if (n > s->out_cap) {
-            if (s->d_out) cudaFree(s->d_out);
-            s->d_out = nullptr;
-            s->out_cap = 0;
-            WS_CUDA(cudaMalloc(&s->d_out, n * sizeof(float2)));
-            s->out_cap = n;
-          }
-          dst = s->d_out;
+    for (int r0 = 0; to_host && r0 < nrhs; r0 += group) {
+      const int r1 = std::min(nrhs, r0 + group);
+      if (r0 > 0) WS_CUDA(finalize(r0, r1));
+      char* const dst = (char*)E_out + per * r0;
+      const void* const from = field ? (const void*)s->d_out : (const void*)(s->d_E + F * r0);
+      if (pageable) {
+        if (r0 > 0 || !copy) {
+          copy.reset(new OutCopy(dst, per * (r1 - r0), s->device));
+          if (!copy->ok()) return fail(WS_ERR_OUT_OF_MEMORY, "no page-locked memory for the fields");
+          WS_CUDA(copy->stage(from, s->stream));
+          WS_CUDA(cudaStreamSynchronize(s->stream));
         }
-        const long long blocks = std::min<long long>(((long long)n + 255) / 256, 8 * kNumSms);
-        k_finalize<<<(unsigned)blocks, 256, 0, s->stream>>>(
-            s->d_E + F * r, s->d_gamma + (s->n_media > 1 ? (long long)r * s->g.npts : 0LL), g, dst);
-        WS_CUDA(cudaGetLastError());
-        if (out_memory != WS_DEVICE)
-          WS_CUDA(cudaMemcpyAsync((float2*)E_out + n * r, s->d_out, n * sizeof(float2), k, s->stream));
-        WS_CUDA(cudaStreamSynchronize(s->stream));
+        WS_CUDA(copy->run());
+      } else {
+        WS_CUDA(cudaMemcpyAsync(dst, from, per * (r1 - r0), cudaMemcpyDeviceToHost, s->stream));
+        WS_CUDA(cudaStreamSynchronize(s->stream));  // d_out takes the next group
       }
-    } else {
-      WS_CUDA(cudaMemcpyAsync(E_out, s->d_E, F * nrhs * sizeof(float2), k, s->stream));
     }
+    if (!to_host && !field)
+      WS_CUDA(cudaMemcpyAsync(E_out, s->d_E, F * nrhs * sizeof(float2), cudaMemcpyDeviceToDevice, s->stream));
     WS_CUDA(cudaStreamSynchronize(s->stream));
   }
   if (diverged) return fail(WS_ERR_DIVERGED, "residual energy is not finite");
@@ -2354,7 +2424,7 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
   Solver* s = reinterpret_cast<Solver*>(h);
   if (!s->fuse) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not fuse K3 with K1");
   WS_CUDA(cudaSetDevice(s->device));
-  use_layout(s, 0);
+  WS_CUDA(use_layout(s, 0));
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2393,7 +2463,7 @@ int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double 
   Solver* s = reinterpret_cast<Solver*>(h);
   if (!s->fuse || !s->lay.mode3d || !(s->lay.xp || s->lay.uni_in)) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
   WS_CUDA(cudaSetDevice(s->device));
-  use_layout(s, 0);
+  WS_CUDA(use_layout(s, 0));
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2439,7 +2509,7 @@ int ws_solver_time_kernels(ws_solver h, int n_iterations, float ms_out[3], doubl
   if (!h || !ms_out || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
   WS_CUDA(cudaSetDevice(s->device));
-  use_layout(s, 0);
+  WS_CUDA(use_layout(s, 0));
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2632,7 +2702,7 @@ static bool apply_choice(Solver* s, const LayoutChoice& c) {
   if (L.mode3d && !L.fi && !L.uni_in && s->g.nx / L.csize != s->pxl.n) return false;
   if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap) * s->nw) != WS_OK) return false;
   s->lays[0] = L;
-  if (set_layouts(s, c) != cudaSuccess) return false;
+  if (set_layouts(s, c) != cudaSuccess || use_layout(s, 0) != cudaSuccess) return false;
   apply_sched(s, c.sched);
   free_graph(s);
   return true;
@@ -2645,7 +2715,7 @@ int ws_solver_autotune(ws_solver h, int n_iterations, int* n_tried, float* ms_be
   if (!h || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
   WS_CUDA(cudaSetDevice(s->device));
-  use_layout(s, 0);
+  WS_CUDA(use_layout(s, 0));
   if (s->hist_cap < 2) {
     const int rc = ensure_hist(s, 2);
     if (rc) return rc;
@@ -2843,6 +2913,7 @@ void ws_run_algorithm_release(void) {
     destroy_solver(s);
     s = nullptr;
   }
+  host_pool().trim();
 }
 
 }  // extern "C"

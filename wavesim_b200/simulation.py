@@ -403,14 +403,14 @@ class WaveSim:
             shape = tuple(int(r[1, d] - r[0, d] + 1) for d in range(4))
         else:
             shape = tuple(int(v) for v in self.N)
-        buf = self._stage().get(np.prod(shape))
-        hist = np.zeros(o.max_iterations + len(self.wiggles) + 1)
+        buf = np.empty(int(np.prod(shape)), np.complex64)
+        hist = np.empty(o.max_iterations + len(self.wiggles) + 1)
         n_it = C.c_int64()
         conv = C.c_int()
         _lib.check(_lib.lib.ws_solver_solve(
             h, len(s.values), blocks, _lib.WS_HOST, C.byref(o), buf.ctypes.data, _lib.WS_HOST,
             hist.ctypes.data_as(C.POINTER(C.c_double)), C.byref(n_it), C.byref(conv)))
-        E = _lib.HostStage.take(buf, shape, "F")
+        E = buf.reshape(shape[::-1]).T
         del keep, cb_keep
         state.it = int(n_it.value) + 1  # Simulation.next leaves it one past the last iteration
         state.diff_energy = hist[:n_it.value].copy()
@@ -472,16 +472,16 @@ class WaveSim:
         init = self._batch_starts(o, warm_starts, R)
         r = self.roi
         shape = tuple(int(r[1, d] - r[0, d] + 1) for d in range(4))
-        buf = self._stage().get(R * np.prod(shape))
+        buf = np.empty(R * int(np.prod(shape)), np.complex64)
         cap = o.max_iterations + len(self.wiggles) + 1
-        hist = np.zeros((R, cap))
+        hist = np.empty((R, cap))
         n_it = np.zeros(R, dtype=np.int64)
         conv = np.zeros(R, dtype=np.int32)
         _lib.check(_lib.lib.ws_solver_solve_batch(
             h, R, (C.c_int64 * R)(*counts), blocks, _lib.WS_HOST, C.byref(o), buf.ctypes.data, _lib.WS_HOST,
             hist.ctypes.data_as(C.POINTER(C.c_double)), cap, n_it.ctypes.data_as(C.POINTER(C.c_int64)),
             conv.ctypes.data_as(C.POINTER(C.c_int))))
-        E = _lib.HostStage.take(buf, (R,) + shape[::-1])  # each field column-major
+        E = buf.reshape((R,) + shape[::-1])  # each field column-major
         del keep, init
         return self._batch_results(h, E, hist, n_it, conv, groups, time.perf_counter() - t0,
                                    warm_starts is not None, lambda idx: self.exec_batch([sources[i] for i in idx]))
@@ -610,7 +610,7 @@ class WaveSim:
         r = self.roi
         shape = tuple(int(r[1, d] - r[0, d] + 1) for d in range(4))
         cap = o.max_iterations + len(self.wiggles) + 1
-        hist = np.zeros((R, cap))
+        hist = np.empty((R, cap))
         n_it = np.zeros(R, dtype=np.int64)
         conv = np.zeros(R, dtype=np.int32)
         Edev = None
@@ -620,7 +620,7 @@ class WaveSim:
                                device=torch.device("cuda", self.device))
             out, mem = Edev.data_ptr(), _lib.WS_DEVICE
         else:
-            buf = self._stage().get(R * np.prod(shape))
+            buf = np.empty(R * int(np.prod(shape)), np.complex64)
             out, mem = buf.ctypes.data, _lib.WS_HOST
         _lib.check(_lib.lib.ws_solver_solve_plane_waves(
             h, R, arr, C.byref(o), out, mem, hist.ctypes.data_as(C.POINTER(C.c_double)), cap,
@@ -630,7 +630,8 @@ class WaveSim:
             import torch
             buf = self._stage().get(Edev.numel())
             torch.from_numpy(buf).copy_(Edev.reshape(-1))
-        E = _lib.HostStage.take(buf, (R,) + shape[::-1])
+            buf = _lib.HostStage.take(buf, (buf.size,))
+        E = buf.reshape((R,) + shape[::-1])
         outs, states = self._batch_results(
             h, E, hist, n_it, conv, list(waves), time.perf_counter() - t0, warm_starts is not None,
             lambda idx: self._exec_plane_waves([waves[i] for i in idx], None, time.perf_counter()))
