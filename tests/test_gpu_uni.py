@@ -123,3 +123,25 @@ def test_loop_over_several_launches_and_batches(gpu):
         assert t.it == s1.it and t.converged
         np.testing.assert_array_equal(e, E1)
     sim.close()
+
+
+@pytest.mark.filterwarnings("ignore:The PSTD code")
+@pytest.mark.parametrize("shape,bw", [((4, 6), [0, 0]), ((48, 40), [8, 8]), ((33, 150), [6, 0]), ((240, 240), [8, 8]),
+                                      ((736, 1068), [16, 16])])
+def test_pstd_in_one_launch_matches_launched_passes(gpu, shape, bw, monkeypatch):
+    """300 steps (two launches of at most 256), against the generic kernels' five launches a step.  Each step rounds to a
+    few 1e-7; their random sum over 300 steps is 5e-6, and 5e-5 leaves ten times that."""
+    import wavesim_b200 as ws
+    n = 1.0 + 0.2 * np.random.default_rng(2).random(shape) + 0.02j
+    opt = {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": bw, "boundary_type": "ARL", "energy_threshold": 1e-30,
+           "source_amplitude": lambda c: np.exp(-2.0j * np.pi * c)}
+    got = []
+    for path in ("", "generic"):
+        monkeypatch.setenv("WAVESIM_B200_PATH", path)
+        p = ws.PSTD(n, opt)
+        got.append(p.exec(ws.Source(np.ones((shape[0], 1)) + 0.5j, [1, 2]), max_iterations=300))
+        p.close()
+    (E, st), (Eg, sg) = got
+    assert st.it == sg.it
+    assert rel(E, Eg) < 5e-5, rel(E, Eg)
+    np.testing.assert_allclose(st.diff_energy, sg.diff_energy, rtol=1e-3)

@@ -463,6 +463,14 @@ static size_t loop_smem(const Layout& L, const Geom& g, int nw, bool e_resident,
          (uni_groups(L.ucol) + (size_t)nw * L.uout.plan.n) * sizeof(float);
 }
 constexpr size_t kLoopSmem = 225 * 1024;
+// ... of PSTD's stepping: two fields, the source and three coefficients a point
+static size_t pstd_loop_smem(const Layout& L, const Geom& g, int* tile_elems = nullptr) {
+  const size_t l = L.ucol.lines;
+  const size_t tile = std::max(l * L.ucol.plan.np, (size_t)L.uout.lines * L.uout.plan.n);
+  if (tile_elems) *tile_elems = (int)tile;
+  return (tile + L.ucol.plan.ntw + L.uout.plan.ntw + 4 * l * g.ny) * sizeof(float2) + l * 16 +
+         (uni_groups(L.ucol) + (size_t)L.uout.plan.n + l * g.ny) * sizeof(float);
+}
 // The layout of single solves of small 2-D grids, `L` being the one of the
 // grid's launched passes; false if there is none.  Measured against the
 // launched passes, us an iteration: 64 x 56 7.6 (12.8), 160 x 264 12.4 (21.4),
@@ -471,10 +479,10 @@ constexpr size_t kLoopSmem = 225 * 1024;
 // it takes every grid whose columns fit the SMs' shared memory, but those with
 // compile-time kernels in both passes only up to 400 000 points.
 static bool loop_layout(const Geom& g, const Layout& L, const LayoutChoice& ch, bool pstd, Layout& out) {
-  if (pstd || L.mode3d || g.nc != 1 || ch.inner == 2 || ch.outer == 2) return false;
+  if (L.mode3d || g.nc != 1 || ch.inner == 2 || ch.outer == 2) return false;
   const char* path = std::getenv("WAVESIM_B200_PATH");
   if (path && std::strcmp(path, "generic") == 0) return false;
-  if (L.fi && L.fp && g.npts > 400000) return false;
+  if (L.fi && L.fp && g.npts > 400000 && !pstd) return false;
   Layout t{};
   if (!uni_plan(g.nx, t.uout.plan) || !uni_plan(g.ny, t.ucol.plan)) return false;
   t.uni_in = t.uni_out = true;
@@ -483,7 +491,7 @@ static bool loop_layout(const Geom& g, const Layout& L, const LayoutChoice& ch, 
   // cluster and meet at its hardware barrier (64 x 56: 7.6 us against 8.6)
   const int sms = t.uout.grid <= 16 && g.npts <= 8192 ? 16 : kNumSms;
   uni_columns(t.ucol, g.nx, (g.nx + sms - 1) / sms);
-  if (loop_smem(t, g, 4, false) > kLoopSmem) return false;
+  if ((pstd ? pstd_loop_smem(t, g) : loop_smem(t, g, 4, false)) > kLoopSmem) return false;
   t.grid_inner = t.ucol.grid;
   t.grid_outer = t.uout.grid;
   t.rset = L.rset;
@@ -858,8 +866,10 @@ static int set_kernel_attributes() {
     for (const void* f : k.col) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.x) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.pencil) WS_CUDA(allow_dynamic_smem(f, optin));
-    WS_CUDA(allow_dynamic_smem(k.loop, optin));
-    WS_CUDA(cudaFuncSetAttribute(k.loop, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (const void* f : {k.loop, k.pstd_loop}) {
+      WS_CUDA(allow_dynamic_smem(f, optin));
+      WS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    }
   }
   for (const XPencil& f : x_pencil_table()) {
     WS_CUDA(allow_dynamic_smem(f.fwd, optin));
@@ -1733,38 +1743,20 @@ static bool loop_fits(const Solver* s, int nrhs) {
          loop_smem(s->lays[1], s->g, s->nw, false) <= kLoopSmem;
 }
 
-// Cycles of the loop in one cooperative launch, from T as K1 left it, until
-// every right-hand side is done or max_cycles have run.
-static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist& h, long long max_cycles) {
+// A launch of a loop kernel with arguments `args`, whose barrier counter is at
+// *arrived: cooperative, or one cluster where 16 blocks have all the tiles (then
+// without a counter).
+static cudaError_t launch_coop(const Solver* s, const void* fn, size_t smem, int nrhs, void* args, unsigned** arrived) {
   const Layout& L = s->lay;
-  uni::LoopArgs a{};
-  a.col = uni_col_args(s, 0, 0, nullptr, nullptr, s->d_T, 1.f);
-  a.pen = uni_pencil_args(s, 0);
-  a.wig = s->ut[1].wigs;
-  a.uwig = s->ut[1].wigs + s->nw;
-  a.src = s->d_src;
-  a.partials = s->d_partials;
-  a.st = s->d_state;
-  a.rule = rule;
-  a.hist = h;
-  a.err = s->d_err;
-  a.arrived = (unsigned*)(s->d_err + 1);
-  a.max_cycles = max_cycles;
-  a.nw = s->nw;
-  a.nrhs = s->nrhs;
-  const void* fn = uni_kernels(std::max(L.ucol.plan.cls, L.uout.plan.cls)).loop;
-  a.groups = uni_groups(L.ucol);
-  a.e_resident = loop_smem(L, s->g, s->nw, true) <= kLoopSmem;
-  const size_t smem = loop_smem(L, s->g, s->nw, a.e_resident != 0, &a.tile_elems);
-  const long long tiles = std::max(L.ucol.grid, L.uout.grid) * s->nrhs;
+  const long long tiles = std::max(L.ucol.grid, L.uout.grid) * nrhs;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)std::min<long long>(tiles, kNumSms));
   const bool cluster = tiles <= 16;
-  cudaError_t e = cudaSuccess;
-  if (cluster)
-    a.arrived = nullptr;
-  else if ((e = cudaMemsetAsync(a.arrived, 0, sizeof(unsigned), s->stream)) != cudaSuccess)
-    return e;
+  *arrived = cluster ? nullptr : (unsigned*)(s->d_err + 1);
+  if (!cluster) {
+    const cudaError_t e = cudaMemsetAsync(*arrived, 0, sizeof(unsigned), s->stream);
+    if (e != cudaSuccess) return e;
+  }
   // a butterfly per thread, or 512
   const int work = std::max(L.ucol.lines * uni_units(L.ucol.plan), L.uout.lines * uni_units(L.uout.plan));
   cfg.blockDim = dim3(work <= 256 ? 256 : uni::kLoopThreads);
@@ -1781,8 +1773,33 @@ static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist
   }
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  void* argv[] = {&a};
+  void* argv[] = {args};
   return cudaLaunchKernelExC(&cfg, fn, argv);
+}
+
+// Cycles of the loop in one cooperative launch, from T as K1 left it, until
+// every right-hand side is done or max_cycles have run.
+static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist& h, long long max_cycles) {
+  const Layout& L = s->lay;
+  uni::LoopArgs a{};
+  a.col = uni_col_args(s, 0, 0, nullptr, nullptr, s->d_T, 1.f);
+  a.pen = uni_pencil_args(s, 0);
+  a.wig = s->ut[1].wigs;
+  a.uwig = s->ut[1].wigs + s->nw;
+  a.src = s->d_src;
+  a.partials = s->d_partials;
+  a.st = s->d_state;
+  a.rule = rule;
+  a.hist = h;
+  a.err = s->d_err;
+  a.max_cycles = max_cycles;
+  a.nw = s->nw;
+  a.nrhs = s->nrhs;
+  const void* fn = uni_kernels(std::max(L.ucol.plan.cls, L.uout.plan.cls)).loop;
+  a.groups = uni_groups(L.ucol);
+  a.e_resident = loop_smem(L, s->g, s->nw, true) <= kLoopSmem;
+  const size_t smem = loop_smem(L, s->g, s->nw, a.e_resident != 0, &a.tile_elems);
+  return launch_coop(s, fn, smem, s->nrhs, &a, &a.arrived);
 }
 
 // Energy histories: per right-hand side r, diff at r * 2cap and fresh at r * 2cap + cap.
@@ -3105,7 +3122,7 @@ int ws_pstd_create(const int64_t N[3], const float* c1, const float* c2, const f
   if (e == cudaSuccess) e = cudaMalloc(&p->d_Ebuf, 2 * npts * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_T2, npts * sizeof(float2));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_c3, npts * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_amp, (kPstdChunk + 1) * sizeof(double2));
+  if (e == cudaSuccess) e = cudaMalloc(&p->d_amp, (kPstdChunk + 1) * std::max(sizeof(double2), sizeof(uni::PstdStepAmp)));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_part, p->nparts * sizeof(double));
   if (e == cudaSuccess) e = cudaMemcpy(p->d_c3, c3, npts * sizeof(float), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
@@ -3167,13 +3184,53 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
   // of max(1000, 2 iterations_per_cycle) steps the run ends unconverged.
   const long long hard_stop =
       opts->max_iterations + std::max<long long>(1000, (long long)std::ceil(2 * opts->iterations_per_cycle));
+  const bool in_one = s->has_loop;
+  std::vector<uni::PstdStepAmp> steps(in_one ? kPstdChunk : 0);
+  if (in_one) {
+    WS_CUDA(use_layout(s, 1));
+    rc = ensure_partials(s, s->lay.grid_inner);
+    if (rc) return rc;
+    WS_CUDA(cudaMemsetAsync(s->d_T, 0, t_stride(s) * sizeof(float2), s->stream));  // the transform of E = 0
+  }
   while (true) {
     const long long K = kPstdChunk;
     hamp[0] = a_last;
     for (long long k = 1; k <= K; ++k)
       amp((double)(it0 - 1 + k) / opts->iterations_per_cycle, &hamp[k].x, &hamp[k].y, opts->user_data);
-    WS_CUDA(cudaMemcpyAsync(p->d_amp, hamp.data(), (K + 1) * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
-    for (long long k = 0; k < K; ++k) {
+    if (in_one) {
+      for (long long k = 0; k < K; ++k) {
+        const double2 A = hamp[k + 1], B = hamp[k];
+        const double dphi = std::atan2(A.y, A.x) - std::atan2(B.y, B.x);
+        steps[k] = uni::PstdStepAmp{make_float2((float)A.x, (float)A.y),
+                                    make_float2((float)std::cos(dphi), (float)std::sin(dphi)), A.x * A.x + A.y * A.y,
+                                    A.x > 0.9};  // MATLAB's A > 0.9 compares the real part
+      }
+      WS_CUDA(cudaMemcpyAsync(p->d_amp, steps.data(), K * sizeof(uni::PstdStepAmp), cudaMemcpyHostToDevice, s->stream));
+      uni::PstdLoopArgs a{};
+      a.col = uni_col_args(s, 0, 0, nullptr, nullptr, s->d_T, 1.f);
+      a.pen = uni_pencil_args(s, 0);
+      a.pen.pstd = 2;
+      a.c3 = p->d_c3;
+      a.src = s->d_src;
+      a.fields = p->d_Ebuf;
+      a.amp = (const uni::PstdStepAmp*)p->d_amp;
+      a.partials = s->d_partials;
+      a.st = s->d_state;
+      a.hist = p->d_hist;
+      a.hist_cap = std::min(p->hist_cap, cap);
+      a.max_iter = rule.max_iter;
+      a.threshold = rule.threshold;
+      a.err = s->d_err;
+      a.steps = (int)K;
+      a.interval = rule.interval;
+      a.groups = uni_groups(s->lay.ucol);
+      const size_t smem = pstd_loop_smem(s->lay, g, &a.tile_elems);
+      WS_CUDA(launch_coop(s, uni_kernels(std::max(s->lay.ucol.plan.cls, s->lay.uout.plan.cls)).pstd_loop, smem, 1, &a,
+                          &a.arrived));
+    } else {
+      WS_CUDA(cudaMemcpyAsync(p->d_amp, hamp.data(), (K + 1) * sizeof(double2), cudaMemcpyHostToDevice, s->stream));
+    }
+    for (long long k = 0; k < K && !in_one; ++k) {
       const long long it = it0 + k;
       float2* E = p->d_Ebuf + (size_t)((it - 1) & 1) * npts;
       float2* Ep = p->d_Ebuf + (size_t)(it & 1) * npts;
@@ -3188,8 +3245,10 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
       WS_CUDA(cudaGetLastError());
     }
     WS_CUDA(cudaMemcpyAsync(&hst, s->d_state, sizeof(hst), cudaMemcpyDeviceToHost, s->stream));
+    int failed = 0;  // a barrier of the loop kernel that gave up
+    if (in_one) WS_CUDA(cudaMemcpyAsync(&failed, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     WS_CUDA(cudaStreamSynchronize(s->stream));
-    if (hst.done || it0 + K > hard_stop) break;
+    if (hst.done || failed || it0 + K > hard_stop) break;
     a_last = hamp[K];
     it0 += K;
   }

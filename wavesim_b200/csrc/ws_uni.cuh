@@ -108,7 +108,8 @@ struct PencilArgs {
   float2* T;
   const DevState* st;
   long long pitch, tstride, cstride;  // cstride: elements between the components of T
-  int lty, nyt, bpr, mode3d, pstd;  // lty: log2 of the y per block
+  int lty, nyt, bpr, mode3d;  // lty: log2 of the y per block
+  int pstd;  // the PSTD Laplacian instead of the Green's function; 1: output conjugated
 };
 
 struct XArgs {
@@ -144,7 +145,35 @@ struct LoopArgs {
   int nw, nrhs;
 };
 
-enum { kFwd = 0, kInv = 1, kStep = 2 };
+// PSTD's stepping of a 2-D grid (PSTD.m:103-127) in one cooperative launch
+// (k_pstd_loop): the outer pencils with the Laplacian, then the column pass
+// with the leapfrog between its two transforms.  Each block keeps the two
+// fields, the coefficients and the source of its columns in shared memory.
+struct PstdStepAmp {
+  float2 A;   // the source's amplitude in the step
+  float2 ps;  // e^{i (arg A - arg A before)}
+  double A2;  // |A|^2
+  int may_end;  // real(A) > 0.9
+};
+struct PstdLoopArgs {
+  ColArgs col;  // gamma: (c1, c2) per point
+  PencilArgs pen;
+  const float* c3;
+  const float2* src;
+  float2* fields;  // two of npts: step it reads (it - 1) % 2 and writes it % 2
+  const PstdStepAmp* amp;  // of the launch's steps
+  double* partials;
+  DevState* st;
+  double* hist;
+  long long hist_cap, max_iter;
+  double threshold;
+  unsigned* arrived;
+  int* err;
+  int steps, interval;
+  int tile_elems, groups;
+};
+
+enum { kFwd = 0, kInv = 1, kStep = 2, kPstd = 3 };
 
 // the kernels compiled for radices up to kClassRadix[c]
 constexpr int kClasses = 3;
@@ -154,6 +183,7 @@ struct Kernels {
   const void* x[2];       // forward, inverse
   const void* pencil[2];  // one component, three
   const void* loop;
+  const void* pstd_loop;
 };
 template <int RM>
 Kernels kernels_up_to();

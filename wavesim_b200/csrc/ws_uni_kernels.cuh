@@ -74,6 +74,10 @@ struct ColMem {
   float* red;                // the energy of each 32 butterflies
   const float2* gamma;
   float2 *dE, *E;            // of the block's first column
+  // kPstd: gamma holds (c1, c2), dE the field, E the one before it (then the one after)
+  const float* c3 = nullptr;
+  const float2* S = nullptr;
+  float2 A{}, ps{};
 };
 
 // the 16-byte blocks inside n elements from p, into L2
@@ -146,62 +150,84 @@ __device__ __forceinline__ void col_body(const ColArgs& a, const ColIter& it, co
         const float2* __restrict__ tw0 = m.tw + S0.two + j;
         float2 v[R];
         if (MODE != kFwd) {
-          const float2 g0 = m.gxz[l];
+          const float2 g0 = MODE == kPstd ? make_float2(1.f, 0.f) : m.gxz[l];
           const float2* __restrict__ gmc = m.gamma + I.goff + j;
           float2* __restrict__ dEc = m.dE + at;
           float2* __restrict__ Ec = m.E + at;
           // the epilogue's loads in groups of H elements, the first group's before the butterfly
           constexpr int H = R <= 5 ? R : (R <= 10 ? (R + 1) / 2 : (R + 2) / 3);
           float2 gm[H], d0[H];
+          if (MODE != kPstd) {
 #pragma unroll
-          for (int r = 0; r < H; ++r) {
-            gm[r] = gmc[r * S0.sub];
-            d0[r] = dEc[r * S0.sub];
+            for (int r = 0; r < H; ++r) {
+              gm[r] = gmc[r * S0.sub];
+              d0[r] = dEc[r * S0.sub];
+            }
           }
 #pragma unroll
           for (int r = 0; r < R; ++r) v[r] = p[r * S0.subp];
 #pragma unroll
           for (int r = 1; r < R; ++r) v[r] = cmul_conj(v[r], tw0[r * S0.sub]);
           Dft<R, true>::run(v);
+          if constexpr (MODE == kPstd) {
 #pragma unroll
-          for (int h = 0; h < R; h += H) {
-            if (h > 0) {
+            for (int r = 0; r < R; ++r) {
+              // E_next = c2 E + c1 E_prev + c3 (ifftn(k fftn(E)) + A S), PSTD.m:103-107
+              const int y = j + r * S0.sub;
+              const float2 t = cadd(v[r], cmul(m.A, m.S[at + r * S0.sub]));
+              const float2 c12 = gmc[r * S0.sub], e = dEc[r * S0.sub], ep = Ec[r * S0.sub];
+              const float c3 = m.c3[at + r * S0.sub];
+              const float2 en = make_float2(c12.y * e.x + c12.x * ep.x + c3 * t.x, c12.y * e.y + c12.x * ep.y + c3 * t.y);
+              Ec[r * S0.sub] = en;
+              if (I.in && y >= g.r0[0] && y < g.r1[0]) {
+                const float2 d = make_float2(en.x - (e.x * m.ps.x - e.y * m.ps.y), en.y - (e.x * m.ps.y + e.y * m.ps.x));
+                esum = fmaf(d.x, d.x, fmaf(d.y, d.y, esum));
+              }
+              v[r] = en;
+            }
+          } else {
+#pragma unroll
+            for (int h = 0; h < R; h += H) {
+              if (h > 0) {
+#pragma unroll
+                for (int r = 0; r < H; ++r)
+                  if (h + r < R) {
+                    gm[r] = gmc[(h + r) * S0.sub];
+                    d0[r] = dEc[(h + r) * S0.sub];
+                  }
+              }
+              float2 e0[H];
+#pragma unroll
+              for (int r = 0; r < H; ++r)
+                if (h + r < R) e0[r] = acc_now ? Ec[(h + r) * S0.sub] : make_float2(0.f, 0.f);
 #pragma unroll
               for (int r = 0; r < H; ++r)
                 if (h + r < R) {
-                  gm[r] = gmc[(h + r) * S0.sub];
-                  d0[r] = dEc[(h + r) * S0.sub];
+                  const int k = h + r, y = j + k * S0.sub;
+                  // Eprop after the conjugate ramps (WaveSim.m:55), f_mix (f_mix.m:3-4), E' += dE'
+                  const float2 ep = cmul_conj(cmul_conj(v[k], g0), m.gy[y]);
+                  const float2 one_m = make_float2(1.f - kAlpha * gm[r].x, -kAlpha * gm[r].y);
+                  const float2 t = cmul(cmul(gm[r], gm[r]), ep);
+                  const float2 dn = cadd(cmul(one_m, d0[r]), make_float2(kAlpha * t.y, -kAlpha * t.x));
+                  dEc[k * S0.sub] = dn;
+                  if (acc_now) Ec[k * S0.sub] = cadd(e0[r], it.acc == kAccPair ? cadd(d0[r], dn) : dn);
+                  if (I.in && y >= g.r0[0] && y < g.r1[0]) esum = fmaf(dn.x, dn.x, fmaf(dn.y, dn.y, esum));
+                  v[k] = dn;
                 }
             }
-            float2 e0[H];
-#pragma unroll
-            for (int r = 0; r < H; ++r)
-              if (h + r < R) e0[r] = acc_now ? Ec[(h + r) * S0.sub] : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < H; ++r)
-              if (h + r < R) {
-                const int k = h + r, y = j + k * S0.sub;
-                // Eprop after the conjugate ramps (WaveSim.m:55), f_mix (f_mix.m:3-4), E' += dE'
-                const float2 ep = cmul_conj(cmul_conj(v[k], g0), m.gy[y]);
-                const float2 one_m = make_float2(1.f - kAlpha * gm[r].x, -kAlpha * gm[r].y);
-                const float2 t = cmul(cmul(gm[r], gm[r]), ep);
-                const float2 dn = cadd(cmul(one_m, d0[r]), make_float2(kAlpha * t.y, -kAlpha * t.x));
-                dEc[k * S0.sub] = dn;
-                if (acc_now) Ec[k * S0.sub] = cadd(e0[r], it.acc == kAccPair ? cadd(d0[r], dn) : dn);
-                if (I.in && y >= g.r0[0] && y < g.r1[0]) esum = fmaf(dn.x, dn.x, fmaf(dn.y, dn.y, esum));
-                v[k] = dn;
-              }
           }
         } else {
 #pragma unroll
           for (int r = 0; r < R; ++r) v[r] = a.dE_in[f0 + at + r * S0.sub];
         }
         if (MODE != kInv) {
-          const float2 g1 = m.gxz1[l];
+          if (MODE != kPstd) {
+            const float2 g1 = m.gxz1[l];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            if (it.src) v[r] = cadd(v[r], cmul(a.A, it.src[f0 + at + r * S0.sub]));
-            v[r] = cmul(cmul(v[r], g1), m.gy1[j + r * S0.sub]);
+            for (int r = 0; r < R; ++r) {
+              if (it.src) v[r] = cadd(v[r], cmul(a.A, it.src[f0 + at + r * S0.sub]));
+              v[r] = cmul(cmul(v[r], g1), m.gy1[j + r * S0.sub]);
+            }
           }
           Dft<R, false>::run(v);
 #pragma unroll
@@ -433,7 +459,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
   for (int c = 0; c < NC; ++c) row_middles<RM, true>(a.po, tile + c * tn, tw, ty, yl, w, W);
 #pragma unroll
   for (int c = 0; c < NC; ++c)
-    rows_out<RM>(a.po.st[0], tw, tile + c * tn, base + c * a.cstride, step, ty, yl, w, W, live, a.pstd != 0);
+    rows_out<RM>(a.po.st[0], tw, tile + c * tn, base + c * a.cstride, step, ty, yl, w, W, live, a.pstd == 1);
 }
 
 template <int RM, int NC>
@@ -648,12 +674,99 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
   if (blockIdx.x == 0 && tid < a.nrhs) a.st[tid] = st[tid];
 }
 
+// us a step at 256^2: 11, against 30 of five launches a step (the inner
+// transform, the outer pencils, the inner transform again for the inverse, the
+// leapfrog, the stop rule), which the host issued one by one.
+template <int RM>
+__global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_constant__ PstdLoopArgs a) {
+  extern __shared__ float2 tile[];
+  __shared__ DevState st;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const Geom& g = a.col.g;
+  const int lines = a.col.lines, elems = lines * g.ny;
+  unsigned target = 0;
+  float2* const tw_col = tile + a.tile_elems;
+  float2* const tw_out = tw_col + a.col.py.ntw;
+  float2* const c12 = tw_out + a.pen.po.ntw;  // the block's columns
+  float2* const E = c12 + elems;              // two fields
+  float2* const S = E + 2 * elems;
+  ColLine* const info = reinterpret_cast<ColLine*>(S + elems);
+  float* const red = reinterpret_cast<float*>(info + lines);
+  float* const po = red + a.groups;
+  float* const c3 = po + a.pen.po.n;
+  const bool own = blockIdx.x < a.col.bpr;
+  const int col0 = blockIdx.x * lines, nl = own ? min(lines, a.col.total - col0) : 0;
+  const long long f0 = (long long)col0 * g.ny;
+  copy_table(tw_col, a.col.py.tw, a.col.py.ntw);
+  copy_table(tw_out, a.pen.po.tw, a.pen.po.ntw);
+  copy_table(po, a.pen.w.pxe, a.pen.po.n);
+  for (int l = tid; l < nl; l += nthr) {
+    const int x = col0 + l;
+    info[l] = ColLine{(long long)l * g.ny, x >= g.r0[1] && x < g.r1[1] && g.r0[2] == 0};
+  }
+  for (int i = tid; i < nl * g.ny; i += nthr) {
+    c12[i] = a.col.gamma[f0 + i];
+    c3[i] = a.c3[f0 + i];
+    S[i] = a.src[f0 + i];
+    E[i] = a.fields[f0 + i];
+    E[elems + i] = a.fields[g.npts + f0 + i];
+  }
+  if (tid == 0) st = *a.st;
+  __syncthreads();
+  for (int k = 0; k < a.steps && !st.done; ++k) {
+    const PstdStepAmp amp = a.amp[k];
+    for (int t = blockIdx.x; t < a.pen.bpr; t += gridDim.x) {
+      pencil_body<RM, 1>(a.pen, a.pen.w, 0, t, tile, tw_out, po);
+      __syncthreads();
+    }
+    if (!grid_barrier(a.arrived, target, a.err)) return;
+    const int cur = (st.it - 1) & 1;
+    if (own) {
+      ColIter it{};
+      it.partials = a.partials;
+      ColMem m{tile, tw_col, nullptr, nullptr, nullptr, nullptr, info, red, c12, E + cur * elems, E + (1 - cur) * elems};
+      m.c3 = c3;
+      m.S = S;
+      m.A = amp.A;
+      m.ps = amp.ps;
+      col_body<RM, kPstd>(a.col, it, m, 0, blockIdx.x);
+    }
+    if (!grid_barrier(a.arrived, target, a.err)) return;
+    // Simulation.next (Simulation.m:193-217) for PSTD.run_algorithm (PSTD.m:108-124), the same in every block
+    if (tid < 32) {
+      const double e = st.calc_energy ? sum_partials(a.partials, a.col.bpr) : 0.0;
+      if (tid == 0) {
+        if (st.calc_energy) st.last_step_energy = e / amp.A2;
+        const double d = st.last_step_energy;
+        const int it = st.it;
+        if (blockIdx.x == 0 && it - 1 < a.hist_cap) a.hist[it - 1] = d;
+        if (it == 1) st.diff1 = d;
+        if (amp.may_end && d / st.diff1 < a.threshold) {
+          st.done = 1;
+          st.converged = 1;
+        } else if (amp.may_end && it >= a.max_iter) {
+          st.done = 1;
+          st.converged = 0;
+        }
+        st.calc_energy = ((it - 1) % a.interval) == 0;
+        st.it = it + 1;
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = tid; i < nl * g.ny; i += nthr) {
+    a.fields[f0 + i] = E[i];
+    a.fields[g.npts + f0 + i] = E[elems + i];
+  }
+  if (blockIdx.x == 0 && tid == 0) *a.st = st;
+}
+
 template <int RM>
 Kernels kernels_up_to() {
   return Kernels{{(const void*)k_col<RM, kFwd>, (const void*)k_col<RM, kInv>, (const void*)k_col<RM, kStep>},
                  {(const void*)k_x<RM, false>, (const void*)k_x<RM, true>},
                  {(const void*)k_pencil<RM, 1>, (const void*)k_pencil<RM, 3>},
-                 (const void*)k_loop<RM>};
+                 (const void*)k_loop<RM>, (const void*)k_pstd_loop<RM>};
 }
 
 }  // namespace uni
