@@ -145,3 +145,21 @@ def test_pstd_in_one_launch_matches_launched_passes(gpu, shape, bw, monkeypatch)
     assert st.it == sg.it
     assert rel(E, Eg) < 5e-5, rel(E, Eg)
     np.testing.assert_allclose(st.diff_energy, sg.diff_energy, rtol=1e-3)
+
+
+@pytest.mark.parametrize("shape,bw,count", [((480, 960), [16, 32], 5), ((256, 448), [32, 32], 16)])
+def test_batched_x_pencils_match_single_solves(gpu, shape, bw, count):
+    """Batches of 2-D grids of 1024 and 512 points along x run their x pencils through the tensor-copy pipeline
+    (tma::kt_pencil with D3 = false), single solves do not."""
+    import wavesim_b200 as ws
+    n = 1.1 + 0.2 * np.random.default_rng(8).random(shape) + 0.01j
+    sim = ws.WaveSim(n, {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": bw, "energy_threshold": 1e-99,
+                         "max_iterations": 12})
+    waves = [ws.PlaneWave((shape[0], 1), (1, 1), 1.0, (0.05 * k, 0.0, 0.0)) for k in range(count)]
+    E, st = sim.exec_batch(waves)
+    for k in (0, count - 1):
+        E1, s1 = sim.exec(ws.Source(waves[k].values()[..., 0], [1, 1]))
+        assert st[k].it == s1.it
+        assert rel(E[k], E1) < TOL, rel(E[k], E1)
+        np.testing.assert_allclose(st[k].diff_energy, s1.diff_energy, rtol=2e-4)
+    sim.close()

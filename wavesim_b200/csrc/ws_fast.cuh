@@ -123,7 +123,14 @@ __device__ __forceinline__ void dft_slice(float2 (&v)[16], int off) {
   for (int r = 0; r < R; ++r) v[off + r] = u[r];
 }
 
-template <int N, bool INV, int S, class Line, class Sync>
+// ST: the twiddles from the stage tables behind the N-point table (tw[N ...],
+// push_twiddles): W^{jm r} of a stage at r Ns + jm, so that neighbouring threads
+// read neighbouring entries.  In the N-point table they lie r N / (Ns R) apart,
+// up to 16 L1 lines a load: 16 x 1024^2 took 315 us an iteration with it in K2
+// and the column pass, 267 with the stage tables; one 1024^2 34 and 28.  (The
+// 256-point passes in 3-D wait for HBM; they gained nothing, and the column
+// pass there keeps the one table.)
+template <int N, bool INV, int S, bool ST = false, class Line, class Sync>
 __device__ __forceinline__ void line_stage(float2 (&v)[16], const Line& L, int p, const float2* __restrict__ tw,
                                            Sync sync) {
   using PL = LinePlan<N>;
@@ -138,7 +145,7 @@ __device__ __forceinline__ void line_stage(float2 (&v)[16], const Line& L, int p
       const int jm = j & (Ns - 1);
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        float2 w = __ldg(&tw[jm * r * TS]);
+        float2 w = __ldg(&tw[ST ? N + (S > 1 ? PL::span(2) : 0) + r * Ns + jm : jm * r * TS]);
         if (INV) w.y = -w.y;
         v[q * R + r] = cmul(v[q * R + r], w);
       }
@@ -194,6 +201,16 @@ __device__ __forceinline__ void line_fft(float2 (&v)[16], const Line& L, int p, 
   line_stage<N, INV, 0>(v, L, p, tw, sync);
   if constexpr (LinePlan<N>::NST > 1) line_stage<N, INV, 1>(v, L, p, tw, sync);
   if constexpr (LinePlan<N>::NST > 2) line_stage<N, INV, 2>(v, L, p, tw, sync);
+}
+
+// line_fft with the twiddles from the stage tables (the same values, so the
+// same results).
+template <int N, bool INV, class Line, class Sync>
+__device__ __forceinline__ void line_fft_st(float2 (&v)[16], const Line& L, int p, const float2* __restrict__ tw,
+                                            Sync sync) {
+  line_stage<N, INV, 0>(v, L, p, tw, sync);
+  if constexpr (LinePlan<N>::NST > 1) line_stage<N, INV, 1, true>(v, L, p, tw, sync);
+  if constexpr (LinePlan<N>::NST > 2) line_stage<N, INV, 2, true>(v, L, p, tw, sync);
 }
 
 template <int N, bool INV, class Line, class Sync>
@@ -455,7 +472,10 @@ __global__ void __launch_bounds__(TY*(NO / 16) < 1024 ? TY*(NO / 16) : 1024, 3)
 #pragma unroll
   for (int r = 0; r < 16; ++r) v[r] = base[ps * (p + P * r)];
   RowLine L{sm + yl, TYS};
-  line_fft<NO, false>(v, L, p, a.po.tw, SyncBlock{});
+  if constexpr (NO > 256)
+    line_fft_st<NO, false>(v, L, p, a.po.tw, SyncBlock{});
+  else
+    line_fft<NO, false>(v, L, p, a.po.tw, SyncBlock{});
   // f_g0_scalar with the 1/N of ifftn: E ./ (px^2 + py^2 + (pz^2 - k02e))
   const float py = a.w.pye[ky];
   const float pxm = a.mode3d ? a.w.pxe[mid] : 0.f;
@@ -479,7 +499,10 @@ __global__ void __launch_bounds__(TY*(NO / 16) < 1024 ? TY*(NO / 16) : 1024, 3)
       v[m] = cmul(v[m], make_float2(dr * inv, -di * inv));
     }
   }
-  line_fft<NO, true>(v, L, p, a.po.tw, SyncBlock{});
+  if constexpr (NO > 256)
+    line_fft_st<NO, true>(v, L, p, a.po.tw, SyncBlock{});
+  else
+    line_fft<NO, true>(v, L, p, a.po.tw, SyncBlock{});
   if (a.pstd)
 #pragma unroll
     for (int m = 0; m < 16; ++m) v[m].y = -v[m].y;
@@ -1301,9 +1324,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int r = 0; r < 16; ++r) v[r] = make_float2(0.f, 0.f);
     }
     if constexpr (P <= 32) {
-      line_fft<N, true>(v, L, p, a.py.tw, SyncWarp{});
+      line_fft_st<N, true>(v, L, p, a.py.tw, SyncWarp{});
     } else {
-      line_fft<N, true>(v, L, p, a.py.tw, SyncBlock{});
+      line_fft_st<N, true>(v, L, p, a.py.tw, SyncBlock{});
     }
     if (live) {
       const int x = (int)(col % nx), c = (int)(col / nx);
@@ -1347,9 +1370,9 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
     }
     if constexpr (P <= 32) {
-      line_fft<N, false>(v, L, p, a.py.tw, SyncWarp{});
+      line_fft_st<N, false>(v, L, p, a.py.tw, SyncWarp{});
     } else {
-      line_fft<N, false>(v, L, p, a.py.tw, SyncBlock{});
+      line_fft_st<N, false>(v, L, p, a.py.tw, SyncBlock{});
     }
     if (live) {
 #pragma unroll

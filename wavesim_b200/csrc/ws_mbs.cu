@@ -263,6 +263,20 @@ static const std::vector<TmaPencil>& tma_pencil_table() {
   return t;
 }
 
+// ... for the x pencils of 2-D grids, in batches
+template <int NO, int TY, int S>
+static TmaPencil tma_pencil2d() {
+  using PT = tma::PencilTile<NO, TY, S>;
+  return TmaPencil{NO, TY, S, (const void*)tma::kt_pencil<NO, TY, S, false>, PT::smem, PT::kThreads};
+}
+static const std::vector<TmaPencil>& tma_pencil2d_table() {
+  // 16 x 1024^2: 4 y x 3 stages 267 us an iteration, 8 x 3 271, 4 x 2 (80
+  // registers) 371; kf_pencil (32-byte rows, nothing in flight while it
+  // computes) 336.  64 x 512^2: 8 x 3 220, 4 x 3 231, 8 x 2 270, kf_pencil 254
+  static const std::vector<TmaPencil> t = {tma_pencil2d<1024, 4, 3>(), tma_pencil2d<512, 8, 3>()};
+  return t;
+}
+
 static const std::vector<FastPencil>& fast_pencil_table() {
   static const std::vector<FastPencil> t = {
       fast_pencil<32, 16>(),  fast_pencil<64, 16>(),  fast_pencil<128, 16>(),
@@ -420,6 +434,7 @@ struct Layout {
   const FastInner* fi = nullptr;   // fast K1/K3, or null (generic)
   const FastPencil* fp = nullptr;  // fast K2, or null (generic)
   const TmaPencil* tp = nullptr;   // persistent TMA K2 (takes precedence over fp), or null
+  const TmaPencil* tp2 = nullptr;  // persistent TMA x pencils of 2-D grids, for batches, or null
   const XPencil* xp = nullptr;     // x passes of the split fused step, or null (one-kernel fused step)
   int rset = kPow2;  // radix set of every plan of the solver
   int mode3d = 0;
@@ -627,6 +642,12 @@ static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutC
         L.tp = &f;
         break;
       }
+  if (!L.mode3d && g.nc == 1 && L.fp && ch.outer == 0 && !(k2 && std::strcmp(k2, "plain") == 0))
+    for (const TmaPencil& f : tma_pencil2d_table())
+      if (f.no == no && g.ny % f.ty == 0 && (!want_tty || f.ty == want_tty) && (!want_ts || f.stages == want_ts)) {
+        L.tp2 = &f;
+        break;
+      }
   // the split fused step (x pencils + column pass) on power-of-two planes;
   // WAVESIM_B200_STEP=cluster keeps the one-kernel step with the cluster
   // exchange, WAVESIM_B200_XTY picks the x pencils' y tile
@@ -807,12 +828,33 @@ static int build_plan(int n, const std::vector<float2>& tw_all_offset_dummy, Fft
   return WS_OK;
 }
 
+// The table exp(-2 pi i k / n); behind it, for the lengths with a compile-time
+// schedule, the tables of its second stage and on: W_{Ns R}^{jm r} at r Ns + jm
+// (fast::line_stage with ST, mixed::Plan::table).
 static void push_twiddles(std::vector<float2>& all, int n, size_t& off) {
   off = all.size();
-  for (int k = 0; k < n; ++k) {
-    const double a = -2.0 * M_PI * (double)k / (double)n;
+  auto push = [&](double k, int of) {
+    const double a = -2.0 * M_PI * k / (double)of;
     all.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+  };
+  for (int k = 0; k < n; ++k) push(k, n);
+  std::vector<int> radix;
+  switch (n) {  // the compile-time schedules
+    case 96: radix = {12, 4, 2}; break;
+    case 160: radix = {10, 4, 4}; break;
+    case 192: radix = {12, 4, 4}; break;
+    case 224: radix = {14, 4, 4}; break;
+    case 320: radix = {4, 4, 4, 5}; break;
+    case 448: radix = {14, 4, 4, 2}; break;
+    case 576: radix = {12, 12, 4}; break;
+    default:
+      if (n < 32 || n > 2048 || (n & (n - 1))) return;
+      radix = {16, n <= 256 ? n / 16 : 16};
+      if (n > 256) radix.push_back(n / 256);
   }
+  for (int s = 1, Ns = radix[0]; s < (int)radix.size(); Ns *= radix[s++])
+    for (int r = 0; r < radix[s]; ++r)
+      for (int j = 0; j < Ns; ++j) push((double)j * r * (n / (Ns * radix[s])), n);
 }
 
 template <typename K>
@@ -861,6 +903,7 @@ static int set_kernel_attributes() {
   }
   for (const FastPencil& f : fast_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (const TmaPencil& f : tma_pencil_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
+  for (const TmaPencil& f : tma_pencil2d_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (int c = 0; c < uni::kClasses; ++c) {
     const uni::Kernels& k = uni_kernels(c);
     for (const void* f : k.col) WS_CUDA(allow_dynamic_smem(f, optin));
@@ -1466,8 +1509,7 @@ static EncodeTiledFn encode_tiled() {
 // T of the current batch as a 3-D float tensor {2 Ny, Nx, Nz Nc nrhs}, box
 // {2 TY, 1, Nz}: every x coordinate the kernel issues is 2 TY yt floats, a
 // multiple of 16 floats (TY >= 8), so each copy starts on a 64-byte boundary.
-static cudaError_t ensure_tmap(Solver* s) {
-  const TmaPencil* f = s->lay.tp;
+static cudaError_t ensure_tmap(Solver* s, const TmaPencil* f) {
   if (s->tmap_base == s->d_T && s->tmap_nrhs == s->nrhs && s->tmap_kernel == f->fn) return cudaSuccess;
   s->tmap_kernel = nullptr;
   s->tma_blocks = 0;
@@ -1476,7 +1518,8 @@ static cudaError_t ensure_tmap(Solver* s) {
   const Geom& g = s->g;
   const cuuint64_t dims[3] = {(cuuint64_t)2 * g.ny, (cuuint64_t)g.nx, (cuuint64_t)g.nz * g.nc * s->nrhs};
   const cuuint64_t strides[2] = {(cuuint64_t)g.ny * sizeof(float2), (cuuint64_t)g.ny * g.nx * sizeof(float2)};
-  const cuuint32_t box[3] = {(cuuint32_t)(2 * f->ty), 1u, (cuuint32_t)f->no};
+  const cuuint32_t line = (cuuint32_t)std::min(f->no, 256);  // along z, or along x of a 2-D grid
+  const cuuint32_t box[3] = {(cuuint32_t)(2 * f->ty), s->lay.mode3d ? 1u : line, s->lay.mode3d ? line : 1u};
   const cuuint32_t estr[3] = {1u, 1u, 1u};
   if (enc(&s->tmap_T, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, s->d_T, dims, strides, box, estr,
           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1488,10 +1531,9 @@ static cudaError_t ensure_tmap(Solver* s) {
   return cudaSuccess;
 }
 
-static cudaError_t launch_k2_tma(const Solver* cs, int w) {
+static cudaError_t launch_k2_tma(const Solver* cs, int w, const TmaPencil* f) {
   Solver* s = const_cast<Solver*>(cs);  // the tensor-map cache only
-  const TmaPencil* f = s->lay.tp;
-  cudaError_t e = ensure_tmap(s);
+  cudaError_t e = ensure_tmap(s, f);
   if (e != cudaSuccess) return e;
   if (s->tma_blocks <= 0) {
     int per_sm = 0;
@@ -1500,7 +1542,7 @@ static cudaError_t launch_k2_tma(const Solver* cs, int w) {
     s->tma_blocks = std::max(1, per_sm) * kNumSms;
   }
   OuterArgs a = outer_args(s, w);
-  int ntiles = s->nrhs * s->g.nx * (s->g.ny / f->ty);
+  int ntiles = s->nrhs * (s->lay.mode3d ? s->g.nx : 1) * (s->g.ny / f->ty);
   const unsigned grid = (unsigned)std::min(ntiles, s->tma_blocks);
   const DevState* st = s->d_state;
   int* err = s->d_err;
@@ -1509,7 +1551,9 @@ static cudaError_t launch_k2_tma(const Solver* cs, int w) {
 }
 
 static cudaError_t launch_k2(const Solver* s, int w) {
-  if (s->lay.tp) return launch_k2_tma(s, w);
+  if (s->lay.tp) return launch_k2_tma(s, w, s->lay.tp);
+  // the pipeline pays from about two tiles per resident block on
+  if (s->lay.tp2 && (long long)s->nrhs * (s->g.ny / s->lay.tp2->ty) >= 4 * kNumSms) return launch_k2_tma(s, w, s->lay.tp2);
   if (s->lay.fp) {
     OuterArgs a = outer_args(s, w);
     const FastPencil* f = s->lay.fp;

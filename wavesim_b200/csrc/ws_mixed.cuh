@@ -70,6 +70,8 @@ struct Plan {
   __host__ __device__ static constexpr int span(int s) {
     return s == 0 ? 1 : (s == 1 ? R0 : (s == 2 ? R0 * R1 : R0 * R1 * R2));
   }
+  // where stage s's twiddles W_{Ns R}^{jm r} lie, at r Ns + jm, behind the N-point table (push_twiddles)
+  __host__ __device__ static constexpr int table(int s) { return s <= 1 ? 0 : table(s - 1) + span(s); }
   static_assert(R0 * R1 * R2 * R3 == N_ && N_ % E_ == 0, "the radices multiply to N, E divides N");
   static_assert(E_ % R0 == 0 && E_ % R1 == 0 && E_ % R2 == 0 && E_ % R3 == 0, "every radix divides E");
   static_assert(NST > 1 || R0 == E_, "a one-stage line is one butterfly per thread");
@@ -89,7 +91,7 @@ template <class PL, bool INV, int S, class Line, class Sync>
 __device__ __forceinline__ void stage(float2 (&v)[PL::E], const Line& L, int p, const float2* __restrict__ tw,
                                       Sync sync) {
   constexpr int E = PL::E, N = PL::N, P = PL::P;
-  constexpr int R = PL::radix(S), Ns = PL::span(S), B = E / R, NR = N / R, TS = N / (Ns * R);
+  constexpr int R = PL::radix(S), Ns = PL::span(S), B = E / R, NR = N / R;
   if constexpr (S == 0 && B > 1) {
     // butterfly q takes v[q + B r]; gather it to v[q R + r]
     float2 t[E];
@@ -109,7 +111,7 @@ __device__ __forceinline__ void stage(float2 (&v)[PL::E], const Line& L, int p, 
       const int jm = j % Ns;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        float2 w = __ldg(&tw[jm * r * TS]);
+        float2 w = __ldg(&tw[N + PL::table(S) + r * Ns + jm]);
         if (INV) w.y = -w.y;
         v[q * R + r] = cmul(v[q * R + r], w);
       }

@@ -79,7 +79,9 @@ __device__ __forceinline__ bool wait_parity(uint64_t* bar, uint32_t parity, long
 
 template <int NO, int TY, int S>
 struct PencilTile {
-  static_assert(NO >= 32 && NO <= 256, "a TMA box dimension holds at most 256 elements");
+  static_assert(NO >= 32 && (NO <= 256 || NO % 256 == 0), "whole boxes");
+  static constexpr int kBox = NO <= 256 ? NO : 256;  // a TMA box dimension holds at most 256 elements
+  static constexpr int kBoxes = NO / kBox;
   static_assert(2 * TY * 4 % 16 == 0 && 2 * TY <= 256, "inner box extent");
   static constexpr int P = NO / 16;
   static constexpr int kThreads = TY * P;
@@ -88,11 +90,13 @@ struct PencilTile {
   static constexpr size_t smem = S * (size_t)kTileBytes + 128;
   // blocks per SM the tiles leave room for (228 KB of shared memory, 1 KB
   // reserved per block, at most 4): the register bound of the kernels
-  static constexpr int kMinBlocks = (int)(228 * 1024 / (smem + 3 * 1024)) >= 4 ? 4
-                                    : ((int)(228 * 1024 / (smem + 3 * 1024)) >= 3 ? 3 : 2);
+  static constexpr int kFit = (int)(228 * 1024 / (smem + 3 * 1024));
+  static constexpr int kMinBlocks = kFit >= 4 ? 4 : (kFit >= 3 ? 3 : (kFit >= 2 || NO <= 256 ? 2 : 1));
 };
 
-template <int NO, int TY, int S>
+// D3 = false: the x pencils of 2-D grids, NO = Nx points (boxes of at most 256)
+// at (2 TY yt, 256 k, rhs) of the same map.
+template <int NO, int TY, int S, bool D3 = true>
 __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO, TY, S>::kMinBlocks)
     kt_pencil(const __grid_constant__ CUtensorMap tmap, OuterArgs a, const DevState* __restrict__ st, int ntiles,
               int* __restrict__ err) {
@@ -106,7 +110,7 @@ __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO
   const int tid = threadIdx.x;
   const int yl = tid % TY, p = tid / TY;
   const int nyt = g.ny / TY;
-  const int per_rhs = nyt * g.nx;
+  const int per_rhs = D3 ? nyt * g.nx : nyt;
   if (tid == 0) {
 #pragma unroll
     for (int b = 0; b < S; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(fast::smem_addr(&full[b])));
@@ -124,19 +128,32 @@ __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO
     int rhs, mid, yt;
     coords(t, rhs, mid, yt);
     expect_bytes(&full[b], PT::kTileBytes);
-    load_3d(fast::smem_addr(buf0 + b * NO * TY), &tmap, 2 * TY * yt, mid, rhs * g.nz, fast::smem_addr(&full[b]));
+    if constexpr (D3) {
+      load_3d(fast::smem_addr(buf0 + b * NO * TY), &tmap, 2 * TY * yt, mid, rhs * g.nz, fast::smem_addr(&full[b]));
+    } else {
+#pragma unroll
+      for (int k = 0; k < PT::kBoxes; ++k)
+        load_3d(fast::smem_addr(buf0 + b * NO * TY + k * PT::kBox * TY), &tmap, 2 * TY * yt, k * PT::kBox, rhs,
+                fast::smem_addr(&full[b]));
+    }
   };
   const int G = gridDim.x;
   const int mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / G + 1 : 0;  // tiles of this block
   if (tid == 0)
     for (int i = 0; i < S - 1 && i < mine; ++i) issue(blockIdx.x + i * G, i);
-  float2 wt[16];  // the second stage's twiddles of this thread, the same for every tile
-  fast::load_tw2<NO>(wt, p, a.po.tw);
+  float2 wt[16];  // the second stage's twiddles of this thread, the same for every tile (two-stage lines)
+  if constexpr (NO <= 256) fast::load_tw2<NO>(wt, p, a.po.tw);
+  auto transform = [&](float2(&v)[16], const fast::RowLine& L, auto inv) {
+    if constexpr (NO <= 256)
+      fast::line_fft_tw2<NO, decltype(inv)::value>(v, L, p, wt, fast::SyncBlock{});
+    else
+      fast::line_fft_st<NO, decltype(inv)::value>(v, L, p, a.po.tw, fast::SyncBlock{});
+  };
   // this thread's part of the Green's function: pz^2 - Re(k0^2 + i eps) for its 16 z
   float pz2[16];
 #pragma unroll
   for (int m = 0; m < 16; ++m) {
-    const float po = a.w.pze[p + P * m];
+    const float po = D3 ? a.w.pze[p + P * m] : a.w.pxe[p + P * m];
     pz2[m] = fmaf(po, po, -a.k02e.x);
   }
   const float di = -a.k02e.y;
@@ -172,10 +189,10 @@ __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO
       // the exchanges go through the tile's own buffer (each starts with a
       // block barrier, so every input has been read before it is overwritten)
       fast::RowLine L{buf + yl, TY};
-      fast::line_fft_tw2<NO, false>(v, L, p, wt, fast::SyncBlock{});
+      transform(v, L, std::false_type{});
       // f_g0_scalar with the 1/N of ifftn: E ./ (px^2 + py^2 + (pz^2 - k02e))
       const float py = a.w.pye[yt * TY + yl];
-      const float pxm = a.w.pxe[mid];
+      const float pxm = D3 ? a.w.pxe[mid] : a.w.pze[0];
       const float base2 = fmaf(pxm, pxm, py * py);
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
@@ -188,7 +205,7 @@ __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO
         }
       }
       refill();
-      fast::line_fft_tw2<NO, true>(v, L, p, wt, fast::SyncBlock{});
+      transform(v, L, std::true_type{});
       if (a.pstd)
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m].y = -v[m].y;
@@ -199,7 +216,13 @@ __global__ void __launch_bounds__(PencilTile<NO, TY, S>::kThreads, PencilTile<NO
     }
     __syncthreads();
     if (tid == 0 && live) {
-      store_3d(&tmap, 2 * TY * yt, mid, rhs * g.nz, fast::smem_addr(buf));
+      if constexpr (D3) {
+        store_3d(&tmap, 2 * TY * yt, mid, rhs * g.nz, fast::smem_addr(buf));
+      } else {
+#pragma unroll
+        for (int k = 0; k < PT::kBoxes; ++k)
+          store_3d(&tmap, 2 * TY * yt, k * PT::kBox, rhs, fast::smem_addr(buf + k * PT::kBox * TY));
+      }
       bulk_commit();
     }
   }
