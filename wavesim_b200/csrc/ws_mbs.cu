@@ -185,12 +185,15 @@ static FastPencil mixed_pencil2d() {
 }
 
 static const std::vector<FastInner>& fast_inner_table() {
+  // 96^2 planes on 3 blocks (288 column-pass blocks at 96^3): 24.9 us an
+  // iteration against 29.6 with one block per plane (96 of the 148 SMs);
+  // 128^2 on 2: 41.5 against 43.8 on 4
   static const std::vector<FastInner> t = {
       fast_inner<64, 1, true>(),     fast_inner<128, 2, true>(),    fast_inner<256, 8, true>(),
       fast_inner<256, 16, true>(),
       fast_inner<64, 1, false>(),    fast_inner<128, 1, false>(),   fast_inner<256, 1, false>(),
       fast_inner<512, 1, false>(),   fast_inner<1024, 1, false>(),  fast_inner<2048, 1, false>(),
-      mixed_inner<Plan192, 6>(),     mixed_inner<Plan96, 1>(),      mixed_inner<Plan160, 5>(),
+      mixed_inner<Plan192, 6>(),     mixed_inner<Plan96, 3>(),      mixed_inner<Plan160, 5>(),
       mixed_inner<Plan224, 7>(),
       mixed_inner2d<Plan192>(),      mixed_inner2d<Plan320>(),      mixed_inner2d<Plan448>(),
       mixed_inner2d<Plan576>()};
