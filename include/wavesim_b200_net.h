@@ -83,6 +83,13 @@ int ws_net_relu_grad_bf16(float* dy, const void* y, int64_t rows, int C, void* o
 /* im2col of a 3x3x3 convolution with zero padding 1: col[vox][kp], entry
  * ((dz*3 + dy)*3 + dx)*C + c, zero for k >= 27 C (C, kp multiples of 8). */
 int ws_net_im2col3(const void* in, void* col, int b, int d, int h, int w, int C, int kp, void* stream);
+/* its transpose, out[k][vox] for k < kp (a multiple of 32) with leading dimension
+ * ldo >= voxels (a multiple of 64), zero for k >= 27 C and from the last voxel on */
+int ws_net_im2col3_t(const void* in, void* out, int b, int d, int h, int w, int C, int kp, int64_t ldo, void* stream);
+/* gw[M][N] += A[M][K] . B[N][K]^T (fp32; A, B bf16 as for ws_gemm_bf16, whose
+ * sums these are bit for bit), for few outputs and a long K */
+int ws_net_wgrad_bf16(const void* A, const void* B, float* gw, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                      int* err_flag, void* stream);
 /* gradient of ws_net_im2col3 (fp32): din[u][c] = sum_t dcol[u - (t - 1)][t C + c] */
 int ws_net_col2im3(const float* dcol, float* din, int b, int d, int h, int w, int C, int kp, void* stream);
 /* out[c][r] = bf16(in[r][c]) (fp32 in, rows x cols), out rows zero-padded to ldo */

@@ -280,3 +280,42 @@ def test_network_warm_start_runs_on_device(gpu):
     E, st = sim.exec(src)
     Ew, sw = sim.exec(src, warm_start=WarmStart())
     assert float(np.linalg.norm(Ew - E) / np.linalg.norm(E)) < 2e-2
+
+
+@pytest.mark.parametrize("vol,C", [((1, 2, 4, 8), 8), ((1, 4, 4, 6), 40), ((2, 6, 4, 10), 24), ((1, 16, 16, 16), 96)])
+def test_transposed_im2col_equals_the_transpose_bit_for_bit(gpu, vol, C):
+    import torch
+    from wavesim_b200.warmstart import lib, pad64
+    L = lib()
+    b, d, h, w = vol
+    nvox, kp = b * d * h * w, pad64(27 * C)
+    ldo = pad64(nvox)
+    x = torch.randn(nvox, C, device="cuda").to(torch.bfloat16)
+    col = torch.empty(nvox, kp, device="cuda", dtype=torch.bfloat16)
+    want = torch.empty(kp, ldo, device="cuda", dtype=torch.bfloat16)
+    got = torch.full((kp, ldo), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert L.ws_net_im2col3(x.data_ptr(), col.data_ptr(), b, d, h, w, C, kp, None) == 0
+    assert L.ws_net_transpose_bf16(col.data_ptr(), want.data_ptr(), nvox, kp, kp, ldo, None) == 0
+    assert L.ws_net_im2col3_t(x.data_ptr(), got.data_ptr(), b, d, h, w, C, kp, ldo, None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 896, 64), (32, 1728, 1088), (128, 3456, 4096), (130, 200, 8256), (96, 33, 128)])
+def test_weight_gradient_is_the_gemm_bit_for_bit(gpu, M, N, K):
+    import torch
+    from wavesim_b200.warmstart import lib
+    L = lib()
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    B = torch.randn(N, K, device="cuda", generator=g).to(torch.bfloat16)
+    gw = torch.randn(M, N, device="cuda", generator=g)
+    want = torch.empty(M, N, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert _lib().ws_gemm_bf16(A.data_ptr(), B.data_ptr(), want.data_ptr(), None, None, M, N, K, K, K, N, 0,
+                               err.data_ptr(), None) == 0
+    want += gw
+    assert L.ws_net_wgrad_bf16(A.data_ptr(), B.data_ptr(), gw.data_ptr(), M, N, K, K, K, err.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    assert torch.equal(gw, want)

@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 
 #include "wavesim_b200.h"
@@ -244,6 +245,44 @@ __global__ void k_im2col3(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* _
     }
     *reinterpret_cast<uint4*>(col + row * kp + k) = val;
   }
+}
+
+// The transpose of im2col3's matrix, out[k][vox] with leading dimension ldo (a
+// multiple of 64; voxels from nvox on zero), written directly: a block gathers 64
+// voxels x 32 k in 16-byte chunks (8 channels of one tap) and turns them over
+// in shared memory, so that the 27-fold matrix crosses HBM once, not three
+// times (a layer of a 64^3 training step 21 us on average, against 21 + 42).
+__global__ void __launch_bounds__(256) k_im2col3_t(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+                                                   Vol v, int C, long long ldo) {
+  __shared__ __align__(16) __nv_bfloat16 tile[32][72];
+  const int t = threadIdx.x;
+  const long long nvox = (long long)v.b * v.d * v.h * v.w;
+  const long long v0 = (long long)blockIdx.x * 64;
+  const int k0 = blockIdx.y * 32;
+  {
+    const long long row = v0 + (t & 63);
+    const int k = k0 + 8 * (t >> 6);
+    const int tap = k / C;
+    uint4 val = make_uint4(0u, 0u, 0u, 0u);
+    if (tap < 27 && row < nvox) {
+      const int c = k - tap * C;
+      const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+      long long r = row;
+      const int x = (int)(r % v.w); r /= v.w;
+      const int y = (int)(r % v.h); r /= v.h;
+      const int z = (int)(r % v.d);
+      const int b = (int)(r / v.d);
+      const int zz = z + dz, yy = y + dy, xx = x + dx;
+      if (zz >= 0 && zz < v.d && yy >= 0 && yy < v.h && xx >= 0 && xx < v.w)
+        val = *reinterpret_cast<const uint4*>(in + vox_index(v, b, zz, yy, xx) * C + c);
+    }
+    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&val);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tile[8 * (t >> 6) + i][t & 63] = e[i];
+  }
+  __syncthreads();
+  const int r = t >> 3, c = (t & 7) * 8;
+  *reinterpret_cast<uint4*>(out + (long long)(k0 + r) * ldo + v0 + c) = *reinterpret_cast<const uint4*>(&tile[r][c]);
 }
 
 // Gradient of im2col3 (a gather, no atomics):
@@ -667,6 +706,120 @@ __global__ void __launch_bounds__(kGemmThreads)
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols));
 }
 
+// The weight gradient gw[M][N] += A[M][K] . B[N][K]^T: few output tiles, a K of
+// all voxels (32768 at 64^3).  k_gemm_bf16 (128 x 128 tiles, its loads behind the
+// same barrier as its MMAs) took 460 us a layer on average, 14 blocks of 512
+// steps of 0.9 us.  Here tiles of 32 columns give four times the blocks, and a
+// ring of cp.async stages keeps three steps in flight: 109 us on average, 276
+// for 512 steps.  What is left is the chain of dependent MMAs (8 or 11 stages,
+// or 64 columns, changed nothing).  K stays in one piece, in k_gemm_bf16's order
+// (16 at a time into the same fp32 accumulator), so the sums are its sums bit for
+// bit.  (Split over K it took 41 us in all, but then the sums round differently,
+// and Adam's first steps, which divide a gradient by its own size, carry that
+// into every weight.)
+constexpr int kWgradN = 32, kWgradStages = 5;
+__global__ void __launch_bounds__(kGemmThreads)
+    k_wgrad(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B, float* __restrict__ gw, int M, int N,
+            int K, long long lda, long long ldb, int* __restrict__ err) {
+  constexpr int NT = kWgradN, S = kWgradStages;
+  using T = ConvTile<NT>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t mbar[S];
+  __shared__ uint32_t tmem_base_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * NT;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"(T::kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+#pragma unroll
+    for (int i = 0; i < S; ++i) mbar_init(&mbar[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // rows of A beyond M: zero in every stage, once
+  const int rows = min(BM, (M - m0 + 15) & ~15);
+  for (int s = 0; s < S; ++s)
+    for (int q = tid; q < (BM - rows) * 8; q += kGemmThreads)
+      *reinterpret_cast<uint4*>(base + s * T::kStage + rows * 128 + q * 16) = make_uint4(0u, 0u, 0u, 0u);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_base_s;
+  const uint32_t sbase = smem_u32(base);
+  const int chunk = tid & 7, r0 = tid >> 3;
+  const uint32_t swz = (uint32_t)((chunk ^ (r0 & 7)) << 4);  // row & 7 is the same for all of a thread's rows
+  auto load_stage = [&](int kt, int s) {
+    const uint32_t sa = sbase + s * T::kStage, sb = sa + T::kA;
+    const long long k = (long long)kt * BK + chunk * 8;
+    for (int row = r0; row < rows; row += 16) {
+      const bool ok = m0 + row < M;
+      cp_async16(sa + row * 128 + swz, ok ? A + (long long)(m0 + row) * lda + k : A, ok ? 16u : 0u);
+    }
+#pragma unroll
+    for (int row = r0; row < NT; row += 16) {
+      const bool ok = n0 + row < N;
+      cp_async16(sb + row * 128 + swz, ok ? B + (long long)(n0 + row) * ldb + k : B, ok ? 16u : 0u);
+    }
+  };
+  const int nk = K / BK;
+  bool failed = false;
+#pragma unroll
+  for (int p = 0; p < S - 2; ++p) {
+    if (p < nk) load_stage(p, p);
+    cp_async_commit();
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    const int s = kt % S, kn = kt + S - 2;
+    if (kn < nk) {
+      // stage kn % S was last read by the MMAs of step kt - 2
+      if (kt >= 2 && !mbar_wait(&mbar[(kt - 2) % S], (uint32_t)(((kt - 2) / S) & 1))) failed = true;
+      if (!failed) load_stage(kn, kn % S);
+    }
+    cp_async_commit();
+    cp_async_wait<S - 2>();  // this thread's chunks of step kt have landed
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (__syncthreads_or(failed)) {
+      failed = true;
+      break;
+    }
+    if (tid == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t a0 = sbase + s * T::kStage, b0 = a0 + T::kA;
+#pragma unroll
+      for (int k = 0; k < BK / 16; ++k)
+        mma_bf16(tmem, make_desc(a0 + 32 * k), make_desc(b0 + 32 * k), T::kIdesc, (kt > 0 || k > 0) ? 1u : 0u);
+      mma_commit(&mbar[s]);
+    }
+  }
+  cp_async_wait<0>();
+  if (!failed && !mbar_wait(&mbar[(nk - 1) % S], (uint32_t)(((nk - 1) / S) & 1))) failed = true;
+  failed = __syncthreads_or(failed);
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!failed) {
+    const int row = m0 + warp * 32 + lane;
+#pragma unroll 1
+    for (int c0 = 0; c0 < NT; c0 += 16) {
+      float v[16];
+      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+      if (row < M) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int col = n0 + c0 + j;
+          if (col < N) gw[(long long)row * N + col] += v[j];
+        }
+      }
+    }
+  } else if (tid == 0) {
+    atomicExch(err, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::kCols));
+}
+
 // Network input features of a ROI (y fastest, then x, then z: the column-major
 // order of the ROI, which is also the network's (z, x, y) voxel order):
 // 8 bf16 channels per voxel [(n - n_bg) / 0.2, source amplitude, cos phi,
@@ -828,6 +981,32 @@ extern "C" int ws_gemm_bf16(const void* A, const void* B, float* C, void* Cb, co
   return WS_OK;
 }
 
+extern "C" int ws_net_wgrad_bf16(const void* A, const void* B, float* gw, int64_t M, int64_t N, int64_t K, int64_t lda,
+                                 int64_t ldb, int* err_flag, void* stream) {
+  if (M < 1 || N < 1 || K < 64 || K % 64 != 0 || K > (1LL << 30) || M > (1LL << 20) || N > (1LL << 30)) {
+    t_err = "ws_net_wgrad_bf16: need M, N >= 1 and K a positive multiple of 64";
+    return WS_ERR_INVALID_ARGUMENT;
+  }
+  if (lda % 8 || ldb % 8 || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || !err_flag) {
+    t_err = "ws_net_wgrad_bf16: A and B rows must be 16-byte aligned, and an error flag is needed";
+    return WS_ERR_INVALID_ARGUMENT;
+  }
+  using T = ConvTile<kWgradN>;
+  const size_t smem = kWgradStages * (size_t)T::kStage + 1024;
+  cudaError_t e = cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) {
+    k_wgrad<<<dim3((unsigned)((N + kWgradN - 1) / kWgradN), (unsigned)((M + BM - 1) / BM)), kGemmThreads, smem,
+              (cudaStream_t)stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)B, gw, (int)M, (int)N, (int)K, lda,
+                                      ldb, err_flag);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) {
+    t_err = std::string("ws_net_wgrad_bf16: ") + cudaGetErrorString(e);
+    return WS_ERR_CUDA;
+  }
+  return WS_OK;
+}
+
 // Layer entry points: device pointers, channels-last volumes of
 // (b, d, h, w) voxels, launched on `stream`.  Return WS_OK or WS_ERR_CUDA.
 #define NET_LAUNCH_CHECK()                                   \
@@ -848,6 +1027,17 @@ extern "C" int ws_net_im2col3(const void* in, void* col, int b, int d, int h, in
   Vol v{b, d, h, w};
   k_im2col3<<<grid_for((long long)b * d * h * w * (kp / 8)), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)in, (__nv_bfloat16*)col, v, C, kp);
+  NET_LAUNCH_CHECK();
+}
+extern "C" int ws_net_im2col3_t(const void* in, void* out, int b, int d, int h, int w, int C, int kp, int64_t ldo,
+                                void* stream) {
+  const int64_t nvox = (int64_t)b * d * h * w;
+  if (C % 8 || kp % 32 || ldo % 64 || ldo < nvox || kp / 32 > 65535 || ((uintptr_t)in & 15) || ((uintptr_t)out & 15)) {
+    t_err = "ws_net_im2col3_t: need C a multiple of 8, kp of 32, ldo >= voxels of 64, and 16-byte aligned buffers";
+    return WS_ERR_INVALID_ARGUMENT;
+  }
+  k_im2col3_t<<<dim3((unsigned)(ldo / 64), (unsigned)(kp / 32)), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)in, (__nv_bfloat16*)out, Vol{b, d, h, w}, C, ldo);
   NET_LAUNCH_CHECK();
 }
 extern "C" int ws_net_col2im3(const float* dcol, float* din, int b, int d, int h, int w, int C, int kp, void* stream) {

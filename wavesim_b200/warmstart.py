@@ -57,6 +57,8 @@ def _bind():
         "ws_net_flip_weights": [P, INT, INT, INT, P, INT, INT, P],
         "ws_net_relu_grad_bf16": [P, P, I64, INT, P, INT, P],
         "ws_net_im2col3": [P, P, INT, INT, INT, INT, INT, INT, P],
+        "ws_net_im2col3_t": [P, P, INT, INT, INT, INT, INT, INT, I64, P],
+        "ws_net_wgrad_bf16": [P, P, P, I64, I64, I64, I64, I64, P, P],
         "ws_net_col2im3": [P, P, INT, INT, INT, INT, INT, INT, P],
         "ws_net_transpose_f32_bf16": [P, P, I64, I64, I64, P],
         "ws_net_transpose_bf16": [P, P, I64, I64, I64, I64, P],
@@ -188,17 +190,13 @@ class Conv3:
         _ck(L.ws_net_add(self.gb.data_ptr(), gb.data_ptr(), self.cout, None), "add")
         # weight gradient: dW[co][k] = sum_vox dy[vox][co] im2col(x)[vox][k]
         voxp = pad64(nvox)
-        col = torch.empty(nvox, self.kp, device=dy.device, dtype=torch.bfloat16)
-        _ck(L.ws_net_im2col3(x.data_ptr(), col.data_ptr(), b, d, h, w, self.cin, self.kp, None), "im2col")
         colT = torch.empty(self.kp, voxp, device=dy.device, dtype=torch.bfloat16)
-        _ck(L.ws_net_transpose_bf16(col.data_ptr(), colT.data_ptr(), nvox, self.kp, self.kp, voxp, None), "transpose")
-        del col
+        _ck(L.ws_net_im2col3_t(x.data_ptr(), colT.data_ptr(), b, d, h, w, self.cin, self.kp, voxp, None), "im2col")
         dyT = torch.empty(self.cout, voxp, device=dy.device, dtype=torch.bfloat16)
         _ck(L.ws_net_transpose_f32_bf16(dy.data_ptr(), dyT.data_ptr(), nvox, self.cout, voxp, None), "transpose")
-        gw = torch.empty(self.cout, self.kp, device=dy.device)
-        _ck(_lib.lib.ws_gemm_bf16(dyT.data_ptr(), colT.data_ptr(), gw.data_ptr(), None, None, self.cout, self.kp,
-                                  voxp, voxp, voxp, self.kp, 0, _ptr(err), None), "gemm wgrad")
-        _ck(L.ws_net_add(self.gw.data_ptr(), gw.data_ptr(), gw.numel(), None), "add")
+        _ck(L.ws_net_wgrad_bf16(dyT.data_ptr(), colT.data_ptr(), self.gw.data_ptr(), self.cout, self.kp, voxp, voxp,
+                                voxp, _ptr(err if err is not None else torch.zeros(1, dtype=torch.int32, device=dy.device)),
+                                None), "gemm wgrad")
         del colT, dyT
         dx = None
         if need_dx:
