@@ -32,6 +32,8 @@ CASES = {
     "3d_64_planes_z_50": ((48, 48, 38), [8, 8, 6], False),
     "3d_vector_26x30x21": ((26, 18, 9), [0, 6, 6], True),
     "3d_vector_63x16x105": ((47, 16, 89), [8, 0, 8], True),
+    "2d_vector_45x60": ((33, 42), [6, 8], True),
+    "2d_vector_64x50": ((64, 50), [0, 0], True),
 }
 
 
@@ -49,7 +51,7 @@ def test_uni_matches_generic_and_oracle(gpu, name, monkeypatch):
     opt = {"lambda": 1.0, "pixel_size": 0.125 if vector else 0.25, "boundary_widths": bw, "energy_threshold": 1e-99,
            "max_iterations": iters}
     val = rng.standard_normal(shape[:2]) + 1j * rng.standard_normal(shape[:2])
-    pos = [1] * len(shape) + ([2] if vector else [])
+    pos = [1] * len(shape) + [1] * (3 - len(shape)) + ([2] if vector else [])
 
     def product():
         sim = (ws.WaveSimVector if vector else ws.WaveSim)(n, opt)

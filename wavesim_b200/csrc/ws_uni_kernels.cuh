@@ -417,7 +417,8 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
         for (int i = 0; i < R; ++i) p[i * ty] = v[i];
       } else {
         // f_g0_vector: div = (p . E) / k02e; E_i <- (E_i - p_i div) / (|p|^2 - k02e); the components
-        // one after the other, so that two lines of registers do for three
+        // one after the other, so that two lines of registers do for three (x, y, z: the pencil's own
+        // p is that of z in 3-D, of x in 2-D)
         float2 pe[R];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
@@ -428,7 +429,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
 #pragma unroll
           for (int i = 0; i < R; ++i) {
             p[c * tn + i * ty] = v[i];
-            const float pc = c == 0 ? pm : (c == 1 ? py : po[u + i * SL.units]);
+            const float pc = c == 1 ? py : ((c == 0) == (a.mode3d != 0) ? pm : po[u + i * SL.units]);
             pe[i] = c == 0 ? cscale(v[i], pc) : make_float2(fmaf(pc, v[i].x, pe[i].x), fmaf(pc, v[i].y, pe[i].y));
           }
         }
@@ -442,7 +443,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
             const float q = po[u + i * SL.units];
             const float dr = fmaf(q, q, base2);
             const float inv = a.norm * __frcp_rn(fmaf(dr, dr, di * di));
-            const float pc = c == 0 ? pm : (c == 1 ? py : q);
+            const float pc = c == 1 ? py : ((c == 0) == (a.mode3d != 0) ? pm : q);
             const float2 e = p[c * tn + i * ty];
             v[i] = cmul(make_float2(fmaf(-pc, pe[i].x, e.x), fmaf(-pc, pe[i].y, e.y)),
                         make_float2(dr * inv, -di * inv));
