@@ -7,7 +7,7 @@
  * tcgen05 tensor cores (bf16 operands, fp32 accumulation in tensor memory):
  * the forward pass and the input gradient as implicit GEMMs that gather
  * their operand in the kernel (ws_conv3_fwd_bf16), the weight gradient as an
- * explicit GEMM (ws_gemm_bf16) of transposed im2col matrices.  The other
+ * explicit GEMM (ws_net_wgrad_bf16) of transposed im2col matrices.  The other
  * entry points are the layer kernels around them.
  *
  * Every pointer is a device pointer; activations are channels-last

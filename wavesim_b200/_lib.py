@@ -203,12 +203,12 @@ def default_options():
 
 
 class HostStage:
-    """A reusable page-locked (pinned) host buffer that a solver's outputs
-    land in, so that the device-to-host copy runs at the bus speed instead of
-    through the driver's pageable staging (64 MB of fields: about 1 ms
-    against 25 ms on the B200 boxes), then copied into an ordinary numpy
+    """A reusable page-locked (pinned) host buffer for outputs that the library
+    does not stage itself (PSTD's field, the device copies of a continuation
+    sweep), so that the device-to-host copy runs at the bus speed instead of
+    through the driver's pageable staging, then copied into an ordinary numpy
     array for the caller.  The buffer grows as needed and is reused by every
-    solve of its owner (one per WaveSim, so concurrent solvers do not share
+    solve of its owner (one per simulation, so concurrent solvers do not share
     one); without CUDA it is plain host memory."""
 
     def __init__(self):

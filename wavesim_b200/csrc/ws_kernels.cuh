@@ -15,8 +15,9 @@
 //                  ifftn folded in), inverse FFT over the outer dimension, in place on T
 // K3 k_inv_inner : inverse FFT over the inner dimensions, conj ramps
 //                  (WaveSim.m:55), f_mix (f_mix.m:3-4), E += dE, the ROI energy
-//                  sum(|dE|^2) (Simulation.m:265-273) and, in the last block to
-//                  finish, the stop rule of Simulation.next (Simulation.m:193-217).
+//                  sum(|dE|^2) (Simulation.m:265-273), per-block partial sums.
+// k_finish_iterations : once per wiggle cycle, adds those sums up and applies the
+//                  stop rule of Simulation.next (Simulation.m:193-217).
 //
 // A 3-D plane that does not fit one block's shared memory is split over a
 // cluster of C blocks along x: the x transform is then one radix-C step across

@@ -2,10 +2,10 @@
 //
 // Host runtime: FFT planning (radix schedules, twiddle tables, tile and
 // cluster shapes), device buffers, the per-solver CUDA stream, and the loop
-// driver.  The loop runs either as one CUDA graph (first wiggle cycle with the
-// source, then a device-side while node over the steady cycle whose condition
-// the last block of the cycle's final K3 sets) or, when a host callback needs
-// the history, as launches from a host loop.
+// driver.  The loop runs as one cooperative launch (small 2-D grids), as one
+// CUDA graph (first wiggle cycle with the source, then a device-side while node
+// over the steady cycle whose condition the cycle's stop-rule launch sets) or,
+// when a host callback needs the history, as launches from a host loop.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -294,7 +294,7 @@ class WaveSim:
         return np.real(n[lo[0]:hi[0], lo[1]:hi[1], lo[2]:hi[2]]).astype(np.float32)
 
     def _stage(self):
-        """This simulation's pinned staging buffer for solver outputs."""
+        """This simulation's pinned staging buffer for the device copies of a continuation sweep."""
         if getattr(self, "_hstage", None) is None:
             self._hstage = _lib.HostStage()
         return self._hstage
