@@ -12,7 +12,10 @@ float64 and written as float literals.
 
 Run:  python gen_codelets.py > ws_codelets.cuh
 """
+import cmath
 import math
+import re
+import struct
 
 RADICES = [2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16]
 
@@ -172,6 +175,42 @@ def codelet(R, inverse):
             f"  static __host__ __device__ __forceinline__ void run(float2 (&v)[{R}]) {{  // {name}\n{body}\n  }}\n}};\n")
 
 
+def single(v):
+    """v rounded to single precision, as the compiler rounds a literal."""
+    return struct.unpack("f", struct.pack("f", v))[0]
+
+
+def matrix(R, inverse):
+    """What codelet(R, inverse) multiplies by, its constants rounded to single precision and its arithmetic exact
+    (in float64): a list of columns."""
+    text = codelet(R, inverse)
+    text = re.sub(r"(\d+(?:\.\d+)?(?:e[+-]\d+)?)f\b", lambda m: repr(single(float(m.group(1)))), text)
+    steps = []
+    for name, expr in re.findall(r"const float (t\d+) = (.*?);", text):
+        steps.append((name, compile(re.sub(r"v\[(\d+)\]\.([xy])", r"v\2[\1]", expr), name, "eval")))
+    outs = [compile("complex(%s)" % e, "out", "eval") for e in re.findall(r"= make_float2\((.*?)\);", text)]
+    cols = []
+    for n in range(R):
+        env = {"fmaf": lambda a, b, c: a * b + c, "vx": [float(i == n) for i in range(R)], "vy": [0.0] * R}
+        for name, code in steps:
+            env[name] = eval(code, env)
+        cols.append([eval(code, env) for code in outs])
+    return cols
+
+
+def gains(R):
+    """The real parts of the relative errors of the butterflies' matrices, averaged: the forward one's by input and by
+    output, the inverse one's by input and by output."""
+    found = []
+    for inverse in (False, True):
+        m = matrix(R, inverse)  # m[n][k]: input n, output k
+        sign = 2j if inverse else -2j
+        e = [[(m[n][k] * cmath.exp(-sign * math.pi * (n * k % R) / R)).real - 1.0 for k in range(R)] for n in range(R)]
+        found.append([sum(e[i]) / R for i in range(R)])
+        found.append([sum(e[n][i] for n in range(R)) / R for i in range(R)])
+    return found
+
+
 def main():
     out = ["// Generated by gen_codelets.py - do not edit by hand.",
            "// Small in-register DFTs: Dft<R, INV>::run(v) transforms v[0..R) in place,",
@@ -190,6 +229,28 @@ def main():
     out.append("constexpr int kNumRadices = %d;" % len(RADICES))
     out.append("constexpr int kRadices[kNumRadices] = {%s};" % ", ".join(map(str, RADICES)))
     out.append("")
+    def table(name, comment, rows):
+        out.extend("// " + c for c in comment)
+        out.append(name + " {")
+        out.append("  constexpr double g[%d][%d][%d] = {" % (len(rows[-1]), max(RADICES) + 1, max(RADICES)))
+        for which in range(len(rows[-1])):
+            out.append("      {")
+            for r in rows:
+                out.append("          {%s}," % ", ".join("%.6e" % v if abs(v) > 1e-12 else "0" for v in (r[which] if r else [])))
+            out.append("      },")
+        out.append("  };")
+
+    g = [gains(R) if R in RADICES else None for R in range(max(RADICES) + 1)]
+    table("inline double butterfly_gain(int which, int R, int i)",
+          ["The butterflies' constants are rounded to single precision: the real part of their matrices' relative error,",
+           "averaged; which = 0, 1: the forward one by input i, by output i; 2, 3: the inverse one."], g)
+    out += ["  return g[which][R][i];", "}"]
+    table("__host__ __device__ constexpr double round_trip(int side, int R, int i)",
+          ["Forward and inverse butterflies in a row multiply by R (1 + gain), apart from what they mix in of the others:",
+           "side 0 the gain of frequency i (inverse, then forward), 1 that of input i (forward, then inverse).  A literal",
+           "where R and i are known."],
+          [q and [[a + b for a, b in zip(q[1], q[2])], [a + b for a, b in zip(q[0], q[3])]] for q in g])
+    out += ["  return g[side][R][i];", "}", ""]
     out.append("}  // namespace ws")
     print("\n".join(out))
 

@@ -1776,4 +1776,134 @@ template <> struct Dft<16, true> {
 constexpr int kNumRadices = 15;
 constexpr int kRadices[kNumRadices] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16};
 
+// The butterflies' constants are rounded to single precision: the real part of their matrices' relative error,
+// averaged; which = 0, 1: the forward one by input i, by output i; 2, 3: the inverse one.
+inline double butterfly_gain(int which, int R, int i) {
+  constexpr double g[4][17][16] = {
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -8.974116e-09, -8.974116e-09},
+          {0, 0, 0, 0},
+          {0, 1.074062e-08, 1.074062e-08, 1.074062e-08, 1.074062e-08},
+          {0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08},
+          {0, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09},
+          {0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09},
+          {0, -1.240993e-08, -1.670447e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08},
+          {0, 1.162006e-08, 2.328697e-08, 2.328697e-08, 1.162006e-08, 0, 1.162006e-08, 2.328697e-08, 2.328697e-08, 1.162006e-08},
+          {0, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09},
+          {0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08},
+          {0, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10},
+          {0, -1.632419e-08, 1.124557e-09, -1.040063e-08, -1.040063e-08, 1.124557e-09, -1.632419e-08, 0, -1.632419e-08, 1.124557e-09, -1.040063e-08, -1.040063e-08, 1.124557e-09, -1.632419e-08},
+          {0, 2.107566e-09, 1.759304e-08, 1.969114e-08, 2.540721e-08, -8.974116e-09, -6.866550e-09, 8.618926e-09, 1.071703e-08, 1.643310e-08, -8.974116e-09, -6.866550e-09, 8.618926e-09, 1.071703e-08, 1.643310e-08},
+          {0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08},
+      },
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -8.974116e-09, -8.974116e-09},
+          {0, 0, 0, 0},
+          {0, 1.074062e-08, 1.074062e-08, 1.074062e-08, 1.074062e-08},
+          {0, -8.974116e-09, -8.974116e-09, -1.794823e-08, -8.974116e-09, -1.794823e-08},
+          {0, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09},
+          {0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09},
+          {0, -1.240993e-08, -1.670447e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08},
+          {0, 1.074062e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08},
+          {0, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09},
+          {0, -8.974116e-09, -8.974116e-09, 0, -8.974116e-09, -1.794823e-08, -1.794823e-08, -8.974116e-09, -8.974116e-09, -1.794823e-08, -1.794823e-08, -8.974116e-09},
+          {0, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10},
+          {0, -5.389529e-09, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08},
+          {0, -5.025859e-09, 1.795115e-10, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08},
+          {0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08},
+      },
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -8.974116e-09, -8.974116e-09},
+          {0, 0, 0, 0},
+          {0, 1.074062e-08, 1.074062e-08, 1.074062e-08, 1.074062e-08},
+          {0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08},
+          {0, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09},
+          {0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09},
+          {0, -1.240993e-08, -1.670447e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08},
+          {0, 1.162006e-08, 2.328697e-08, 2.328697e-08, 1.162006e-08, 0, 1.162006e-08, 2.328697e-08, 2.328697e-08, 1.162006e-08},
+          {0, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09},
+          {0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08, 0, -1.570470e-08, -1.570470e-08},
+          {0, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10},
+          {0, -1.632419e-08, 1.124557e-09, -1.040063e-08, -1.040063e-08, 1.124557e-09, -1.632419e-08, 0, -1.632419e-08, 1.124557e-09, -1.040063e-08, -1.040063e-08, 1.124557e-09, -1.632419e-08},
+          {0, 2.107566e-09, 1.759304e-08, 1.969114e-08, 2.540721e-08, -8.974116e-09, -6.866550e-09, 8.618926e-09, 1.071703e-08, 1.643310e-08, -8.974116e-09, -6.866550e-09, 8.618926e-09, 1.071703e-08, 1.643310e-08},
+          {0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08},
+      },
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -8.974116e-09, -8.974116e-09},
+          {0, 0, 0, 0},
+          {0, 1.074062e-08, 1.074062e-08, 1.074062e-08, 1.074062e-08},
+          {0, -8.974116e-09, -8.974116e-09, -1.794823e-08, -8.974116e-09, -1.794823e-08},
+          {0, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09, -5.389529e-09},
+          {0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09, 0, -8.557136e-09},
+          {0, -1.240993e-08, -1.670447e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08, -8.974116e-09, -2.138405e-08, -2.567859e-08},
+          {0, 1.074062e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08, 1.074062e-08, 2.148125e-08},
+          {0, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09, -3.575949e-09},
+          {0, -8.974116e-09, -8.974116e-09, 0, -8.974116e-09, -1.794823e-08, -1.794823e-08, -8.974116e-09, -8.974116e-09, -1.794823e-08, -1.794823e-08, -8.974116e-09},
+          {0, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10, 6.025156e-10},
+          {0, -5.389529e-09, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08, -5.389529e-09, -1.077906e-08},
+          {0, -5.025859e-09, 1.795115e-10, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08, 1.074062e-08, 5.714763e-09, 1.092013e-08},
+          {0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08, 0, -1.854571e-08, -8.557136e-09, -1.854571e-08},
+      },
+  };
+  return g[which][R][i];
+}
+// Forward and inverse butterflies in a row multiply by R (1 + gain), apart from what they mix in of the others:
+// side 0 the gain of frequency i (inverse, then forward), 1 that of input i (forward, then inverse).  A literal
+// where R and i are known.
+__host__ __device__ constexpr double round_trip(int side, int R, int i) {
+  constexpr double g[2][17][16] = {
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -1.794823e-08, -1.794823e-08},
+          {0, 0, 0, 0},
+          {0, 2.148125e-08, 2.148125e-08, 2.148125e-08, 2.148125e-08},
+          {0, -2.467882e-08, -2.467882e-08, -1.794823e-08, -2.467882e-08, -3.365293e-08},
+          {0, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08},
+          {0, -1.711427e-08, 0, -1.711427e-08, 0, -1.711427e-08, 0, -1.711427e-08},
+          {0, -2.481987e-08, -3.340894e-08, -1.794823e-08, -4.276810e-08, -5.135717e-08, -1.794823e-08, -4.276810e-08, -5.135717e-08},
+          {0, 2.236068e-08, 3.402759e-08, 4.476821e-08, 2.236068e-08, 2.148125e-08, 2.236068e-08, 4.476821e-08, 3.402759e-08, 3.310130e-08},
+          {0, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09},
+          {0, -2.467882e-08, -2.467882e-08, 0, -2.467882e-08, -3.365293e-08, -1.794823e-08, -2.467882e-08, -2.467882e-08, -1.794823e-08, -3.365293e-08, -2.467882e-08},
+          {0, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09},
+          {0, -2.171372e-08, -4.264971e-09, -2.117969e-08, -1.579016e-08, -9.654500e-09, -2.171372e-08, -1.077906e-08, -2.171372e-08, -9.654500e-09, -1.579016e-08, -2.117969e-08, -4.264971e-09, -2.710325e-08},
+          {0, -2.918294e-09, 1.777255e-08, 3.043176e-08, 3.112198e-08, 1.946019e-09, 3.874073e-09, 1.433369e-08, 2.163716e-08, 2.717372e-08, -3.259352e-09, 4.053584e-09, 1.935955e-08, 1.643179e-08, 2.735323e-08},
+          {0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08},
+      },
+      {
+          {},
+          {},
+          {0, 0},
+          {0, -1.794823e-08, -1.794823e-08},
+          {0, 0, 0, 0},
+          {0, 2.148125e-08, 2.148125e-08, 2.148125e-08, 2.148125e-08},
+          {0, -2.467882e-08, -2.467882e-08, -1.794823e-08, -2.467882e-08, -3.365293e-08},
+          {0, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08, -1.077906e-08},
+          {0, -1.711427e-08, 0, -1.711427e-08, 0, -1.711427e-08, 0, -1.711427e-08},
+          {0, -2.481987e-08, -3.340894e-08, -1.794823e-08, -4.276810e-08, -5.135717e-08, -1.794823e-08, -4.276810e-08, -5.135717e-08},
+          {0, 2.236068e-08, 3.402759e-08, 4.476821e-08, 2.236068e-08, 2.148125e-08, 2.236068e-08, 4.476821e-08, 3.402759e-08, 3.310130e-08},
+          {0, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09, -7.151898e-09},
+          {0, -2.467882e-08, -2.467882e-08, 0, -2.467882e-08, -3.365293e-08, -1.794823e-08, -2.467882e-08, -2.467882e-08, -1.794823e-08, -3.365293e-08, -2.467882e-08},
+          {0, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09, 1.205031e-09},
+          {0, -2.171372e-08, -4.264971e-09, -2.117969e-08, -1.579016e-08, -9.654500e-09, -2.171372e-08, -1.077906e-08, -2.171372e-08, -9.654500e-09, -1.579016e-08, -2.117969e-08, -4.264971e-09, -2.710325e-08},
+          {0, -2.918294e-09, 1.777255e-08, 3.043176e-08, 3.112198e-08, 1.946019e-09, 3.874073e-09, 1.433369e-08, 2.163716e-08, 2.717372e-08, -3.259352e-09, 4.053584e-09, 1.935955e-08, 1.643179e-08, 2.735323e-08},
+          {0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08, 0, -3.709142e-08, -1.711427e-08, -3.709142e-08},
+      },
+  };
+  return g[side][R][i];
+}
+
 }  // namespace ws

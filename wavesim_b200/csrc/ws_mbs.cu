@@ -16,6 +16,7 @@
 #include <string>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <vector>
 
 #include "wavesim_b200.h"
@@ -32,6 +33,7 @@ constexpr int kEmax = 16;           // max elements per thread per FFT stage
 constexpr int kMaxThreadsPow2 = 512;
 constexpr int kMaxThreadsMixed = 512;
 constexpr size_t kSmemBudget = 150 * 1024;  // per-block tile budget (bytes)
+constexpr size_t kSmemMax = 227 * 1024;     // what a block can have
 constexpr int kNumSms = 148;
 constexpr long long kLoopCycles = 512;  // wiggle cycles of one cooperative launch (uni::k_loop)
 
@@ -366,6 +368,12 @@ static bool uni_plan(int n, uni::Plan& P) {
   return true;
 }
 
+// W_n^{j r} of a stage on blocks of n
+static float2 uni_twiddle(int j, int r, int n) {
+  const double a = -2.0 * M_PI * (double)((long long)j * r % n) / (double)n;
+  return make_float2((float)std::cos(a), (float)std::sin(a));
+}
+
 // The frequency of each element of a forward transform in the order of T.
 static std::vector<int> uni_permutation(const uni::Plan& P) {
   std::vector<int> k(P.n);
@@ -381,6 +389,72 @@ static std::vector<int> uni_permutation(const uni::Plan& P) {
     for (int i = 0; i < L.R; ++i) k[u + i * L.units] = rev + i * L.units;
   }
   return k;
+}
+
+// |w| - 1 of a rounded twiddle
+static double excess(float2 w) { return 0.5 * ((double)w.x * w.x + (double)w.y * w.y - 1.0); }
+
+// The rounded constants of the butterflies and the twiddles make a forward and
+// an inverse transform in a row multiply by N (1 + a few 1e-8) instead of N, the same
+// in every iteration of a solve.  To first order the factor is 1 + p + f: p a
+// function of the position (each stage's butterfly on that input, and the mean
+// |W|^2 - 1 of its twiddles over the butterfly's outputs), f one of the frequency with
+// a mean of zero (the butterflies' outputs, and the mean over the positions).
+// pos: p of j + r n / R0 is pos[j] + round_trip(1, R0, r); freq, in the order of
+// T: f of u + i n / RL is freq[u] + round_trip(0, RL, i) (both are 0 for r = i = 0).
+static void uni_gains(const uni::Plan& P, std::vector<double>& pos, std::vector<double>& freq) {
+  pos.assign(P.n, 0.0);
+  freq.assign(P.n, 0.0);
+  double mean = 0.0;
+  for (int s = 0, span = P.n; s < P.nst; ++s) {
+    const uni::Stage& S = P.st[s];
+    std::vector<double> tin(S.sub, 0.0), out(S.R, 0.0);
+    for (int r = 0; r < S.R; ++r) {
+      for (int j = 0; j < S.sub; ++j) {
+        const double g = 2.0 * excess(uni_twiddle(j, r, S.R * S.sub));
+        tin[j] += g / S.R;
+        out[r] += g / S.sub;
+      }
+      out[r] += round_trip(0, S.R, r);
+      mean += out[r] / S.R;
+    }
+    for (int i = 0; i < P.n; ++i) pos[i] += tin[i % S.sub] + round_trip(1, S.R, i / S.sub % S.R);
+    // the digit of stage s of element u + i n / RL: of u, or i
+    const int units = P.st[P.nst - 1].units;
+    span = s < P.nst - 1 ? span / S.R : 1;
+    for (int k = 0; k < P.n; ++k)
+      freq[k] += s < P.nst - 1 ? out[k % units / (span / P.st[P.nst - 1].R) % S.R] : out[k / units];
+  }
+  for (double& f : freq) f -= mean;
+}
+
+// The same for the compile-time schedules of columns (Stockham: stage s takes
+// the digit of weight N / (R0 .. Rs) of its input, multiplies it by W_{Ns Rs}^{jm r},
+// jm the digits of the output so far, and gives the output's digit of weight
+// Ns = R0 .. Rs-1; the inverse is the same with conjugate constants).
+static void line_gains(const std::vector<int>& radix, std::vector<double>& pos, std::vector<double>& freq) {
+  const int n = std::accumulate(radix.begin(), radix.end(), 1, std::multiplies<int>());
+  pos.assign(n, 0.0);
+  freq.assign(n, 0.0);
+  int Ns = 1, rest = n;
+  for (int R : radix) {
+    rest /= R;
+    std::vector<double> by_input(R, 0.0), by_output(Ns, 0.0);  // of the twiddles
+    for (int r = 0; r < R; ++r)
+      for (int j = 0; j < Ns; ++j) {
+        const double g = excess(uni_twiddle(j, r, Ns * R));
+        by_input[r] += g / Ns;
+        by_output[j] += g / R;
+      }
+    for (int i = 0; i < n; ++i) {
+      const int in = i / rest % R, out = i / Ns % R;
+      pos[i] += butterfly_gain(0, R, in) + by_input[in] + butterfly_gain(3, R, out) + by_output[i % Ns];
+      freq[i] += butterfly_gain(1, R, out) + by_output[i % Ns] + butterfly_gain(2, R, in) + by_input[in];
+    }
+    Ns *= R;
+  }
+  const double mean = std::accumulate(freq.begin(), freq.end(), 0.0) / n;
+  for (double& f : freq) f -= mean;
 }
 
 static int uni_units(const uni::Plan& P) {
@@ -422,7 +496,7 @@ static void uni_pencils(UniPass& p, int ny, int nc, long long mids) {
   int w = std::max(1, std::min(um, uni::kMaxThreads / ty));
   while ((w * ty) % 32 && w * ty + ty <= uni::kMaxThreads) ++w;
   p.threads = w * ty;
-  p.smem = ty * row + p.plan.n * sizeof(float);
+  p.smem = ty * row + (p.plan.n + p.plan.st[p.plan.nst - 1].units) * sizeof(float);
   p.grid = (long long)((ny + ty - 1) / ty) * mids;
 }
 
@@ -478,7 +552,7 @@ static size_t loop_smem(const Layout& L, const Geom& g, int nw, bool e_resident,
   if (tile_elems) *tile_elems = (int)tile;
   const size_t tables = L.ucol.plan.ntw + L.uout.plan.ntw + nw * (g.ny + l);
   return (tile + tables + l * g.ny * (e_resident ? 3 : 2)) * sizeof(float2) + l * 16 +
-         (uni_groups(L.ucol) + (size_t)nw * L.uout.plan.n) * sizeof(float);
+         (uni_groups(L.ucol) + (size_t)nw * L.uout.plan.n + L.uout.plan.st[L.uout.plan.nst - 1].units) * sizeof(float);
 }
 constexpr size_t kLoopSmem = 225 * 1024;
 // ... of PSTD's stepping: two fields, the source and three coefficients a point
@@ -487,7 +561,7 @@ static size_t pstd_loop_smem(const Layout& L, const Geom& g, int* tile_elems = n
   const size_t tile = std::max(l * L.ucol.plan.np, (size_t)L.uout.lines * L.uout.plan.n);
   if (tile_elems) *tile_elems = (int)tile;
   return (tile + L.ucol.plan.ntw + L.uout.plan.ntw + 4 * l * g.ny) * sizeof(float2) + l * 16 +
-         (uni_groups(L.ucol) + (size_t)L.uout.plan.n + l * g.ny) * sizeof(float);
+         (uni_groups(L.ucol) + (size_t)L.uout.plan.n + l * g.ny + L.uout.plan.st[L.uout.plan.nst - 1].units) * sizeof(float);
 }
 // The layout of single solves of small 2-D grids, `L` being the one of the
 // grid's launched passes; false if there is none.  Measured against the
@@ -681,18 +755,20 @@ static int make_layout(const Geom& g, Layout& L, std::string& why, const LayoutC
   // along the lines that those kernels transform: along the outer dimension
   // for every pairing, along y and x only if they run both passes.  (PSTD
   // feeds T through K1 a second time, which needs natural order there.)
-  L.uni_out = !L.tp && !L.fp && ch.outer != 2 && uni_plan(no, L.uout.plan);
-  if (L.uni_out) {
+  if (!L.tp && !L.fp && ch.outer != 2 && uni_plan(no, L.uout.plan)) {
     uni_pencils(L.uout, g.ny, g.nc, mids);
-    L.grid_outer = L.uout.grid;
+    L.uni_out = L.uout.smem <= kSmemMax;
+    if (L.uni_out) L.grid_outer = L.uout.grid;
   }
-  L.uni_in = L.uni_out && !L.fi && !pstd && ch.inner != 2 && !ch.csize && !ch.ncols && !ch.sched &&
-             uni_plan(g.ny, L.ucol.plan) && (!L.mode3d || uni_plan(g.nx, L.ux.plan));
-  if (L.uni_in) {
+  if (L.uni_out && !L.fi && !pstd && ch.inner != 2 && !ch.csize && !ch.ncols && !ch.sched &&
+      uni_plan(g.ny, L.ucol.plan) && (!L.mode3d || uni_plan(g.nx, L.ux.plan))) {
     uni_columns(L.ucol, (long long)g.nx * g.nz * g.nc);
     if (L.mode3d) uni_pencils(L.ux, g.ny, 1, (long long)g.nz * g.nc);
-    L.grid_inner = L.ucol.grid;
-    L.pitch = (g.ny + 3) / 4 * 4;
+    L.uni_in = std::max(L.ucol.smem, L.ux.smem) <= kSmemMax;  // a column of 8192 points does not fit
+    if (L.uni_in) {
+      L.grid_inner = L.ucol.grid;
+      L.pitch = (g.ny + 3) / 4 * 4;
+    }
   }
   return WS_OK;
 }
@@ -713,11 +789,17 @@ struct GraphKey {
 };
 
 // Device tables of a layout's run-time scheduled plans, in one buffer: the
-// wiggles (natural, and with the p tables in the order of T), the twiddles, the
-// permutation of the p tables, the permuted p tables.
+// wiggles (p tables in the order of T, ramps of k_balance_ramps), the twiddles,
+// the ramps, the permutation of the p tables, what takes the transforms' gains
+// out again by frequency and by position (minus uni_gains; 0 along the axes that
+// other kernels transform), the permuted p tables.
 struct UniTables {
   Wig* wigs = nullptr;
+  float2* ramp = nullptr;
   int* perm = nullptr;
+  int axes = 0;  // bit d: axis d (x, y, z) takes its ramps from k_balance_ramps
+  float* efreq = nullptr;
+  float* epos = nullptr;
   float* p = nullptr;
   std::vector<Wig> uwig;
 };
@@ -831,6 +913,22 @@ static int build_plan(int n, const std::vector<float2>& tw_all_offset_dummy, Fft
   return WS_OK;
 }
 
+// The radices of the compile-time schedules (empty: none).
+static std::vector<int> line_radices(int n) {
+  switch (n) {
+    case 96: return {12, 4, 2};
+    case 160: return {10, 4, 4};
+    case 192: return {12, 4, 4};
+    case 224: return {14, 4, 4};
+    case 320: return {4, 4, 4, 5};
+    case 448: return {14, 4, 4, 2};
+    case 576: return {12, 12, 4};
+  }
+  if (n < 32 || n > 2048 || (n & (n - 1))) return {};
+  if (n <= 256) return {16, n / 16};
+  return {16, 16, n / 256};
+}
+
 // The table exp(-2 pi i k / n); behind it, for the lengths with a compile-time
 // schedule, the tables of its second stage and on: W_{Ns R}^{jm r} at r Ns + jm
 // (fast::line_stage with ST, mixed::Plan::table).
@@ -841,20 +939,8 @@ static void push_twiddles(std::vector<float2>& all, int n, size_t& off) {
     all.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
   };
   for (int k = 0; k < n; ++k) push(k, n);
-  std::vector<int> radix;
-  switch (n) {  // the compile-time schedules
-    case 96: radix = {12, 4, 2}; break;
-    case 160: radix = {10, 4, 4}; break;
-    case 192: radix = {12, 4, 4}; break;
-    case 224: radix = {14, 4, 4}; break;
-    case 320: radix = {4, 4, 4, 5}; break;
-    case 448: radix = {14, 4, 4, 2}; break;
-    case 576: radix = {12, 12, 4}; break;
-    default:
-      if (n < 32 || n > 2048 || (n & (n - 1))) return;
-      radix = {16, n <= 256 ? n / 16 : 16};
-      if (n > 256) radix.push_back(n / 256);
-  }
+  const std::vector<int> radix = line_radices(n);
+  if (radix.empty()) return;
   for (int s = 1, Ns = radix[0]; s < (int)radix.size(); Ns *= radix[s++])
     for (int r = 0; r < radix[s]; ++r)
       for (int j = 0; j < Ns; ++j) push((double)j * r * (n / (Ns * radix[s])), n);
@@ -909,7 +995,8 @@ static int set_kernel_attributes() {
   for (const TmaPencil& f : tma_pencil2d_table()) WS_CUDA(allow_dynamic_smem(f.fn, optin));
   for (int c = 0; c < uni::kClasses; ++c) {
     const uni::Kernels& k = uni_kernels(c);
-    for (const void* f : k.col) WS_CUDA(allow_dynamic_smem(f, optin));
+    for (const auto& dims : k.col)
+      for (const void* f : dims) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.x) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : k.pencil) WS_CUDA(allow_dynamic_smem(f, optin));
     for (const void* f : {k.loop, k.pstd_loop}) {
@@ -968,13 +1055,56 @@ static __global__ void k_permute_tables(float* __restrict__ per, const float* __
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nf) per[(long long)blockIdx.y * nf + i] = nat[(long long)blockIdx.y * nf + perm[i]];
 }
+// The ramps with moduli that take the transforms' gains by position out:
+// |g|^2 = 1 - pos, 1e-8 from 1, is no pair of floats, so each element takes the
+// neighbour (of up to one ulp each way) that brings the sum over its 32
+// elements nearest to it.  That also takes out the mean of the plain rounding.
+// (Ramps of another modulus than 1 keep it.)  Rounding the ramps alone moves
+// the converged field of 81 x 360 points by 6.0e-7, these by 2.6e-7 (165 x 400:
+// 3.9e-7, 2.6e-7).
+static __global__ void k_balance_ramps(float2* __restrict__ out, const float2* __restrict__ ramp,
+                                       const float* __restrict__ epos, int nx, int ny, int nf, int axes) {
+  const int i0 = 32 * (blockIdx.x * blockDim.x + threadIdx.x);
+  out += (long long)blockIdx.y * nf;
+  ramp += (long long)blockIdx.y * nf;
+  double carry = 0.0;
+  for (int i = i0; i < min(nf, i0 + 32); ++i) {
+    const float2 g = ramp[i];
+    float2 best = g;
+    if (i == nx || i == nx + ny) carry = 0.0;
+    if (axes >> (i < nx ? 0 : (i < nx + ny ? 1 : 2)) & 1) {
+      double m = (double)g.x * g.x + (double)g.y * g.y;
+      if (fabs(m - 1.0) < 1e-6) m = 1.0;
+      const double want = m * (1.0 + epos[i]) + carry;
+      double least = 1e300, rest = 0.0;
+      for (int k = 0; k < 9; ++k) {
+        const int a = k / 3, b = k % 3;
+        if (b && g.y == 0.f) continue;
+        const float2 c = make_float2(a ? nextafterf(g.x, a == 1 ? 2.f : -2.f) : g.x,
+                                     b ? nextafterf(g.y, b == 1 ? 2.f : -2.f) : g.y);
+        const double left = want - ((double)c.x * c.x + (double)c.y * c.y);
+        const double cost = fabs(left) + 0.05 * (fabs((double)c.x - g.x) + fabs((double)c.y - g.y));
+        if (cost < least) {
+          least = cost;
+          rest = left;
+          best = c;
+        }
+      }
+      carry = fabs(rest) < 1e-6 ? rest : 0.0;
+    }
+    out[i] = best;
+  }
+}
 static cudaError_t permute_wiggles(Solver* s) {
   cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);  // the tables' uploads
   if (e != cudaSuccess) return e;
   const int nf = s->g.nx + s->g.ny + s->g.nz;
   for (const UniTables& t : s->ut)
-    if (t.wigs)
+    if (t.wigs) {
       k_permute_tables<<<dim3((nf + 255) / 256, s->nw), 256, 0, s->stream>>>(t.p, s->d_wigf, t.perm, nf);
+      k_balance_ramps<<<dim3((nf + 1023) / 1024, s->nw), 32, 0, s->stream>>>(t.ramp, s->d_wigc, t.epos, s->g.nx, s->g.ny,
+                                                                           nf, t.axes);
+    }
   return cudaGetLastError();
 }
 
@@ -995,26 +1125,40 @@ static cudaError_t make_tables(Solver* s, int k) {
       const uni::Stage& S = plans[q]->st[i];
       const int n = S.R * S.sub;
       for (int r = 0; r < S.R; ++r)
-        for (int j = 0; j < S.sub; ++j) {
-          const double a = -2.0 * M_PI * (double)((long long)j * r % n) / (double)n;
-          tw.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
-        }
+        for (int j = 0; j < S.sub; ++j) tw.push_back(uni_twiddle(j, r, n));
     }
   }
   std::vector<int> perm;
+  std::vector<float> efreq, epos;
   for (int d = 0; d < 3; ++d) {
     const int off = (int)perm.size();
     const std::vector<int> f = axis[d] ? uni_permutation(*axis[d]) : std::vector<int>();
-    for (int i = 0; i < len[d]; ++i) perm.push_back(off + (axis[d] ? f[i] : i));
+    std::vector<double> pos(len[d], 0.0), freq(len[d], 0.0);
+    const bool columns = d == 1 && L.fi && !L.mode3d;  // compile-time columns, inside these kernels' pencils
+    if (axis[d]) uni_gains(*axis[d], pos, freq);
+    if (columns) line_gains(line_radices(g.ny), pos, freq);
+    // without ramps of its own (PSTD, other column passes), the mean of the part by position
+    const bool ramps = (L.uni_in || (L.fi && !L.mode3d)) && !s->pstd;
+    const double mean = ramps ? 0.0 : std::accumulate(pos.begin(), pos.end(), 0.0) / len[d];
+    if (ramps && (axis[d] || columns)) t.axes |= 1 << d;
+    for (int i = 0; i < len[d]; ++i) {
+      perm.push_back(off + (axis[d] ? f[i] : i));
+      efreq.push_back((float)-(freq[i] + mean));
+      epos.push_back((float)-pos[i]);
+    }
   }
-  const size_t wb = 2 * s->nw * sizeof(Wig), twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
+  const size_t wb = s->nw * sizeof(Wig), twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
+  const size_t rb = 2 * pb * s->nw;  // the ramps
   char* buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, wb + twb + pb * (1 + s->nw));
+  cudaError_t e = cudaMalloc(&buf, wb + twb + rb + pb * (3 + s->nw));
   if (e != cudaSuccess) return e;
   t.wigs = reinterpret_cast<Wig*>(buf);
   float2* const d_tw = reinterpret_cast<float2*>(buf + wb);
-  t.perm = reinterpret_cast<int*>(buf + wb + twb);
-  t.p = reinterpret_cast<float*>(buf + wb + twb + pb);
+  t.ramp = reinterpret_cast<float2*>(buf + wb + twb);
+  t.perm = reinterpret_cast<int*>(buf + wb + twb + rb);
+  t.efreq = reinterpret_cast<float*>(buf + wb + twb + rb + pb);
+  t.epos = reinterpret_cast<float*>(buf + wb + twb + rb + 2 * pb);
+  t.p = reinterpret_cast<float*>(buf + wb + twb + rb + 3 * pb);
   for (int q = 0; q < 3; ++q) plans[q]->tw = d_tw + at[q];
   t.uwig = s->wig;
   for (int w = 0; w < s->nw; ++w) {
@@ -1022,12 +1166,16 @@ static cudaError_t make_tables(Solver* s, int k) {
     t.uwig[w].pxe = f;
     t.uwig[w].pye = f + g.nx;
     t.uwig[w].pze = f + g.nx + g.ny;
+    const float2* c = t.ramp + perm.size() * w;
+    t.uwig[w].gx = c;
+    t.uwig[w].gy = c + g.nx;
+    t.uwig[w].gz = c + g.nx + g.ny;
   }
-  std::vector<Wig> wigs(s->wig);
-  wigs.insert(wigs.end(), t.uwig.begin(), t.uwig.end());
-  e = cudaMemcpyAsync(t.wigs, wigs.data(), wb, cudaMemcpyHostToDevice, s->stream);
+  e = cudaMemcpyAsync(t.wigs, t.uwig.data(), wb, cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_tw, tw.data(), twb, cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(t.perm, perm.data(), pb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(t.efreq, efreq.data(), pb, cudaMemcpyHostToDevice, s->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(t.epos, epos.data(), pb, cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // the host tables end here
   return e;
 }
@@ -1248,12 +1396,17 @@ static double* partials_of(const Solver* s, int i) {
   return s->d_partials + (long long)(i % s->nw) * s->lay.grid_inner * s->nrhs;
 }
 
+// the ramps of the inner passes: those that take the gains out, if pencils of ws_uni.cuh follow
+static const Wig& ramps_of(const Solver* s, int w) {
+  return s->lay.uni_out ? s->ut[s->active].uwig[w] : s->wig[w];
+}
+
 // iteration i of a cycle (wiggle i mod Nw)
 static InnerArgs inner_args(const Solver* s, int i) {
   const int w = i % s->nw;
   InnerArgs a{};
   a.g = s->g;
-  a.w = s->wig[w];
+  a.w = ramps_of(s, w);
   a.py = s->py;
   a.pxl = s->pxl;
   a.twx = s->twx;
@@ -1389,12 +1542,13 @@ static uni::ColArgs uni_col_args(const Solver* s, int w, int w1, const float2* i
   uni::ColArgs a{};
   a.g = s->g;
   a.py = p.plan;
-  a.it.gx = s->wig[w].gx;
-  a.it.gy = s->wig[w].gy;
-  a.it.gz = s->wig[w].gz;
-  a.it.gx1 = s->wig[w1].gx;
-  a.it.gy1 = s->wig[w1].gy;
-  a.it.gz1 = s->wig[w1].gz;
+  const std::vector<Wig>& wig = s->ut[s->active].uwig;
+  a.it.gx = wig[w].gx;
+  a.it.gy = wig[w].gy;
+  a.it.gz = wig[w].gz;
+  a.it.gx1 = wig[w1].gx;
+  a.it.gy1 = wig[w1].gy;
+  a.it.gz1 = wig[w1].gz;
   a.dE_in = in;
   a.it.src = src;
   a.A = make_float2(0.f, a_mult * (float)(1.0f / s->eps / (float)s->nw));  // 1i/epsilon/Nwiggles
@@ -1417,7 +1571,7 @@ static uni::ColArgs uni_col_args(const Solver* s, int w, int w1, const float2* i
 static cudaError_t launch_uni_col(const Solver* s, int mode, int w, int w1, const float2* in, const float2* src,
                                   float2* T, float a_mult) {
   uni::ColArgs a = uni_col_args(s, w, w1, in, src, T, a_mult);
-  return launch_uni(s, uni_kernels(a.py.cls).col[mode], s->lay.ucol, &a);
+  return launch_uni(s, uni_kernels(a.py.cls).col[s->lay.mode3d][mode], s->lay.ucol, &a);
 }
 
 static uni::XArgs uni_x_args(const Solver* s, float2* T) {
@@ -1450,6 +1604,10 @@ static uni::PencilArgs uni_pencil_args(const Solver* s, int w) {
   const double kk = (double)s->k02e.x * s->k02e.x + (double)s->k02e.y * s->k02e.y;
   if (kk > 0) a.ik02e = make_float2((float)(s->k02e.x / kk), (float)(-s->k02e.y / kk));
   a.norm = (float)(1.0 / ((double)s->g.npts));
+  a.norm_e = (float)(1.0 / ((double)s->g.npts * a.norm) - 1.0);
+  a.ex = s->ut[s->active].efreq;
+  a.ey = a.ex + s->g.nx;
+  a.ez = a.ey + s->g.ny;
   a.T = s->d_T;
   a.st = s->d_state;
   a.pitch = s->lay.pitch;
@@ -1649,7 +1807,7 @@ static cudaError_t launch_k3k1(const Solver* s, int w, int w1, bool src_next) {
   }
   InnerArgs a = inner_args(s, w);
   a.ncols = s->lay.ncols;
-  Wig W1 = s->wig[w1];
+  Wig W1 = ramps_of(s, w1);
   const float2* src1 = src_next ? s->d_src : nullptr;
   float2 A = make_float2(0.f, (float)(1.0f / s->eps / (float)s->nw));
   float2* T = s->d_T;
@@ -1731,7 +1889,7 @@ static cudaError_t launch_xpencil(const Solver* cs, bool inv) {
 static cudaError_t launch_colstep(const Solver* s, int w, int w1, bool src_next) {
   InnerArgs a = inner_args(s, w);
   a.ncols = s->lay.ncols;
-  Wig W1 = s->wig[w1];
+  Wig W1 = ramps_of(s, w1);
   const float2* src1 = src_next ? s->d_src : nullptr;
   float2 A = make_float2(0.f, (float)(1.0f / s->eps / (float)s->nw));
   float2* T = s->d_T;
@@ -1832,7 +1990,6 @@ static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist
   a.col = uni_col_args(s, 0, 0, nullptr, nullptr, s->d_T, 1.f);
   a.pen = uni_pencil_args(s, 0);
   a.wig = s->ut[1].wigs;
-  a.uwig = s->ut[1].wigs + s->nw;
   a.src = s->d_src;
   a.partials = s->d_partials;
   a.st = s->d_state;

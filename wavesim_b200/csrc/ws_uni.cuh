@@ -25,6 +25,18 @@
 //   are the same butterfly on the same elements and stay in registers.  A
 //   two-stage line crosses shared memory twice in the whole pass.
 //
+// The constants of the butterflies and the twiddles are rounded, so that a
+// forward and an inverse transform in a row multiply by N (1 + g) with |g| up
+// to a few 1e-8 per axis: the same in every iteration, which a solve of 200
+// iterations adds up to a few 1e-6.  g is known from the schedule, as a part by
+// position and one by frequency (uni_gains in ws_mbs.cu).  The first goes into
+// the rounding of the ramps (k_balance_ramps), the second into the Green's
+// function.  Converged fields (energies) against 64 bits on the same tables,
+// without and with it: 252 x 432 4.6e-6 (2.3e-6) and 7e-7 (8e-8), 81 x 360
+// 2.1e-6 (1.2e-6) and 8e-7 (1.3e-7), the latter half by the order of f_mix in
+// 2-D (col_body).  The times stay within 3% (batches between compile-time columns and
+// these pencils 2-6% longer).
+//
 // T has its y pitch rounded up to 4 elements (one 32-byte sector), so that
 // the pencils' rows start on sectors for odd Ny too.
 //
@@ -104,7 +116,8 @@ struct PencilArgs {
   Plan po;
   Wig w;  // p tables in the order of T
   float2 k02e, ik02e;  // k0^2 e + i e and its inverse
-  float norm;
+  float norm, norm_e;  // 1/N, and what the float lacks of it (relative)
+  const float *ex, *ey, *ez;  // the gains' inverses by frequency, in the order of T
   float2* T;
   const DevState* st;
   long long pitch, tstride, cstride;  // cstride: elements between the components of T
@@ -129,8 +142,7 @@ constexpr int kLoopThreads = 512;
 struct LoopArgs {
   ColArgs col;
   PencilArgs pen;
-  const Wig* wig;   // nw of them: natural order,
-  const Wig* uwig;  //   and with the p tables in the order of T
+  const Wig* wig;  // nw of them, the p tables in the order of T
   const float2* src;
   double* partials;  // slot i: bpr nrhs energies of iteration i of a cycle
   DevState* st;
@@ -179,7 +191,7 @@ enum { kFwd = 0, kInv = 1, kStep = 2, kPstd = 3 };
 constexpr int kClasses = 3;
 constexpr int kClassRadix[kClasses] = {8, 12, 16};
 struct Kernels {
-  const void* col[3];     // by kFwd, kInv, kStep
+  const void* col[2][3];  // 2-D, 3-D; by kFwd, kInv, kStep
   const void* x[2];       // forward, inverse
   const void* pencil[2];  // one component, three
   const void* loop;

@@ -105,7 +105,7 @@ __device__ __forceinline__ void col_middles(const ColArgs& a, float2* tile, cons
   }
 }
 
-template <int RM, int MODE>
+template <int RM, int MODE, bool D3>
 __device__ __forceinline__ void col_body(const ColArgs& a, const ColIter& it, const ColMem& m, int rhs, int bid) {
   const bool acc_now = MODE != kFwd && it.acc != kAccSkip;
   const Geom& g = a.g;
@@ -206,9 +206,21 @@ __device__ __forceinline__ void col_body(const ColArgs& a, const ColIter& it, co
                   const int k = h + r, y = j + k * S0.sub;
                   // Eprop after the conjugate ramps (WaveSim.m:55), f_mix (f_mix.m:3-4), E' += dE'
                   const float2 ep = cmul_conj(cmul_conj(v[k], g0), m.gy[y]);
-                  const float2 one_m = make_float2(1.f - kAlpha * gm[r].x, -kAlpha * gm[r].y);
-                  const float2 t = cmul(cmul(gm[r], gm[r]), ep);
-                  const float2 dn = cadd(cmul(one_m, d0[r]), make_float2(kAlpha * t.y, -kAlpha * t.x));
+                  float2 dn;
+                  if (D3) {
+                    // 1 - alpha gamma and gamma^2 first, as the compile-time kernels have it: of a medium of a few
+                    // values (spheres) their rounding is the same everywhere, and so the same at every size
+                    const float2 one_m = make_float2(1.f - kAlpha * gm[r].x, -kAlpha * gm[r].y);
+                    const float2 t = cmul(cmul(gm[r], gm[r]), ep);
+                    dn = cadd(cmul(one_m, d0[r]), make_float2(kAlpha * t.y, -kAlpha * t.x));
+                  } else {
+                    // dE - alpha gamma (dE + i gamma Eprop): nothing is rounded alike in every iteration (81 x 360,
+                    // 197 iterations: field 8e-7 from that of 64 bits on the same tables, energies 1.3e-7; as above
+                    // 1.5e-6 and 5e-7)
+                    const float2 u = cmul(gm[r], ep);
+                    const float2 t = cmul(gm[r], make_float2(d0[r].x - u.y, d0[r].y + u.x));
+                    dn = make_float2(fmaf(-kAlpha, t.x, d0[r].x), fmaf(-kAlpha, t.y, d0[r].y));
+                  }
                   dEc[k * S0.sub] = dn;
                   if (acc_now) Ec[k * S0.sub] = cadd(e0[r], it.acc == kAccPair ? cadd(d0[r], dn) : dn);
                   if (I.in && y >= g.r0[0] && y < g.r1[0]) esum = fmaf(dn.x, dn.x, fmaf(dn.y, dn.y, esum));
@@ -272,7 +284,7 @@ __device__ __forceinline__ void col_body(const ColArgs& a, const ColIter& it, co
   }
 }
 
-template <int RM, int MODE>
+template <int RM, int MODE, bool D3>
 __global__ void __launch_bounds__(kMaxThreads, (MODE == kFwd ? kBlocks<RM> : kBlocksHeavy<RM>)) k_col(
     const __grid_constant__ ColArgs a) {
   const int rhs = blockIdx.x / a.bpr, bid = blockIdx.x - rhs * a.bpr;
@@ -307,7 +319,7 @@ __global__ void __launch_bounds__(kMaxThreads, (MODE == kFwd ? kBlocks<RM> : kBl
     I.in = x >= g.r0[1] && x < g.r1[1] && z >= g.r0[2] && z < g.r1[2] && c >= g.r0[3] && c < g.r1[3];
     info[l] = I;
   }
-  col_body<RM, MODE>(a, a.it, ColMem{tile, a.py.tw, gy, gy1, gxz, gxz + a.lines, info, red, a.gamma, a.dE + f0, a.E + f0}, rhs, bid);
+  col_body<RM, MODE, D3>(a, a.it, ColMem{tile, a.py.tw, gy, gy1, gxz, gxz + a.lines, info, red, a.gamma, a.dE + f0, a.E + f0}, rhs, bid);
 }
 
 // Pencils --------------------------------------------------------------------
@@ -368,10 +380,32 @@ __device__ __forceinline__ void rows_out(const Stage& S, const float2* tw, const
   });
 }
 
-// K2: forward transform along the outer dimension, Green's function, inverse
-template <int RM, int NC>
+// a + b and what its rounding leaves
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+  const float s = a + b, t = s - a;
+  return make_float2(s, (a - (s - t)) + (b - t));
+}
+
+// norm (1 + e) / (dr + i di), for an e below the rounding of norm itself: as a
+// float, norm / (dr^2 + di^2) would lose e (always, where norm is a power of
+// two), so it is carried in two floats into the products with dr and di,
+// whose roundings e then shifts on average.  (81 x 360 with the gains by
+// position alone: 5e-7 more on the energies.)
+__device__ __forceinline__ float2 green(float dr, float di, float norm, float e) {
+  const float d = fmaf(dr, dr, di * di);
+  const float r = __frcp_rn(d);
+  const float inv = norm * r;
+  const float lo = fmaf(inv, fmaf(-r, fminf(d, 3e38f), 1.f) + e, fmaf(norm, r, -inv));
+  return make_float2(fmaf(dr, inv, dr * lo), fmaf(-di, inv, -di * lo));
+}
+
+// K2: forward transform along the outer dimension, Green's function, inverse.
+// po, eo: p and (of the first n / RL elements) the gain's inverse along the outer dimension.
+// PSTD: the Laplacian instead (kEither: as a.pstd says)
+enum { kGreen = 0, kLaplacian = 1, kEither = 2 };
+template <int RM, int NC, int PSTD>
 __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, int rhs, int bid, float2* tile, const float2* tw,
-                                            const float* po) {
+                                            const float* po, const float* eo) {
   const Geom& g = a.g;
   const int ty = 1 << a.lty, yl = threadIdx.x & (ty - 1), w = threadIdx.x >> a.lty, W = blockDim.x >> a.lty;
   const int mid = bid / a.nyt, y = (bid - mid * a.nyt) * ty + yl;
@@ -381,19 +415,24 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
   const int n = a.po.n, tn = n * ty;
   const float py = live ? __ldg(&wg.pye[y]) : 0.f;
   const float pm = a.mode3d ? __ldg(&wg.pxe[mid]) : __ldg(&wg.pze[0]);
+  const float e2 = a.norm_e + (live ? __ldg(&a.ey[y]) : 0.f) + (a.mode3d ? __ldg(&a.ex[mid]) : 0.f);
 #pragma unroll
   for (int c = 0; c < NC; ++c) rows_in<RM>(a.po.st[0], tw, base + c * a.cstride, step, tile + c * tn, ty, yl, w, W, live);
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < NC; ++c) row_middles<RM, false>(a.po, tile + c * tn, tw, ty, yl, w, W);
   const Stage& SL = a.po.st[a.po.nst - 1];
-  // |p|^2 - Re k02e with the difference taken first: near resonance only the small part is rounded
-  const float base2 = fmaf(py, py, fmaf(pm, pm, -a.k02e.x));
+  // |p|^2 - Re k02e: near resonance the difference of two numbers 10 times its size, so
+  // what does not depend on the pencil's own p is kept in two floats
+  const float py2 = py * py, pm2 = pm * pm;
+  const float2 s1 = two_sum(pm2, -a.k02e.x), s2 = two_sum(s1.x, py2);
+  const float base2 = s2.x, low2 = (s1.y + s2.y) + (fmaf(pm, pm, -pm2) + fmaf(py, py, -py2));
   const float di = -a.k02e.y;
   with_radix<RM>(SL.R, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
     for (int u = w; u < SL.units; u += W) {
       float2* p = tile + u * R * ty + yl;
+      const float eu = e2 + eo[u];
       if constexpr (NC == 1) {
         float2 v[R];
 #pragma unroll
@@ -404,12 +443,13 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
 #pragma unroll
         for (int i = 0; i < R; ++i) {
           const float q = po[u + i * SL.units];
-          const float dr = fmaf(q, q, base2);
-          if (a.pstd) {
-            v[i] = make_float2(-dr * a.norm * v[i].x, -dr * a.norm * v[i].y);
+          const float dr = fmaf(q, q, base2) + low2;
+          const float e = eu - (float)round_trip(0, R, i);
+          if (PSTD == kLaplacian || (PSTD == kEither && a.pstd)) {
+            const float s = -dr * a.norm, lo = fmaf(s, e, fmaf(-dr, a.norm, -s));
+            v[i] = make_float2(fmaf(s, v[i].x, lo * v[i].x), fmaf(s, v[i].y, lo * v[i].y));
           } else {
-            const float inv = a.norm * __frcp_rn(fmaf(dr, dr, di * di));
-            v[i] = cmul(v[i], make_float2(dr * inv, -di * inv));
+            v[i] = cmul(v[i], green(dr, di, a.norm, e));
           }
         }
         Dft<R, true>::run(v);
@@ -441,12 +481,11 @@ __device__ __forceinline__ void pencil_body(const PencilArgs& a, const Wig& wg, 
 #pragma unroll
           for (int i = 0; i < R; ++i) {
             const float q = po[u + i * SL.units];
-            const float dr = fmaf(q, q, base2);
-            const float inv = a.norm * __frcp_rn(fmaf(dr, dr, di * di));
+            const float dr = fmaf(q, q, base2) + low2;
             const float pc = c == 1 ? py : ((c == 0) == (a.mode3d != 0) ? pm : q);
-            const float2 e = p[c * tn + i * ty];
-            v[i] = cmul(make_float2(fmaf(-pc, pe[i].x, e.x), fmaf(-pc, pe[i].y, e.y)),
-                        make_float2(dr * inv, -di * inv));
+            const float2 f = p[c * tn + i * ty];
+            v[i] = cmul(make_float2(fmaf(-pc, pe[i].x, f.x), fmaf(-pc, pe[i].y, f.y)),
+                        green(dr, di, a.norm, eu - (float)round_trip(0, R, i)));
           }
           Dft<R, true>::run(v);
 #pragma unroll
@@ -470,8 +509,10 @@ __global__ void __launch_bounds__(kMaxThreads, (NC == 1 ? kBlocks<RM> : kBlocksH
   if (load_done(a.st + rhs)) return;
   extern __shared__ float2 tile[];
   float* const po = reinterpret_cast<float*>(tile + NC * (a.po.n << a.lty));
+  float* const eo = po + a.po.n;
   copy_table(po, a.mode3d ? a.w.pze : a.w.pxe, a.po.n);
-  pencil_body<RM, NC>(a, a.w, rhs, bid, tile, a.po.tw, po);
+  copy_table(eo, a.mode3d ? a.ez : a.ex, a.po.st[a.po.nst - 1].units);
+  pencil_body<RM, NC, NC == 1 ? kEither : kGreen>(a, a.w, rhs, bid, tile, a.po.tw, po, eo);
 }
 
 // The x transforms of a 3-D grid, in place on T
@@ -592,7 +633,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
   float2* const Es = dE + lines * g.ny;
   ColLine* const info = reinterpret_cast<ColLine*>(Es + (a.e_resident ? lines * g.ny : 0));
   float* const red = reinterpret_cast<float*>(info + lines);
-  float* const po = red + a.groups;  // nw p tables of the outer dimension
+  float* const eo = red + a.groups;  // the gain's inverse and nw p tables of the outer dimension
+  const int neo = a.pen.po.st[a.pen.po.nst - 1].units;
+  float* const po = eo + neo;
   const bool own = blockIdx.x < columns;  // the block's column tile
   const int crhs = own ? blockIdx.x / a.col.bpr : 0, cbid = blockIdx.x - crhs * a.col.bpr;
   const int col0 = cbid * lines, nl = own ? min(lines, a.col.total - col0) : 0;
@@ -600,9 +643,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
   float2* const E = a.e_resident ? Es : a.col.E + f0;
   copy_table(tw_col, a.col.py.tw, a.col.py.ntw);
   copy_table(tw_out, a.pen.po.tw, a.pen.po.ntw);
+  copy_table(eo, a.pen.ex, neo);
   for (int i = 0; i < nw; ++i) {
     copy_table(gy + i * g.ny, a.wig[i].gy, g.ny);
-    copy_table(po + i * a.pen.po.n, a.uwig[i].pxe, a.pen.po.n);
+    copy_table(po + i * a.pen.po.n, a.wig[i].pxe, a.pen.po.n);
   }
   for (int l = tid; l < nl; l += nthr) {
     const int x = col0 + l;
@@ -630,7 +674,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
       for (int t = blockIdx.x; t < pencils; t += gridDim.x) {
         const int rhs = a.nrhs > 1 ? t / a.pen.bpr : 0;
         if (!st[rhs].done)
-          pencil_body<RM, 1>(a.pen, a.uwig[i], rhs, t - rhs * a.pen.bpr, tile, tw_out, po + i * a.pen.po.n);
+          pencil_body<RM, 1, kGreen>(a.pen, a.wig[i], rhs, t - rhs * a.pen.bpr, tile, tw_out, po + i * a.pen.po.n, eo);
         __syncthreads();
       }
       if (!grid_barrier(a.arrived, target, a.err)) return;
@@ -639,7 +683,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
         it.src = first && i1 > 0 ? a.src : nullptr;
         it.partials = a.partials + (long long)i * columns;
         it.acc = nw % 2 ? kAccEach : (i % 2 ? kAccPair : kAccSkip);
-        col_body<RM, kStep>(a.col, it,
+        col_body<RM, kStep, false>(a.col, it,
                             ColMem{tile, tw_col, gy + i * g.ny, gy + i1 * g.ny, gxz + i * lines, gxz + i1 * lines, info,
                                    red, gamma, dE, E},
                             crhs, cbid);
@@ -694,13 +738,16 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
   ColLine* const info = reinterpret_cast<ColLine*>(S + elems);
   float* const red = reinterpret_cast<float*>(info + lines);
   float* const po = red + a.groups;
-  float* const c3 = po + a.pen.po.n;
+  float* const eo = po + a.pen.po.n;
+  const int neo = a.pen.po.st[a.pen.po.nst - 1].units;
+  float* const c3 = eo + neo;
   const bool own = blockIdx.x < a.col.bpr;
   const int col0 = blockIdx.x * lines, nl = own ? min(lines, a.col.total - col0) : 0;
   const long long f0 = (long long)col0 * g.ny;
   copy_table(tw_col, a.col.py.tw, a.col.py.ntw);
   copy_table(tw_out, a.pen.po.tw, a.pen.po.ntw);
   copy_table(po, a.pen.w.pxe, a.pen.po.n);
+  copy_table(eo, a.pen.ex, neo);
   for (int l = tid; l < nl; l += nthr) {
     const int x = col0 + l;
     info[l] = ColLine{(long long)l * g.ny, x >= g.r0[1] && x < g.r1[1] && g.r0[2] == 0};
@@ -717,7 +764,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
   for (int k = 0; k < a.steps && !st.done; ++k) {
     const PstdStepAmp amp = a.amp[k];
     for (int t = blockIdx.x; t < a.pen.bpr; t += gridDim.x) {
-      pencil_body<RM, 1>(a.pen, a.pen.w, 0, t, tile, tw_out, po);
+      pencil_body<RM, 1, kLaplacian>(a.pen, a.pen.w, 0, t, tile, tw_out, po, eo);
       __syncthreads();
     }
     if (!grid_barrier(a.arrived, target, a.err)) return;
@@ -730,7 +777,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
       m.S = S;
       m.A = amp.A;
       m.ps = amp.ps;
-      col_body<RM, kPstd>(a.col, it, m, 0, blockIdx.x);
+      col_body<RM, kPstd, false>(a.col, it, m, 0, blockIdx.x);
     }
     if (!grid_barrier(a.arrived, target, a.err)) return;
     // Simulation.next (Simulation.m:193-217) for PSTD.run_algorithm (PSTD.m:108-124), the same in every block
@@ -764,7 +811,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
 
 template <int RM>
 Kernels kernels_up_to() {
-  return Kernels{{(const void*)k_col<RM, kFwd>, (const void*)k_col<RM, kInv>, (const void*)k_col<RM, kStep>},
+  const void* const fwd = (const void*)k_col<RM, kFwd, true>;  // the same for both
+  return Kernels{{{fwd, (const void*)k_col<RM, kInv, false>, (const void*)k_col<RM, kStep, false>},
+                  {fwd, (const void*)k_col<RM, kInv, true>, (const void*)k_col<RM, kStep, true>}},
                  {(const void*)k_x<RM, false>, (const void*)k_x<RM, true>},
                  {(const void*)k_pencil<RM, 1>, (const void*)k_pencil<RM, 3>},
                  (const void*)k_loop<RM>, (const void*)k_pstd_loop<RM>};
