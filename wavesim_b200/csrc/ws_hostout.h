@@ -88,14 +88,28 @@ inline HostPool& host_pool() {
   return *pool;
 }
 
-// A buffer of the pool for the length of a scope.
+// A buffer of the pool for the length of a scope, and until the device is done
+// with it: a scope may be left with copies into it still queued (an error
+// return), and the pool's next taker must not get them.
 struct HostLease {
   void* p = nullptr;
   size_t bytes = 0;
   explicit HostLease(size_t n) { p = host_pool().get(n, &bytes); }
   HostLease(const HostLease&) = delete;
   HostLease& operator=(const HostLease&) = delete;
-  ~HostLease() { host_pool().put(p, bytes); }
+  ~HostLease() {
+    // (after an error the device may still hold it: then it is not used again)
+    if (!busy_ || cudaStreamSynchronize(stream_) == cudaSuccess) host_pool().put(p, bytes);
+  }
+  void queued(cudaStream_t stream) {  // copies on `stream` may write to it
+    stream_ = stream;
+    busy_ = true;
+  }
+  void settled() { busy_ = false; }  // the caller has waited for them
+
+ private:
+  cudaStream_t stream_ = nullptr;
+  bool busy_ = false;
 };
 
 class OutCopy {
@@ -125,10 +139,13 @@ class OutCopy {
   cudaError_t stage(const void* src, cudaStream_t stream) {
     src_ = (const char*)src;
     stream_ = stream;
-    return whole_ ? cudaMemcpyAsync(slots_.p, src, bytes_, cudaMemcpyDeviceToHost, stream) : cudaSuccess;
+    if (!whole_) return cudaSuccess;
+    slots_.queued(stream);
+    return cudaMemcpyAsync(slots_.p, src, bytes_, cudaMemcpyDeviceToHost, stream);
   }
   // The staged result into the destination; returns when it is there.
   cudaError_t run() {
+    slots_.settled();
     {
       std::lock_guard<std::mutex> lock(mu_);
       go_ = 1;
@@ -194,6 +211,7 @@ class OutCopy {
     if (e != cudaSuccess) {
       std::lock_guard<std::mutex> lock(mu_);
       err_ = (int)e;
+      slots_.queued(stream_);  // a chunk may still be under way
     }
   }
 

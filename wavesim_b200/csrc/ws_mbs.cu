@@ -2327,11 +2327,17 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   const double* const hhead = (const double*)((char*)back.p + state_bytes + 16);
   const long long nhead = std::min<long long>((long long)kHead, s->hist_cap);
   auto fetch_state = [&]() -> cudaError_t {
+    back.queued(s->stream);
     cudaError_t e = cudaMemcpyAsync((void*)hs, s->d_state, nrhs * sizeof(DevState), cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync((void*)kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream);
     for (int r = 0; head && r < nrhs && e == cudaSuccess; ++r)
       e = cudaMemcpyAsync((void*)(hhead + r * kHead), s->d_hist + r * hs_stride, nhead * sizeof(double),
                           cudaMemcpyDeviceToHost, s->stream);
+    return e;
+  };
+  auto wait = [&]() -> cudaError_t {
+    const cudaError_t e = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) back.settled();
     return e;
   };
   auto all_done = [&]() {
@@ -2398,7 +2404,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
       if (E_out) WS_CUDA(finalize(0, to_host ? group : nrhs));
       WS_CUDA(fetch_state());
       WS_CUDA(begin_copy());
-      WS_CUDA(cudaStreamSynchronize(s->stream));
+      WS_CUDA(wait());
       if (all_done() || *kerr) break;
     }
   } else if (opt.use_graph && !want_cb) {
@@ -2413,7 +2419,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     if (E_out) WS_CUDA(finalize(0, to_host ? group : nrhs));
     WS_CUDA(fetch_state());
     WS_CUDA(begin_copy());
-    WS_CUDA(cudaStreamSynchronize(s->stream));
+    WS_CUDA(wait());
   } else {
     std::vector<double> hist;
     const long long cb_int = std::max<int64_t>(1, opt.callback_interval);
@@ -2431,7 +2437,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
         }
       }
       WS_CUDA(fetch_state());
-      WS_CUDA(cudaStreamSynchronize(s->stream));
+      WS_CUDA(wait());
       if (want_cb) {
         const long long done_it = hs[0].it - 1;
         hist.resize(done_it);
