@@ -13,6 +13,8 @@ CUDA_INC = "/usr/local/cuda/include"
 
 FAKE = r"""
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -24,6 +26,13 @@ static std::vector<Copy> queue;      // of the one stream
 static std::recursive_mutex queue_mu;
 static int host_allocs_left = 1 << 30, event_records_left = 1 << 30;
 static int live = 0;                 // page-locked buffers
+static std::atomic<int> news_left{1 << 30};
+void* operator new(size_t n) {
+  if (news_left-- <= 0) throw std::bad_alloc();
+  return std::malloc(n);
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, size_t) noexcept { std::free(p); }
 static void drain() {
   std::lock_guard<std::recursive_mutex> l(queue_mu);
   for (const Copy& c : queue) std::memcpy(c.dst, c.src, c.n);
@@ -91,6 +100,35 @@ BODIES = {
   size_t got = 0;
   void* p = ws::host_pool().get(1, &got);
   CHECK(p && !queued_into(p, got));
+  return 0;""",
+    # no memory at any one of the allocations that staging a result makes: it arrives, or the call throws, but the
+    # process goes on
+    "no_memory": r"""
+  std::vector<char> src(70 << 20, 7), dst(src.size(), 1);
+  for (int k = 0; k < 40; ++k) {
+    std::fill(dst.begin(), dst.end(), 1);
+    news_left = k;
+    bool arrived = false;
+    try {
+      ws::OutCopy c(dst.data(), dst.size(), 0);
+      news_left = 1 << 30;
+      c.touch();
+      CHECK(c.stage(src.data(), nullptr) == cudaSuccess);
+      arrived = c.run() == cudaSuccess;
+    } catch (const std::bad_alloc&) {
+    }
+    news_left = 1 << 30;
+    CHECK(!arrived || dst == src);
+    // as the pool takes its buffers back
+    void* p[3];
+    size_t got[3];
+    for (int i = 0; i < 3; ++i) p[i] = ws::host_pool().get(4096, &got[i]);
+    news_left = k % 4;
+    for (int i = 0; i < 3; ++i) ws::host_pool().put(p[i], got[i]);
+    news_left = 1 << 30;
+    ws::host_pool().trim();
+    CHECK(live == 0);
+  }
   return 0;""",
     # and the ordinary way, whole and in chunks
     "results_arrive": r"""

@@ -18,8 +18,8 @@
 #include <condition_variable>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -58,11 +58,12 @@ class HostPool {
     if (!p) return;
     {
       std::lock_guard<std::mutex> lock(mu_);
-      if (idle_ + bytes <= kKeep) {
-        free_.push_back(Buf{p, bytes});
-        idle_ += bytes;
-        return;
-      }
+      if (idle_ + bytes <= kKeep) try {
+          free_.push_back(Buf{p, bytes});
+          idle_ += bytes;
+          return;
+        } catch (const std::exception&) {  // no memory to remember it by: given back below
+        }
     }
     cudaFreeHost(p);
   }
@@ -120,12 +121,10 @@ class OutCopy {
         chunk_(whole_ ? std::max<size_t>(bytes, 1) : std::min(kChunk, (bytes / 4 + 4095) / 4096 * 4096)),
         workers_(workers_of(bytes, chunk_)), slots_(workers_ * chunk_) {
     if (!slots_.p) return;
-    for (int w = 1; w < workers_; ++w) {
-      try {
-        threads_.emplace_back([this, w] { work(w); });
-      } catch (const std::system_error&) {
-        break;  // the caller's thread takes the chunks of the missing ones
-      }
+    try {
+      threads_.reserve(workers_);  // nothing below may throw once a thread runs
+      for (int w = 1; w < workers_; ++w) threads_.emplace_back([this, w] { work(w); });
+    } catch (const std::exception&) {  // no threads or no memory: the caller takes the chunks of the missing ones
     }
   }
   ~OutCopy() { finish(-1); }
