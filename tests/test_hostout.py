@@ -101,6 +101,22 @@ BODIES = {
   void* p = ws::host_pool().get(1, &got);
   CHECK(p && !queued_into(p, got));
   return 0;""",
+    # no page-locked memory at all: through ordinary memory
+    "no_page_locked_memory": r"""
+  host_allocs_left = 0;
+  for (size_t n : {(size_t)4097, (size_t)(9 << 20) + 13}) {
+    std::vector<char> src(n, 7), dst(n, 1);
+    ws::HostLease state(100);
+    CHECK(state.p);
+    ws::OutCopy c(dst.data(), n, 0);
+    CHECK(c.ok());
+    c.touch();
+    CHECK(c.stage(src.data(), nullptr) == cudaSuccess);
+    cudaStreamSynchronize(nullptr);
+    CHECK(c.run() == cudaSuccess);
+    CHECK(dst == src);
+  }
+  return 0;""",
     # no memory at any one of the allocations that staging a result makes: it arrives, or the call throws, but the
     # process goes on
     "no_memory": r"""

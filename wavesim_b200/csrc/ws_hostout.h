@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <condition_variable>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <exception>
 #include <mutex>
@@ -89,18 +90,27 @@ inline HostPool& host_pool() {
   return *pool;
 }
 
-// A buffer of the pool for the length of a scope, and until the device is done
-// with it: a scope may be left with copies into it still queued (an error
+// A buffer of the pool for the length of a scope (where no page-locked memory is
+// to be had, ordinary memory: slower copies), and until the device is done with
+// it: a scope may be left with copies into it still queued (an error
 // return), and the pool's next taker must not get them.
 struct HostLease {
   void* p = nullptr;
   size_t bytes = 0;
-  explicit HostLease(size_t n) { p = host_pool().get(n, &bytes); }
+  explicit HostLease(size_t n) {
+    p = host_pool().get(n, &bytes);
+    pooled_ = p != nullptr;
+    if (!pooled_) p = std::malloc(n);
+  }
   HostLease(const HostLease&) = delete;
   HostLease& operator=(const HostLease&) = delete;
   ~HostLease() {
     // (after an error the device may still hold it: then it is not used again)
-    if (!busy_ || cudaStreamSynchronize(stream_) == cudaSuccess) host_pool().put(p, bytes);
+    if (busy_ && cudaStreamSynchronize(stream_) != cudaSuccess) return;
+    if (pooled_)
+      host_pool().put(p, bytes);
+    else
+      std::free(p);
   }
   void queued(cudaStream_t stream) {  // copies on `stream` may write to it
     stream_ = stream;
@@ -110,7 +120,7 @@ struct HostLease {
 
  private:
   cudaStream_t stream_ = nullptr;
-  bool busy_ = false;
+  bool busy_ = false, pooled_ = false;
 };
 
 class OutCopy {

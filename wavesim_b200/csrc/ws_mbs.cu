@@ -2321,7 +2321,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   const bool head = diff_out && nrhs <= 16;
   const size_t state_bytes = (nrhs * sizeof(DevState) + 15) / 16 * 16;
   HostLease back(state_bytes + 16 + (head ? nrhs * kHead * sizeof(double) : 0));
-  if (!back.p) return fail(WS_ERR_OUT_OF_MEMORY, "no page-locked memory for the loop's state");
+  if (!back.p) return fail(WS_ERR_OUT_OF_MEMORY, "no memory for the loop's state");
   const DevState* const hs = (const DevState*)back.p;
   const int* const kerr = (const int*)((char*)back.p + state_bytes);
   const double* const hhead = (const double*)((char*)back.p + state_bytes + 16);
@@ -2382,7 +2382,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   auto begin_copy = [&]() -> cudaError_t {
     if (!pageable) return cudaSuccess;
     if (!copy) copy.reset(new OutCopy(E_out, per * group, s->device));
-    if (!copy->ok()) return cudaErrorMemoryAllocation;
+    if (!copy->ok()) return cudaErrorMemoryAllocation;  // no host memory at all
     const cudaError_t e = copy->stage(field ? (const void*)s->d_out : (const void*)s->d_E, s->stream);
     copy->touch();
     return e;
@@ -2477,7 +2477,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
       if (pageable) {
         if (r0 > 0 || !copy) {
           copy.reset(new OutCopy(dst, per * (r1 - r0), s->device));
-          if (!copy->ok()) return fail(WS_ERR_OUT_OF_MEMORY, "no page-locked memory for the fields");
+          if (!copy->ok()) return fail(WS_ERR_OUT_OF_MEMORY, "no memory for the fields");
           WS_CUDA(copy->stage(from, s->stream));
           WS_CUDA(cudaStreamSynchronize(s->stream));
         }
