@@ -782,9 +782,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
     if (!grid_barrier(a.arrived, target, a.err)) return;
     // Simulation.next (Simulation.m:193-217) for PSTD.run_algorithm (PSTD.m:108-124), the same in every block
     if (tid < 32) {
-      const double e = st.calc_energy ? sum_partials(a.partials, a.col.bpr) : 0.0;
+      const int calc = st.calc_energy;
+      __syncwarp();  // lane 0 changes it below, and without an energy nothing else holds it back
+      const double e = calc ? sum_partials(a.partials, a.col.bpr) : 0.0;
       if (tid == 0) {
-        if (st.calc_energy) st.last_step_energy = e / amp.A2;
+        if (calc) st.last_step_energy = e / amp.A2;
         const double d = st.last_step_energy;
         const int it = st.it;
         if (blockIdx.x == 0 && it - 1 < a.hist_cap) a.hist[it - 1] = d;
