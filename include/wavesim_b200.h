@@ -250,11 +250,12 @@ int ws_solver_buffers(ws_solver s, void** E_prime, void** stream);
  * iterations only, and every stop of the loop falls after an even one). */
 int ws_solver_time_kernels(ws_solver s, int n_iterations, float ms_out[3], double bytes_out[3]);
 
-/* Bound of the waits of the TMA-pipelined outer pass (K2 of 3-D grids): a
- * block whose tile load has not arrived after `clocks` SM clocks gives up,
- * waits for its copies still in flight (with the default bound), and the
- * solve returns WS_ERR_CUDA ("timed out") instead of hanging.  0 restores the
- * default (5e7 clocks, ~25 ms).  A very small bound makes the waits run out
+/* Bound of the waits of the TMA-pipelined outer pass (K2 of 3-D grids, batches of
+ * 2-D ones) and of the barrier of the loop in one launch (small 2-D grids): a
+ * block whose tile load has not arrived, or that has not met all other blocks,
+ * after `clocks` SM clocks gives up, waits for its copies still in flight (with
+ * the default bound), and the solve returns WS_ERR_CUDA ("timed out") instead
+ * of hanging.  0 restores the defaults (5e7 clocks, ~25 ms; the barrier 2e9, ~1 s).  A very small bound makes the waits run out
  * on purpose: the failure path can be tested without a GPU fault.  No
  * counterpart in the reference. */
 int ws_solver_set_wait_limit(ws_solver s, int64_t clocks);

@@ -854,7 +854,7 @@ struct Solver {
   int fuse = 0;                  // the loop runs K3 of each iteration fused with K1 of the next
   LayoutChoice tuned{};          // the autotuner's choice (all zero: the heuristics)
   double warm_ratio = 0.0;       // discard threshold of the current solve
-  long long wait_clocks = 0;     // bound of the TMA pencils' tile waits (0: the default)
+  long long wait_clocks = 0;     // bound of the TMA pencils' tile waits and the loop's barrier (0: the defaults)
   int pdl = 0;                   // WAVESIM_B200_PDL=1: launch the loop's kernels with programmatic
                                  // dependent launch (measured: 256^3 solve 46.3 against 44.3 ms,
                                  // 96^3 3.38 against 2.80 ms, 1024^2 8.50 against 8.71 ms; off)
@@ -1982,6 +1982,8 @@ static cudaError_t launch_coop(const Solver* s, const void* fn, size_t smem, int
   return cudaLaunchKernelExC(&cfg, fn, argv);
 }
 
+static long long barrier_limit(const Solver* s) { return s->wait_clocks > 0 ? s->wait_clocks : uni::kBarrierClocks; }
+
 // Cycles of the loop in one cooperative launch, from T as K1 left it, until
 // every right-hand side is done or max_cycles have run.
 static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist& h, long long max_cycles) {
@@ -1996,6 +1998,7 @@ static cudaError_t launch_loop(const Solver* s, const StopRule& rule, const Hist
   a.rule = rule;
   a.hist = h;
   a.err = s->d_err;
+  a.limit = barrier_limit(s);
   a.max_cycles = max_cycles;
   a.nw = s->nw;
   a.nrhs = s->nrhs;
@@ -2452,7 +2455,7 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
   }
   if (*kerr) {
     cudaMemset(s->d_err, 0, sizeof(int));
-    return fail(WS_ERR_CUDA, "a bounded wait of the FFT kernels (cluster exchange or TMA tile load) timed out");
+    return fail(WS_ERR_CUDA, "a bounded wait of the FFT kernels (cluster exchange, TMA tile load or the loop's barrier) timed out");
   }
   bool diverged = false;
   for (int r = 0; r < nrhs; ++r) {
@@ -3431,6 +3434,7 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
       a.max_iter = rule.max_iter;
       a.threshold = rule.threshold;
       a.err = s->d_err;
+      a.limit = barrier_limit(s);
       a.steps = (int)K;
       a.interval = rule.interval;
       a.groups = uni_groups(s->lay.ucol);

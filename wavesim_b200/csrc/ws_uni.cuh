@@ -139,6 +139,7 @@ struct XArgs {
 // at a barrier in global memory after each pass.
 constexpr int kLoopRhs = 16;  // right-hand sides that it takes
 constexpr int kLoopThreads = 512;
+constexpr long long kBarrierClocks = 2000000000LL;  // ~1 s: a bound, not a delay that ever occurs
 struct LoopArgs {
   ColArgs col;
   PencilArgs pen;
@@ -150,6 +151,7 @@ struct LoopArgs {
   Hist hist;
   unsigned* arrived;  // zero at launch
   int* err;
+  long long limit;    // clocks that a block waits for the others
   long long max_cycles;  // of this launch
   int tile_elems;        // shared memory: the passes' tile, in float2
   int groups;            // energies of 32 butterflies of a column tile
@@ -181,6 +183,7 @@ struct PstdLoopArgs {
   double threshold;
   unsigned* arrived;
   int* err;
+  long long limit;
   int steps, interval;
   int tile_elems, groups;
 };

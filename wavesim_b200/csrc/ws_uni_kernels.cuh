@@ -579,12 +579,11 @@ __global__ void __launch_bounds__(kMaxThreads, kBlocks<RM>) k_x(const __grid_con
 // 18.8, 12.6; 1100 x 768 38, 28.  With the fields left in global memory: 9.4,
 // 14.5, 14.6, 16.3, 34.  In 3-D (four barriers, more work per point) it lost:
 // 96^3 39 against 30, 63 x 77 x 70 x 3 58 against 49, so those stay launched.
-constexpr long long kBarrierClocks = 2000000000LL;  // ~1 s: a bound, not a delay that ever occurs
 
 // Barrier of all blocks of a cooperative launch; false (in every thread)
-// after kBarrierClocks, with *err set.  What a block wrote before it is
+// after `limit` clocks, with *err set.  What a block wrote before it is
 // visible to loads past L1 (__ldcg) of the others after it.
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, int* err) {
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target, int* err, long long limit) {
   __shared__ int ok;
   if (!arrived) {  // the grid is one cluster
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -601,7 +600,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned& target
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
       if ((int)(v - target) >= 0) break;
-      if (clock64() - t0 > kBarrierClocks) {
+      if (clock64() - t0 > limit) {
         atomicExch(err, 1);
         good = 0;
         break;
@@ -677,7 +676,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
           pencil_body<RM, 1, kGreen>(a.pen, a.wig[i], rhs, t - rhs * a.pen.bpr, tile, tw_out, po + i * a.pen.po.n, eo);
         __syncthreads();
       }
-      if (!grid_barrier(a.arrived, target, a.err)) return;
+      if (!grid_barrier(a.arrived, target, a.err, a.limit)) return;
       if (own && !st[crhs].done) {
         ColIter it{};
         it.src = first && i1 > 0 ? a.src : nullptr;
@@ -688,7 +687,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_loop(const __grid_constant_
                                    red, gamma, dE, E},
                             crhs, cbid);
       }
-      if (!grid_barrier(a.arrived, target, a.err)) return;
+      if (!grid_barrier(a.arrived, target, a.err, a.limit)) return;
     }
     // the stop rule of the cycle, the same in every block
     for (int r = 0; r < a.nrhs; ++r) {
@@ -767,7 +766,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
       pencil_body<RM, 1, kLaplacian>(a.pen, a.pen.w, 0, t, tile, tw_out, po, eo);
       __syncthreads();
     }
-    if (!grid_barrier(a.arrived, target, a.err)) return;
+    if (!grid_barrier(a.arrived, target, a.err, a.limit)) return;
     const int cur = (st.it - 1) & 1;
     if (own) {
       ColIter it{};
@@ -779,7 +778,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_pstd_loop(const __grid_cons
       m.ps = amp.ps;
       col_body<RM, kPstd, false>(a.col, it, m, 0, blockIdx.x);
     }
-    if (!grid_barrier(a.arrived, target, a.err)) return;
+    if (!grid_barrier(a.arrived, target, a.err, a.limit)) return;
     // Simulation.next (Simulation.m:193-217) for PSTD.run_algorithm (PSTD.m:108-124), the same in every block
     if (tid < 32) {
       const int calc = st.calc_energy;
