@@ -365,6 +365,9 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
                 const ws_pstd_options* opts, ws_complex* E_out, double* diff_energy_out, int64_t diff_capacity,
                 int64_t* n_iterations, int* converged);
 
+/* ws_solver_set_wait_limit for the solver's runs. */
+int ws_pstd_set_wait_limit(ws_pstd h, int64_t clocks);
+
 int ws_pstd_destroy(ws_pstd h);
 
 /*

@@ -73,7 +73,7 @@ EXPORTS = [
     "ws_solver_launches_per_iteration", "ws_solver_fused", "ws_solver_set_wait_limit", "ws_solver_time_fused", "ws_solver_warm_report", "ws_solver_warm_residual", "ws_solver_autotune", "ws_solver_get_layout", "ws_solver_set_layout", "ws_solver_destroy",
     "ws_run_algorithm_noalloc", "ws_medium_reduce", "ws_build_gamma", "ws_setup_last_error",
     "ws_noalloc_scratch_bytes", "ws_noalloc_last_error",
-    "ws_pstd_default_options", "ws_pstd_create", "ws_pstd_run", "ws_pstd_destroy",
+    "ws_pstd_default_options", "ws_pstd_create", "ws_pstd_run", "ws_pstd_set_wait_limit", "ws_pstd_destroy",
 ]
 
 
@@ -171,6 +171,8 @@ def _load():
     lib.ws_pstd_run.argtypes = [P, C.c_int64, C.POINTER(ws_source_block), C.c_int, C.POINTER(ws_pstd_options), P,
                                 C.POINTER(C.c_double), C.c_int64, i64p, C.POINTER(C.c_int)]
     lib.ws_pstd_run.restype = C.c_int
+    lib.ws_pstd_set_wait_limit.argtypes = [P, C.c_int64]
+    lib.ws_pstd_set_wait_limit.restype = C.c_int
     lib.ws_pstd_destroy.argtypes = [P]
     lib.ws_pstd_destroy.restype = C.c_int
     lib.ws_gemm_bf16.argtypes = [P, P, P, P, P, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,

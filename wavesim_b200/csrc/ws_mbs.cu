@@ -3468,7 +3468,10 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
   }
   int kerr = 0;
   WS_CUDA(cudaMemcpy(&kerr, s->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (kerr) return fail(WS_ERR_CUDA, "a kernel's bounded wait gave up (cluster exchange or TMA load)");
+  if (kerr) {
+    cudaMemset(s->d_err, 0, sizeof(int));
+    return fail(WS_ERR_CUDA, "a bounded wait of the kernels (cluster exchange, TMA tile load or the loop's barrier) timed out");
+  }
   const long long last = hst.it - 1;  // the last step run
   double are = 1.0, aim = 0.0;
   amp((double)hst.it / opts->iterations_per_cycle, &are, &aim, opts->user_data);  // PSTD.m:125
@@ -3493,6 +3496,11 @@ int ws_pstd_run(ws_pstd h, int64_t n_blocks, const ws_source_block* source, int 
   if (n_iterations) *n_iterations = last;
   if (converged) *converged = hst.converged;
   return WS_OK;
+}
+
+int ws_pstd_set_wait_limit(ws_pstd h, int64_t clocks) {
+  if (!h) return fail(WS_ERR_INVALID_ARGUMENT, "null solver");
+  return ws_solver_set_wait_limit(reinterpret_cast<ws_solver>(reinterpret_cast<Pstd*>(h)->s), clocks);
 }
 
 int ws_pstd_destroy(ws_pstd h) {
