@@ -261,7 +261,9 @@ int ws_solver_time_kernels(ws_solver s, int n_iterations, float ms_out[3], doubl
 int ws_solver_set_wait_limit(ws_solver s, int64_t clocks);
 
 /* Number of kernel launches one iteration makes (the stop rule is one more per
- * wiggle cycle). */
+ * wiggle cycle).  This, ws_solver_fused and the ws_solver_time_... are about the
+ * launched passes; single solves of small 2-D grids run the whole loop in one
+ * launch instead. */
 int ws_solver_launches_per_iteration(ws_solver s);
 
 /* 1 if the solver's loop fuses K3 of an iteration with K1 of the next (the

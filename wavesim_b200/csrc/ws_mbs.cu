@@ -2637,8 +2637,8 @@ int ws_solver_launches_per_iteration(ws_solver h) {
   if (!h) return 0;
   const Solver* s = reinterpret_cast<Solver*>(h);
   // K2, K3 + next K1 (one kernel, or the split step's three); or K1, K2, K3
-  // (the stop rule is one launch per wiggle cycle)
-  if (!s->fuse) return 3;
+  // (the stop rule is one launch per wiggle cycle), of the launched passes
+  if (!s->fuses[0]) return 3;
   const Layout& L = s->lays[0];
   if (!L.mode3d) return 2;
   return L.xp || L.uni_in ? 4 : 2;
@@ -2646,15 +2646,15 @@ int ws_solver_launches_per_iteration(ws_solver h) {
 
 int ws_solver_fused(ws_solver h) {
   if (!h) return 0;
-  return reinterpret_cast<Solver*>(h)->fuse ? 1 : 0;
+  return reinterpret_cast<Solver*>(h)->fuses[0] ? 1 : 0;
 }
 
 int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* bytes_out) {
   if (!h || !ms_out || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
-  if (!s->fuse) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not fuse K3 with K1");
   WS_CUDA(cudaSetDevice(s->device));
-  WS_CUDA(use_layout(s, 0));
+  WS_CUDA(use_layout(s, 0));  // the launched passes
+  if (!s->fuse) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not fuse K3 with K1");
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
@@ -2691,9 +2691,9 @@ int ws_solver_time_fused(ws_solver h, int n_iterations, float* ms_out, double* b
 int ws_solver_time_split(ws_solver h, int n_iterations, float ms_out[3], double bytes_out[3]) {
   if (!h || !ms_out || n_iterations < 1) return fail(WS_ERR_INVALID_ARGUMENT, "bad argument");
   Solver* s = reinterpret_cast<Solver*>(h);
-  if (!s->fuse || !s->lay.mode3d || !(s->lay.xp || s->lay.uni_in)) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
   WS_CUDA(cudaSetDevice(s->device));
   WS_CUDA(use_layout(s, 0));
+  if (!s->fuse || !s->lay.mode3d || !(s->lay.xp || s->lay.uni_in)) return fail(WS_ERR_UNSUPPORTED, "this solver's loop does not run the split step");
   const long long cap = n_iterations + 1;
   if (s->hist_cap < cap) {
     const int rc = ensure_hist(s, cap);
