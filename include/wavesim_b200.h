@@ -266,6 +266,10 @@ int ws_solver_set_wait_limit(ws_solver s, int64_t clocks);
  * launch instead. */
 int ws_solver_launches_per_iteration(ws_solver s);
 
+/* 1 if single solves run the loop in one launch: 2-D scalar grids whose columns
+ * fit the shared memory of the SMs that the process has. */
+int ws_solver_loop_in_one_launch(ws_solver s);
+
 /* 1 if the solver's loop fuses K3 of an iteration with K1 of the next (the
  * one-kernel step on a cluster, the split step of 3-D planes, the column
  * pass of 2-D grids), 0 if it runs K1, K2 and K3 as separate kernels.  No

@@ -4,6 +4,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from oracle import mbs_oracle as ref
+
 pytestmark = pytest.mark.gpu
 
 
@@ -28,3 +30,43 @@ def test_queries_are_about_the_launched_passes(gpu):
         assert s1.it == s0.it
         np.testing.assert_array_equal(E1, E0)
     sim.close()
+
+
+@pytest.mark.parametrize("shape,bw,room", [((96, 200), [32, 32], 131), ((96, 200), [32, 32], 0), ((48, 40), [8, 8], 15),
+                                           ((48, 40), [8, 8], 7)])
+def test_without_room_for_the_loop_the_passes_are_launched(gpu, shape, bw, room, monkeypatch):
+    """160 x 264 has 132 column tiles, 64 x 56 has 14 (and 16 tiles of pencils): with fewer blocks at a time than column
+    tiles the solve runs the launched passes; with fewer than all tiles the loop is no cluster.  A dozen iterations of
+    single precision differ by a few 1e-7."""
+    import wavesim_b200 as ws
+    from wavesim_b200 import _lib
+    n = 1.1 + 0.2 * np.random.default_rng(5).random(shape) + 0.01j
+    opt = {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": bw, "energy_threshold": 1e-99, "max_iterations": 12}
+    src = ws.Source(np.ones((shape[0], 1)) + 0.4j, [1, 1])
+    sim = ws.WaveSim(n, opt)
+    assert _lib.lib.ws_solver_loop_in_one_launch(sim.solver()) == 1
+    E0, s0 = sim.exec(src)
+    sim.close()
+    monkeypatch.setenv("WAVESIM_B200_LOOP", str(room))
+    sim = ws.WaveSim(n, opt)
+    assert _lib.lib.ws_solver_loop_in_one_launch(sim.solver()) == (1 if room == 15 else 0)
+    E1, s1 = sim.exec(src)
+    sim.close()
+    assert s1.it == s0.it
+    assert np.linalg.norm(E1 - E0) < 1e-5 * np.linalg.norm(E0)
+    monkeypatch.delenv("WAVESIM_B200_LOOP")
+
+
+@pytest.mark.filterwarnings("ignore:The PSTD code")
+def test_pstd_without_room_for_its_loop(gpu, monkeypatch):
+    import wavesim_b200 as ws
+    n = 1.0 + 0.2 * np.random.default_rng(2).random((60, 70)) + 0.02j
+    opt = {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": [8, 8], "boundary_type": "ARL", "energy_threshold": 1e-30}
+    got = []
+    for room in ("", "9"):
+        if room:
+            monkeypatch.setenv("WAVESIM_B200_LOOP", room)
+        p = ws.PSTD(n, opt)
+        got.append(p.exec(ws.Source(np.ones((60, 1)), [1, 2]), max_iterations=100)[0])
+        p.close()
+    assert np.linalg.norm(got[1] - got[0]) < 5e-5 * np.linalg.norm(got[0])

@@ -861,6 +861,8 @@ struct Solver {
   float2* d_tw = nullptr;
   Layout lays[2];                // the layouts of the launched passes [0] and of the loop in one launch [1];
   bool has_loop = false;         //   `lay` is the one in use, lays[active]
+  int loop_blocks = 0;           // the loop's blocks that run at a time
+  bool loop_clusters = false;    // up to 16 of them as one cluster
   int active = 0;
   int fuses[2] = {};             // `fuse` of each
   UniTables ut[2];               // their tables
@@ -1194,10 +1196,62 @@ static cudaError_t use_layout(Solver* s, int k) {
   return cudaSuccess;
 }
 
+// Threads of the loop's blocks: a butterfly each, or 512.
+static int loop_threads(const Layout& L) {
+  const int work = std::max(L.ucol.lines * uni_units(L.ucol.plan), L.uout.lines * uni_units(L.uout.plan));
+  return work <= 256 ? 256 : uni::kLoopThreads;
+}
+// Tiles of the loop, and whether its blocks form one cluster.
+static long long loop_tiles(const Solver* s, int nrhs) {
+  return std::max(s->lays[1].ucol.grid, s->lays[1].uout.grid) * nrhs;
+}
+static bool loop_cluster(const Solver* s, int nrhs) { return s->loop_clusters && loop_tiles(s, nrhs) <= 16; }
+
+// How many of the loop's blocks run at a time: one an SM, as many as the device
+// has free for this process (a share of it has fewer than kNumSms, and would
+// refuse the launch).  WAVESIM_B200_LOOP=n: at most n (0: no loop in one launch).
+static cudaError_t loop_room(Solver* s) {
+  const Layout& L = s->lays[1];
+  const uni::Kernels& k = uni_kernels(std::max(L.ucol.plan.cls, L.uout.plan.cls));
+  const void* fn = s->pstd ? k.pstd_loop : k.loop;
+  size_t smem = s->pstd ? pstd_loop_smem(L, s->g) : loop_smem(L, s->g, s->nw, true);
+  if (smem > kLoopSmem) smem = loop_smem(L, s->g, s->nw, false);
+  const int threads = loop_threads(L);
+  int sms = 0, per_sm = 0, clusters = 0;
+  s->loop_blocks = 0;
+  s->loop_clusters = false;
+  if (smem > kLoopSmem) return cudaSuccess;
+  cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
+  if (e != cudaSuccess) return e;
+  s->loop_blocks = per_sm > 0 ? std::min(sms, kNumSms) : 0;
+  if (const char* most = std::getenv("WAVESIM_B200_LOOP")) s->loop_blocks = std::min(s->loop_blocks, std::max(0, std::atoi(most)));
+  const long long tiles = loop_tiles(s, 1);
+  if (tiles > std::min(16, s->loop_blocks)) return cudaSuccess;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)tiles;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)tiles);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  s->loop_clusters = cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0;
+  cudaGetLastError();
+  return cudaSuccess;
+}
+
 // The layouts for choice ch of the launched passes (lays[0], made by the
 // caller); the one of single solves is then in use.
 static cudaError_t set_layouts(Solver* s, const LayoutChoice& ch) {
   s->has_loop = loop_layout(s->g, s->lays[0], ch, s->pstd != 0, s->lays[1]);
+  if (s->has_loop) {
+    const cudaError_t e = loop_room(s);
+    if (e != cudaSuccess) return e;
+    s->has_loop = s->lays[1].ucol.grid <= s->loop_blocks;
+  }
   for (int k = 0; k < 2; ++k) {
     if (s->ut[k].wigs) cudaFree(s->ut[k].wigs);
     s->ut[k] = UniTables{};
@@ -1944,7 +1998,7 @@ static cudaError_t launch_iteration(const Solver* s, int it0, bool with_source) 
 // Whether nrhs right-hand sides can run as one launch of the loop
 // (uni::k_loop): a column tile of each on an SM of its own.
 static bool loop_fits(const Solver* s, int nrhs) {
-  return s->has_loop && nrhs <= uni::kLoopRhs && nrhs * s->lays[1].ucol.grid <= kNumSms &&
+  return s->has_loop && nrhs <= uni::kLoopRhs && nrhs * s->lays[1].ucol.grid <= s->loop_blocks &&
          loop_smem(s->lays[1], s->g, s->nw, false) <= kLoopSmem;
 }
 
@@ -1953,18 +2007,15 @@ static bool loop_fits(const Solver* s, int nrhs) {
 // without a counter).
 static cudaError_t launch_coop(const Solver* s, const void* fn, size_t smem, int nrhs, void* args, unsigned** arrived) {
   const Layout& L = s->lay;
-  const long long tiles = std::max(L.ucol.grid, L.uout.grid) * nrhs;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)std::min<long long>(tiles, kNumSms));
-  const bool cluster = tiles <= 16;
+  cfg.gridDim = dim3((unsigned)std::min<long long>(loop_tiles(s, nrhs), s->loop_blocks));
+  const bool cluster = loop_cluster(s, nrhs);
   *arrived = cluster ? nullptr : (unsigned*)(s->d_err + 1);
   if (!cluster) {
     const cudaError_t e = cudaMemsetAsync(*arrived, 0, sizeof(unsigned), s->stream);
     if (e != cudaSuccess) return e;
   }
-  // a butterfly per thread, or 512
-  const int work = std::max(L.ucol.lines * uni_units(L.ucol.plan), L.uout.lines * uni_units(L.uout.plan));
-  cfg.blockDim = dim3(work <= 256 ? 256 : uni::kLoopThreads);
+  cfg.blockDim = dim3(loop_threads(L));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s->stream;
   cudaLaunchAttribute attr[1];
@@ -2642,6 +2693,12 @@ int ws_solver_launches_per_iteration(ws_solver h) {
   const Layout& L = s->lays[0];
   if (!L.mode3d) return 2;
   return L.xp || L.uni_in ? 4 : 2;
+}
+
+int ws_solver_loop_in_one_launch(ws_solver h) {
+  if (!h) return 0;
+  const Solver* s = reinterpret_cast<Solver*>(h);
+  return loop_fits(s, 1) && s->fuses[1] ? 1 : 0;
 }
 
 int ws_solver_fused(ws_solver h) {
