@@ -317,7 +317,9 @@ int ws_solver_warm_residual(ws_solver s, int64_t rhs, double* cold_residual_ener
  * and uses them from the next solve on.  A candidate must first reproduce one iteration of the current
  * layout to 1e-4.  Outputs (may be NULL): candidates tried, and the time of
  * one iteration (K1 + K2 + K3, ms) before and after.  Overwrites the solver's
- * fields; call it between solves. */
+ * fields; call it between solves.  Single solves that run the loop in one launch
+ * (ws_solver_loop_in_one_launch) do so whatever was chosen for the launched
+ * passes, which then serve batches. */
 int ws_solver_autotune(ws_solver s, int n_iterations, int* n_tried, float* ms_before, float* ms_after);
 
 /* The solver's layout choice as 7 integers (the autotuner's pick, or zeros

@@ -32,6 +32,25 @@ def test_queries_are_about_the_launched_passes(gpu):
     sim.close()
 
 
+def test_a_tuned_layout_leaves_the_loop_in_one_launch(gpu):
+    import wavesim_b200 as ws
+    from wavesim_b200 import _lib
+    from wavesim_b200.autotune import set_layout
+    n = 1.1 + 0.2 * np.random.default_rng(3).random((96, 80)) + 0.01j
+    sim = ws.WaveSim(n, {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": [16, 16], "energy_threshold": 1e-3})
+    src = ws.Source(1.0, [48, 40])
+    E0, s0 = sim.exec(src)
+    h = sim.solver()
+    for choose in (lambda: set_layout(sim, [2, 2, 0, 0, 0, 0, 0]), lambda: set_layout(sim, [0, 2, 0, 0, 4, 0, 0]),
+                   lambda: _lib.check(_lib.lib.ws_solver_autotune(h, 4, None, None, None))):
+        choose()
+        assert _lib.lib.ws_solver_loop_in_one_launch(h) == 1
+        E1, s1 = sim.exec(src)
+        assert s1.it == s0.it
+        np.testing.assert_array_equal(E1, E0)
+    sim.close()
+
+
 @pytest.mark.parametrize("shape,bw,room", [((96, 200), [32, 32], 131), ((96, 200), [32, 32], 0), ((48, 40), [8, 8], 15),
                                            ((48, 40), [8, 8], 7)])
 def test_without_room_for_the_loop_the_passes_are_launched(gpu, shape, bw, room, monkeypatch):

@@ -569,9 +569,12 @@ static size_t pstd_loop_smem(const Layout& L, const Geom& g, int* tile_elems = n
 // 396 x 315 11.0 (19.7), 512^2 12.6 (18.8, compile-time kernels), 632^2 20.3
 // (23.9), 1100 x 768 27.8 (38); 1024^2 38.7 (34.2, compile-time kernels).  So
 // it takes every grid whose columns fit the SMs' shared memory, but those with
-// compile-time kernels in both passes only up to 400 000 points.
-static bool loop_layout(const Geom& g, const Layout& L, const LayoutChoice& ch, bool pstd, Layout& out) {
-  if (L.mode3d || g.nc != 1 || ch.inner == 2 || ch.outer == 2) return false;
+// compile-time kernels in both passes only up to 400 000 points.  A choice of
+// the launched passes' kernels (the autotuner's, which times only those) leaves
+// it as it is: `heuristic` is their layout without one.
+static bool loop_layout(const Geom& g, const Layout& heuristic, bool pstd, Layout& out) {
+  const Layout& L = heuristic;
+  if (L.mode3d || g.nc != 1) return false;
   const char* path = std::getenv("WAVESIM_B200_PATH");
   if (path && std::strcmp(path, "generic") == 0) return false;
   if (L.fi && L.fp && g.npts > 400000 && !pstd) return false;
@@ -1243,10 +1246,13 @@ static cudaError_t loop_room(Solver* s) {
   return cudaSuccess;
 }
 
-// The layouts for choice ch of the launched passes (lays[0], made by the
+// The layouts beside that of the launched passes (lays[0], made by the
 // caller); the one of single solves is then in use.
-static cudaError_t set_layouts(Solver* s, const LayoutChoice& ch) {
-  s->has_loop = loop_layout(s->g, s->lays[0], ch, s->pstd != 0, s->lays[1]);
+static cudaError_t set_layouts(Solver* s) {
+  Layout heuristic;
+  std::string why;
+  s->has_loop = make_layout(s->g, heuristic, why, LayoutChoice{}, s->pstd != 0) == WS_OK &&
+                loop_layout(s->g, heuristic, s->pstd != 0, s->lays[1]);
   if (s->has_loop) {
     const cudaError_t e = loop_room(s);
     if (e != cudaSuccess) return e;
@@ -1392,7 +1398,7 @@ static int create_solver(const int64_t N[4], const ws_complex* gamma, int64_t n_
     s->wig.push_back(Wig{f, f + g.nx, f + g.nx + g.ny, c, c + g.nx, c + g.nx + g.ny});
   }
   s->lays[0] = s->lay;
-  WS_TRY(set_layouts(s, LayoutChoice{}));
+  WS_TRY(set_layouts(s));
   WS_TRY(cudaMalloc(&s->d_gamma, (size_t)g.npts * sizeof(float2)));
   WS_TRY(cudaMemcpy(s->d_gamma, gamma, (size_t)g.npts * sizeof(float2), kind));
 #undef WS_TRY
@@ -2989,7 +2995,7 @@ static bool apply_choice(Solver* s, const LayoutChoice& c) {
   if (L.mode3d && !L.fi && !L.uni_in && s->g.nx / L.csize != s->pxl.n) return false;
   if (ensure_partials(s, L.grid_inner * std::max(1, s->batch_cap) * s->nw) != WS_OK) return false;
   s->lays[0] = L;
-  if (set_layouts(s, c) != cudaSuccess || use_layout(s, 0) != cudaSuccess) return false;
+  if (set_layouts(s) != cudaSuccess || use_layout(s, 0) != cudaSuccess) return false;
   apply_sched(s, c.sched);
   free_graph(s);
   return true;
