@@ -89,3 +89,41 @@ def test_pstd_without_room_for_its_loop(gpu, monkeypatch):
         got.append(p.exec(ws.Source(np.ones((60, 1)), [1, 2]), max_iterations=100)[0])
         p.close()
     assert np.linalg.norm(got[1] - got[0]) < 5e-5 * np.linalg.norm(got[0])
+
+
+# The compile-time kernels of 2-D grids: single solves of these sizes run the loop in one launch, batches too large for
+# it still run these passes.
+FAST = {"64": ((32, 32), [16, 16]), "128x256": ((96, 224), [16, 16]), "512": ((448, 448), [32, 32]),
+        "320": ((256, 256), [32, 32]), "448": ((384, 384), [32, 32]), "576": ((512, 512), [32, 32]),
+        "192": ((160, 160), [16, 16]), "320x100": ((256, 68), [32, 16]), "256x192": ((224, 160), [16, 16]),
+        "512x120": ((448, 100), [32, 10])}
+
+
+@pytest.mark.parametrize("name", list(FAST))
+def test_compile_time_kernels_without_the_loop(gpu, name, monkeypatch):
+    """Against the FP32 oracle, and the fused column pass against K1 and K3 as kernels of their own, bit for bit.  16
+    iterations of single precision differ by a few 1e-7; 1e-5 leaves none for a wrong element."""
+    import wavesim_b200 as ws
+    from wavesim_b200 import _lib
+    shape, bw = FAST[name]
+    rng = np.random.default_rng(7)
+    n = 1.2 + 0.2 * rng.random(shape) + 0.005j
+    opt = {"lambda": 1.0, "pixel_size": 0.25, "boundary_widths": bw, "energy_threshold": 1e-99, "max_iterations": 16}
+    val = rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+    monkeypatch.setenv("WAVESIM_B200_LOOP", "0")
+    got = []
+    for fuse in ("1", "0"):
+        monkeypatch.setenv("WAVESIM_B200_FUSE", fuse)
+        sim = ws.WaveSim(n, opt)
+        assert _lib.lib.ws_solver_loop_in_one_launch(sim.solver()) == 0
+        assert _lib.lib.ws_solver_fused(sim.solver()) == int(fuse)
+        got.append(sim.exec(ws.Source(val, [1, 1])))
+        sim.close()
+    (E, st), (Eu, su) = got
+    Eo, so = ref.WaveSim(n, opt).exec(ref.Source(val, [1, 1, 1]), max_iterations=16)
+    assert st.it == su.it == so.it
+    np.testing.assert_array_equal(E, Eu)
+    np.testing.assert_array_equal(st.diff_energy, su.diff_energy)
+    Eo = Eo.reshape(E.shape)
+    assert np.linalg.norm(E - Eo) < 1e-5 * np.linalg.norm(Eo)
+    np.testing.assert_allclose(st.diff_energy, so.diff_energy, rtol=2e-4)
