@@ -402,7 +402,8 @@ static double excess(float2 w) { return 0.5 * ((double)w.x * w.x + (double)w.y *
 // a mean of zero (the butterflies' outputs, and the mean over the positions).
 // pos: p of j + r n / R0 is pos[j] + round_trip(1, R0, r); freq, in the order of
 // T: f of u + i n / RL is freq[u] + round_trip(0, RL, i) (both are 0 for r = i = 0).
-static void uni_gains(const uni::Plan& P, std::vector<double>& pos, std::vector<double>& freq) {
+// tw: the plan's twiddles.
+static void uni_gains(const uni::Plan& P, const float2* tw, std::vector<double>& pos, std::vector<double>& freq) {
   pos.assign(P.n, 0.0);
   freq.assign(P.n, 0.0);
   double mean = 0.0;
@@ -411,7 +412,7 @@ static void uni_gains(const uni::Plan& P, std::vector<double>& pos, std::vector<
     std::vector<double> tin(S.sub, 0.0), out(S.R, 0.0);
     for (int r = 0; r < S.R; ++r) {
       for (int j = 0; j < S.sub; ++j) {
-        const double g = 2.0 * excess(uni_twiddle(j, r, S.R * S.sub));
+        const double g = 2.0 * excess(tw[S.two + r * S.sub + j]);
         tin[j] += g / S.R;
         out[r] += g / S.sub;
       }
@@ -797,6 +798,7 @@ struct GraphKey {
 // out again by frequency and by position (minus uni_gains; 0 along the axes that
 // other kernels transform), the permuted p tables.
 struct UniTables {
+  void* buf = nullptr;
   Wig* wigs = nullptr;
   float2* ramp = nullptr;
   int* perm = nullptr;
@@ -899,7 +901,7 @@ static void destroy_solver(Solver* s) {
   free_graph(s);
   void* ptrs[] = {s->d_wigf, s->d_wigc,  s->d_gamma,  s->d_E,        s->d_dE, s->d_T,   s->d_src,
                   s->d_stage, s->d_out, s->d_state, s->d_hist, s->d_energy, s->d_tw, s->d_partials, s->d_init,
-                  s->d_err, s->ut[0].wigs, s->ut[1].wigs};
+                  s->d_err, s->ut[0].buf, s->ut[1].buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (auto& e : s->ev)
@@ -1133,6 +1135,7 @@ static cudaError_t make_tables(Solver* s, int k) {
         for (int j = 0; j < S.sub; ++j) tw.push_back(uni_twiddle(j, r, n));
     }
   }
+  const size_t nf = (size_t)g.nx + g.ny + g.nz;
   std::vector<int> perm;
   std::vector<float> efreq, epos;
   for (int d = 0; d < 3; ++d) {
@@ -1140,7 +1143,8 @@ static cudaError_t make_tables(Solver* s, int k) {
     const std::vector<int> f = axis[d] ? uni_permutation(*axis[d]) : std::vector<int>();
     std::vector<double> pos(len[d], 0.0), freq(len[d], 0.0);
     const bool columns = d == 1 && L.fi && !L.mode3d;  // compile-time columns, inside these kernels' pencils
-    if (axis[d]) uni_gains(*axis[d], pos, freq);
+    for (int q = 0; q < 3; ++q)
+      if (axis[d] && axis[d] == plans[q]) uni_gains(*axis[d], tw.data() + at[q], pos, freq);
     if (columns) line_gains(line_radices(g.ny), pos, freq);
     // without ramps of its own (PSTD, other column passes), the mean of the part by position
     const bool ramps = (L.uni_in || (L.fi && !L.mode3d)) && !s->pstd;
@@ -1152,46 +1156,58 @@ static cudaError_t make_tables(Solver* s, int k) {
       epos.push_back((float)-pos[i]);
     }
   }
-  const size_t wb = s->nw * sizeof(Wig), twb = tw.size() * sizeof(float2), pb = perm.size() * sizeof(int);
-  const size_t rb = 2 * pb * s->nw;  // the ramps
+  // one buffer: the ramps, what the host has (in one copy), the p tables
+  const size_t rb = nf * s->nw * sizeof(float2), wb = s->nw * sizeof(Wig), twb = tw.size() * sizeof(float2),
+               tb = nf * sizeof(float);
+  std::vector<char> host(wb + twb + 3 * tb);
   char* buf = nullptr;
-  cudaError_t e = cudaMalloc(&buf, wb + twb + rb + pb * (3 + s->nw));
+  cudaError_t e = cudaMalloc(&buf, rb + host.size() + tb * s->nw);
   if (e != cudaSuccess) return e;
-  t.wigs = reinterpret_cast<Wig*>(buf);
-  float2* const d_tw = reinterpret_cast<float2*>(buf + wb);
-  t.ramp = reinterpret_cast<float2*>(buf + wb + twb);
-  t.perm = reinterpret_cast<int*>(buf + wb + twb + rb);
-  t.efreq = reinterpret_cast<float*>(buf + wb + twb + rb + pb);
-  t.epos = reinterpret_cast<float*>(buf + wb + twb + rb + 2 * pb);
-  t.p = reinterpret_cast<float*>(buf + wb + twb + rb + 3 * pb);
+  t.ramp = reinterpret_cast<float2*>(buf);
+  t.wigs = reinterpret_cast<Wig*>(buf + rb);
+  float2* const d_tw = reinterpret_cast<float2*>(buf + rb + wb);
+  t.perm = reinterpret_cast<int*>(buf + rb + wb + twb);
+  t.efreq = reinterpret_cast<float*>(buf + rb + wb + twb + tb);
+  t.epos = t.efreq + nf;
+  t.p = t.epos + nf;
   for (int q = 0; q < 3; ++q) plans[q]->tw = d_tw + at[q];
   t.uwig = s->wig;
   for (int w = 0; w < s->nw; ++w) {
-    const float* f = t.p + perm.size() * w;
+    const float* f = t.p + nf * w;
     t.uwig[w].pxe = f;
     t.uwig[w].pye = f + g.nx;
     t.uwig[w].pze = f + g.nx + g.ny;
-    const float2* c = t.ramp + perm.size() * w;
+    const float2* c = t.ramp + nf * w;
     t.uwig[w].gx = c;
     t.uwig[w].gy = c + g.nx;
     t.uwig[w].gz = c + g.nx + g.ny;
   }
-  e = cudaMemcpyAsync(t.wigs, t.uwig.data(), wb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_tw, tw.data(), twb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(t.perm, perm.data(), pb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(t.efreq, efreq.data(), pb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(t.epos, epos.data(), pb, cudaMemcpyHostToDevice, s->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);  // the host tables end here
-  return e;
+  std::memcpy(host.data(), t.uwig.data(), wb);
+  std::memcpy(host.data() + wb, tw.data(), twb);
+  std::memcpy(host.data() + wb + twb, perm.data(), tb);
+  std::memcpy(host.data() + wb + twb + tb, efreq.data(), tb);
+  std::memcpy(host.data() + wb + twb + 2 * tb, epos.data(), tb);
+  e = cudaMemcpyAsync(t.wigs, host.data(), host.size(), cudaMemcpyHostToDevice, s->stream);  // pageable: taken at once
+  if (e != cudaSuccess) {  // nothing half made is kept
+    cudaFree(buf);
+    t = UniTables{};
+    return e;
+  }
+  t.buf = buf;
+  return cudaSuccess;
 }
 
 // Makes lays[k] the layout in use, with its tables (made on its first use:
 // few solvers run both).
 static cudaError_t use_layout(Solver* s, int k) {
-  if (s->lays[k].uni_out && !s->ut[k].wigs) {
+  if (s->lays[k].uni_out && !s->ut[k].buf) {
     cudaError_t e = make_tables(s, k);
-    if (e == cudaSuccess) e = permute_wiggles(s);
     if (e != cudaSuccess) return e;
+    if ((e = permute_wiggles(s)) != cudaSuccess) {
+      cudaFree(s->ut[k].buf);
+      s->ut[k] = UniTables{};
+      return e;
+    }
   }
   s->active = k;
   s->lay = s->lays[k];
@@ -1259,7 +1275,7 @@ static cudaError_t set_layouts(Solver* s) {
     s->has_loop = s->lays[1].ucol.grid <= s->loop_blocks;
   }
   for (int k = 0; k < 2; ++k) {
-    if (s->ut[k].wigs) cudaFree(s->ut[k].wigs);
+    if (s->ut[k].buf) cudaFree(s->ut[k].buf);
     s->ut[k] = UniTables{};
     s->fuses[k] = fuse_of(s, s->lays[k]);
   }
