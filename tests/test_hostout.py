@@ -101,6 +101,22 @@ BODIES = {
   void* p = ws::host_pool().get(1, &got);
   CHECK(p && !queued_into(p, got));
   return 0;""",
+    # groups of fields in a device buffer: the largest half, quarter, .. that fits, one field if need be, and no other error
+    # taken for a lack of memory
+    "groups_that_fit": r"""
+  for (int room : {100, 16, 15, 5, 1}) {
+    int tries = 0;
+    cudaError_t e;
+    const int g = ws::fitting_group(16, [&](int n) { ++tries; return n <= room ? cudaSuccess : cudaErrorMemoryAllocation; }, &e);
+    CHECK(e == cudaSuccess && g <= room && g >= 1 && tries <= 5);
+    CHECK(room < 16 || g == 16);
+  }
+  cudaError_t e;
+  CHECK(ws::fitting_group(16, [](int) { return cudaErrorMemoryAllocation; }, &e) == 1 && e == cudaErrorMemoryAllocation);
+  int tries = 0;
+  ws::fitting_group(16, [&](int) { ++tries; return cudaErrorUnknown; }, &e);
+  CHECK(e == cudaErrorUnknown && tries == 1);
+  return 0;""",
     # no page-locked memory at all: through ordinary memory
     "no_page_locked_memory": r"""
   host_allocs_left = 0;

@@ -123,6 +123,17 @@ struct HostLease {
   bool busy_ = false, pooled_ = false;
 };
 
+// The first of `group`, half of it, .. 1 for which make() finds memory (with its
+// error, if it is another); *e: the last one's.
+template <class Make>
+int fitting_group(int group, Make make, cudaError_t* e) {
+  while ((*e = make(group)) == cudaErrorMemoryAllocation && group > 1) {
+    cudaGetLastError();
+    group = (group + 1) / 2;
+  }
+  return group;
+}
+
 class OutCopy {
  public:
   // The threads touch dst's pages from here to run().

@@ -2422,17 +2422,20 @@ static int solve_batch(Solver* s, int nrhs, const int64_t* counts, const ws_sour
     return all;
   };
   // The fields: E' itself, or E on the roi through k_finalize (in groups of
-  // right-hand sides for host memory, so that the device copy stays below 512 MB).
+  // right-hand sides for host memory, so that the device copy, which the solver
+  // keeps, stays below 128 MB or one field; smaller groups where that does not fit).
   const size_t F = field_elems(s);
   const bool field = opt.output == WS_OUTPUT_FIELD;
   const size_t per = (field ? roi_elems(s->g) : F) * sizeof(float2);  // bytes of a right-hand side
   const bool to_host = E_out && out_memory != WS_DEVICE;
-  const int group = (int)std::min<size_t>(nrhs, std::max<size_t>(1, (512u << 20) / per));
+  int group = (int)std::min<size_t>(nrhs, std::max<size_t>(1, (128u << 20) / per));
   if (to_host && field && group * (per / sizeof(float2)) > s->out_cap) {
     if (s->d_out) cudaFree(s->d_out);
     s->d_out = nullptr;
     s->out_cap = 0;
-    WS_CUDA(cudaMalloc(&s->d_out, group * per));
+    cudaError_t e;
+    group = fitting_group(group, [&](int n) { return cudaMalloc(&s->d_out, n * per); }, &e);
+    WS_CUDA(e);
     s->out_cap = group * (per / sizeof(float2));
   }
   bool pageable = false;
