@@ -42,12 +42,13 @@
 //
 // Measured against the generic three-pass kernels (ws_kernels.cuh), which
 // hold every radix inlined with all of a thread's elements in local memory
-// (1.3-3.7 KB a thread), device time of one iteration: 125 x 144 x 99 64 us
-// against 361, 210 x 189 x 216 334 against 2311, 1100 x 768 40 against 102,
-// 63 x 77 x 70 x 3 52 against 138, 105 x 120 x 63 x 3 85 against 490.  Grids
-// whose passes fit the L2 are bound by the latency of a pass (load, two
-// butterflies, store) and the launches; larger ones by memory, at 2-3 times
-// the bytes' time.  The compile-time schedules stay where they exist: 192^3
+// (1.3-3.7 KB a thread), device time of one iteration of the launched passes:
+// 125 x 144 x 99 62 us against 361, 210 x 189 x 216 305 against 2311, 1100 x
+// 768 36 against 102, 63 x 77 x 70 x 3 49 against 138, 105 x 120 x 63 x 3 85
+// against 490.  Single solves of 2-D grids run them in k_loop instead, where
+// their columns fit the SMs' shared memory (1100 x 768: 30).  Grids whose
+// passes fit the L2 are bound by the latency of a pass (load, two butterflies,
+// store) and the launches; larger ones by memory, at 2-3 times the bytes' time.  The compile-time schedules stay where they exist: 192^3
 // takes 153 us with them and 232 with these.
 #pragma once
 #include "ws_kernels.cuh"
