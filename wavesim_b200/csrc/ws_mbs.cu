@@ -568,7 +568,7 @@ static size_t pstd_loop_smem(const Layout& L, const Geom& g, int* tile_elems = n
 // grid's launched passes; false if there is none.  Measured against the
 // launched passes, us an iteration: 64 x 56 7.6 (12.8), 160 x 264 12.4 (21.4),
 // 396 x 315 11.0 (19.7), 512^2 12.6 (18.8, compile-time kernels), 632^2 20.3
-// (23.9), 1100 x 768 27.8 (38); 1024^2 38.7 (34.2, compile-time kernels).  So
+// (23.9), 1100 x 768 30 (38); 1024^2 38.7 (34.2, compile-time kernels).  So
 // it takes every grid whose columns fit the SMs' shared memory, but those with
 // compile-time kernels in both passes only up to 400 000 points.  A choice of
 // the launched passes' kernels (the autotuner's, which times only those) leaves

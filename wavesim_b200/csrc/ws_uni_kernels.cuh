@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(kMaxThreads, kBlocks<RM>) k_x(const __grid_con
 // in shared memory.  Every block steps the stop rule for itself, so that no
 // barrier is spent on it.  us an iteration, before (one launch per pass) and
 // now: 64 x 56 12.8, 7.5; 160 x 264 21.4, 12.4; 396 x 315 19.7, 11.0; 512^2
-// 18.8, 12.6; 1100 x 768 38, 28.  With the fields left in global memory: 9.4,
+// 18.8, 12.7; 1100 x 768 38, 30.  With the fields left in global memory: 9.4,
 // 14.5, 14.6, 16.3, 34.  In 3-D (four barriers, more work per point) it lost:
 // 96^3 39 against 30, 63 x 77 x 70 x 3 58 against 49, so those stay launched.
 
